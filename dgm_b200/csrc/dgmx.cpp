@@ -226,15 +226,20 @@ struct dgmx_domain {
     return e;
   }
   bool ns() const { return prm.physics == DGMX_NS2D || prm.physics == DGMX_NS3D; }
+  // the tile whose viscous kernels and stage kernel run (they go together:
+  // what the viscous kernels leave in Pv is the stage kernel's affair)
+  const KernelOps *ns_ops() const { return visc32 && (visc_tc || !ops->ns_visc32) ? vops : ops; }
+  bool separate_grad() const { return visc32 ? ns_ops()->ns_grad32 != nullptr : ops->ns_grad != nullptr; }
   cudaError_t ns_grad(const StageArgs &a, bool nodal, cudaStream_t s) const {
+    if (!separate_grad()) return cudaSuccess;
     if (visc32 && visc_tc) return vops->ns_grad32tc(a, nodal, s);
-    return visc32 ? vops->ns_grad32(a, nodal, s) : ops->ns_grad(a, nodal, s);
+    return visc32 ? ns_ops()->ns_grad32(a, nodal, s) : ops->ns_grad(a, nodal, s);
   }
   cudaError_t ns_visc(const StageArgs &a, bool nodal, cudaStream_t s) const {
     if (visc32 && visc_tc) return vops->ns_visc32tc(a, nodal, s);
-    return visc32 ? vops->ns_visc32(a, nodal, s) : ops->ns_visc(a, nodal, s);
+    return visc32 ? ns_ops()->ns_visc32(a, nodal, s) : ops->ns_visc(a, nodal, s);
   }
-  int visc_epb() const { return (visc32 ? vops : ops)->epb; }
+  int visc_epb() const { return ns_ops()->epb; }
   // the viscous flux kernel over tile list which (0 boundary, 1 interior);
   // no launch for an empty list
   cudaError_t ns_visc_tiles(StageArgs a, int which, cudaStream_t s) const {
@@ -244,7 +249,7 @@ struct dgmx_domain {
     return ns_visc(a, false, s);
   }
   bool mixed() const { return prm.precision == DGMX_MIXED; }
-  const KernelOps *stage_ops() const { return mixed() ? ops_m : ops; }
+  const KernelOps *stage_ops() const { return mixed() ? ops_m : (ns() ? ns_ops() : ops); }
 
   void release() {
     if (graph) cudaGraphExecDestroy(graph);
@@ -561,7 +566,7 @@ dgmx_status enqueue_step(dgmx_domain *d, double dt) {
     cudaError_t e;
     if (d->ns()) {
       if ((e = d->ns_grad(a, false, d->stream)) != cudaSuccess) return d->cuda(e, "viscous gradient kernel");
-      ++d->launches;
+      if (d->separate_grad()) ++d->launches;
       if (overlaps(d)) {
         const dgmx_status xs = visc_overlapped(d, a);
         if (xs != DGMX_OK) return xs;
@@ -600,7 +605,7 @@ int launches_per_stage(const dgmx_domain *d) {
   // the viscous flux kernel
   const int split = (overlaps(d) && !d->hold ? 1 : 0) + (overlaps(d) && d->ns() ? 1 : 0);
   const int hold = d->hold ? (rank ? 3 : 2) : 0;   // (scatter,) reduce, apply
-  return (d->ns() ? 3 : 1) + split + hold + halo;
+  return (d->ns() ? (d->separate_grad() ? 3 : 2) : 1) + split + hold + halo;
 }
 
 // Host repeat of launch_reference_integrals' summation order over the
@@ -911,8 +916,10 @@ dgmx_status create_impl(const dgmx_mesh *m, const dgmx_params *p, dgmx_domain **
   }
   d->ops = find_ops(phys, pp + 1, qq);
   if (d->visc32) {
-    d->vops = d->ops;
-    if (!d->vops || !d->vops->ns_grad32) {
+    if (const std::vector<KernelOps> *vs = find_variants(phys, pp + 1, qq))
+      for (const KernelOps &o : *vs)
+        if (o.ns_grad32) { d->vops = &o; break; }
+    if (!d->vops) {
       g_create_error = "no FP32 viscous kernels built for p=" + std::to_string(pp) + ", q=" + std::to_string(qq);
       return DGMX_ERR_UNSUPPORTED;
     }
@@ -981,6 +988,7 @@ dgmx_status create_impl(const dgmx_mesh *m, const dgmx_params *p, dgmx_domain **
   };
   st = DGMX_OK;
   if (!chk(d->ops->init(d->tab), "kernel table upload")) { g_create_error = d->errmsg; d->release(); return st; }
+  if (d->vops && d->vops != d->ops && !chk(d->vops->init(d->tab), "kernel table upload")) { g_create_error = d->errmsg; d->release(); return st; }
   if (d->ops_m && !chk(d->ops_m->init(d->tab), "kernel table upload")) { g_create_error = d->errmsg; d->release(); return st; }
   if (!chk(cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking), "stream")) { g_create_error = d->errmsg; d->release(); return st; }
   bool ok = chk(dalloc(&d->U, d->nmodal()), "alloc U") && chk(dalloc(&d->Ut, d->nmodal()), "alloc Ut") &&
@@ -999,7 +1007,7 @@ dgmx_status create_impl(const dgmx_mesh *m, const dgmx_params *p, dgmx_domain **
                              chk(dalloc(&d->uref, (size_t)kUrefStride), "alloc reference state"))) &&
             (!d->ns() || (chk(dalloc(&d->Ghat, (size_t)d->ne * (d->dim + 1) * d->dim * d->ld), "alloc gradients") &&
                           chk(dalloc(&d->Vtr, (size_t)d->nslot * d->nfaces * (d->nf - 1) * d->gf), "alloc viscous traces") &&
-                          chk(dalloc(&d->Pv, (size_t)d->ne * (d->nf - 1) * d->ld), "alloc viscous divergence"))) &&
+                          chk(dalloc(&d->Pv, (size_t)d->ne * d->nf * d->ld), "alloc viscous divergence"))) &&
             (!d->ns() || d->dim != 3 || (chk(dalloc(&d->R0, (size_t)d->ne * d->nf), "alloc hold coefficients") &&
                                           chk(dalloc(&d->cbar, (size_t)d->nf), "alloc hold means"))) &&
             (gid_host.empty() ||
@@ -1554,11 +1562,11 @@ dgmx_status dgmx_time_derivative_device(dgmx_domain *d, const double *U_dev, dou
   if (d->ns()) {
     if ((e = d->ns_grad(a, true, d->stream)) != cudaSuccess) return d->cuda(e, "viscous gradient kernel");
     if ((e = d->ns_visc(a, true, d->stream)) != cudaSuccess) return d->cuda(e, "viscous flux kernel");
-    d->launches += 2;
+    d->launches += d->separate_grad() ? 2 : 1;
     if ((xs = exchange(d, visc_halo(d))) != DGMX_OK) return xs;
   }
   a.R0 = d->hold ? d->R0 : nullptr;
-  e = d->ops->rhs_nodal(a, d->stream);
+  e = (d->ns() ? d->ns_ops() : d->ops)->rhs_nodal(a, d->stream);
   ++d->launches;
   if (e != cudaSuccess) return d->cuda(e, "nodal rhs kernel");
   if (d->hold) {
@@ -1726,9 +1734,19 @@ dgmx_status dgmx_autotune(dgmx_domain *d, int reps, double *rows, int cap, int *
     a.kind = kRHS; a.X = d->U; a.U = d->U; a.Ut = d->Ut; a.A = scratch;
     a.Tin = d->T[d->tcur]; a.Tout = d->T[d->tcur ^ 1];
     if (d->mixed()) { a.Utf = d->Utf; a.Tinf = d->Tf[d->tcur]; a.Toutf = d->Tf[d->tcur ^ 1]; }
-    for (int w = 0; w < 2; ++w) e = v.stage(a, d->stream);
+    // Navier-Stokes: with the tile's viscous kernels (the tensor-core form's
+    // are fixed, and so is the stage kernel that goes with them)
+    auto pass = [&]() {
+      cudaError_t q = cudaSuccess;
+      if (d->ns() && !d->visc32) {
+        if (v.ns_grad) q = v.ns_grad(a, false, d->stream);
+        if (q == cudaSuccess) q = v.ns_visc(a, false, d->stream);
+      }
+      return q == cudaSuccess ? v.stage(a, d->stream) : q;
+    };
+    for (int w = 0; w < 2 && e == cudaSuccess; ++w) e = pass();
     cudaEventRecord(e0, d->stream);
-    for (int r = 0; r < reps && e == cudaSuccess; ++r) e = v.stage(a, d->stream);
+    for (int r = 0; r < reps && e == cudaSuccess; ++r) e = pass();
     cudaEventRecord(e1, d->stream);
     if (e == cudaSuccess) e = cudaEventSynchronize(e1);
     if (e != cudaSuccess) { st = d->cuda(e, "autotune launch"); break; }
@@ -2013,7 +2031,7 @@ dgmx_status dgmx_group_advance(dgmx_group *g, double dt, int nsteps) {
           const StageArgs a = stage_args(d, sp, dt);
           if (e == cudaSuccess) e = d->ns_grad(a, false, s);
           if (e == cudaSuccess) e = d->ns_visc_tiles(a, 0, s);
-          d->launches += 2;
+          d->launches += d->separate_grad() ? 2 : 1;
         }
         if (e == cudaSuccess) e = cudaEventRecord(g->ev_b, s);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(g->xs, g->ev_b, 0);

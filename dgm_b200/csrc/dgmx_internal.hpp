@@ -250,7 +250,8 @@ struct StageArgs {
   // Navier-Stokes BR1 (src/Navier_Stokes3d.cpp:182-391)
   double *Ghat;           // projected primitive gradients, modal [e][comp][dir][L^d]
   double *V;              // viscous normal-flux traces [e][face][field-1][gf]
-  double *Pv;             // projected viscous divergence, modal [e][field-1][L^d]
+  double *Pv;             // projected viscous divergence, modal [e][field-1][L^d], or
+                          // (tiles without ns_grad) that of the whole volume flux, [e][field][L^d]
   // boundary types t = 1..15 (GeomClass::bc): kind (DGMX_BC_*) and parameters
   int bckind[kMaxBcTypes + 1];
   double bcpar[kMaxBcTypes + 1][5];
@@ -291,6 +292,7 @@ constexpr int kMixedKey = 1000;
 struct KernelOps {
   int epb = 0, nt = 0, minb = 0, mixed = 0;
   int warp = 0;                                        // kind: 0 CTA tile, 2 prefetching persistent kernel
+  int preferred = 0;                                   // the default tile of its (physics, L, Q) when set
   size_t smem = 0;
   cudaError_t (*init)(const Tables1D &t) = nullptr;   // tables + smem attributes, current device
   cudaError_t (*stage)(const StageArgs &a, cudaStream_t s) = nullptr;
@@ -303,7 +305,9 @@ struct KernelOps {
   cudaError_t (*rhs_nodal)(const StageArgs &a, cudaStream_t s) = nullptr;
   cudaError_t (*forward)(const StageArgs &a, const double *Un, double *Um, cudaStream_t s) = nullptr;
   cudaError_t (*backward)(const StageArgs &a, const double *Um, double *Un, cudaStream_t s) = nullptr;
-  // Navier-Stokes only: lifted gradients, then viscous traces + divergence;
+  // Navier-Stokes only: lifted gradients, then viscous traces + divergence
+  // (no ns_grad: ns_visc does both and leaves the projected divergence of the
+  // whole volume flux in a.Pv for this tile's stage and rhs_nodal);
   // nodal = read GLL values from a.Xn instead of the modal register a.X
   cudaError_t (*ns_grad)(const StageArgs &a, bool nodal, cudaStream_t s) = nullptr;
   cudaError_t (*ns_visc)(const StageArgs &a, bool nodal, cudaStream_t s) = nullptr;

@@ -4,6 +4,7 @@
 
 #include "ns.cuh"
 #include "pipeline.cuh"
+#include "form3.cuh"
 #include "stage2.cuh"
 
 namespace dgmx {
@@ -447,6 +448,82 @@ void reg2() {
   constexpr int A72 = blocks_for_regs<CA>(NTA, 72), B72 = blocks_for_regs<CB>(NTB, 72);
   if constexpr (!MIXED && A72 >= 2 && A72 != A80) reg2_variant<PHYS, P, Q, 1, NTA, A72, MIXED>();
   if constexpr (!MIXED && B72 >= 2 && B72 != B80) reg2_variant<PHYS, P, Q, 1, NTB, B72, MIXED>();
+}
+
+// Threads of a third-form tile: about one per modal row, 64 to 256.
+constexpr int form3_threads(int L) {
+  const int t = (5 * L * L + 31) / 32 * 32;
+  return t < 64 ? 64 : (t > 256 ? 256 : t);
+}
+// CTAs per SM that smem bytes and a cap of r registers per thread allow.
+constexpr int form3_blocks(size_t smem, int nt, int r) {
+  const int per_part = 16384 / (32 * r), by_regs = per_part * 4 / ((nt + 31) / 32);
+  const int by_smem = (int)((228 * 1024) / (smem + 1024));
+  const int b = by_regs < by_smem ? by_regs : by_smem;
+  return b < 1 ? 1 : b;
+}
+
+// Navier-Stokes 3-D in the third form: ns_flux_kernel, then ns_update_kernel
+// as the stage kernel (every stage kind).  The projections and trace kernels
+// come from the plain tile.
+template <int PHYS, int L, int Q>
+struct Launch3Ns {
+  using Base = Launch<PHYS, L, Q, default_epb(3, Q), 0>;
+  static constexpr int NT = form3_threads(L);
+  using C0 = Cfg3<PHYS, L, Q, NT, 0, false>;
+  using CF = Cfg3<PHYS, L, Q, NT, form3_blocks(NsFlux<C0>::SMEM, NT, 112), false>;
+  using CU = Cfg3<PHYS, L, Q, NT, form3_blocks(NsUpdate<C0>::SMEM, NT, 80), false>;
+  using F = NsFlux<CF>;
+  using N = NsUpdate<CU>;
+  static cudaError_t init(const Tables1D &t) {
+    cudaError_t e = Base::init(t);
+    if (e == cudaSuccess) e = upload_tables2_lq<L, Q, double>(t);
+    auto attr = [&](auto k, size_t smem) {
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    };
+    attr(ns_flux_kernel<CF, PHYS, false>, F::SMEM);
+    attr(ns_flux_kernel<CF, PHYS, true>, F::SMEM);
+    attr(ns_update_kernel<CU, PHYS, false>, N::SMEM);
+    attr(ns_update_kernel<CU, PHYS, true>, N::SMEM);
+    return e;
+  }
+  static cudaError_t flux(const StageArgs &a, bool nodal, cudaStream_t s) {
+    const unsigned g = a.vtiles ? a.nvtiles : a.ne;
+    if (nodal) ns_flux_kernel<CF, PHYS, true><<<g, NT, F::SMEM, s>>>(a);
+    else ns_flux_kernel<CF, PHYS, false><<<g, NT, F::SMEM, s>>>(a);
+    return cudaGetLastError();
+  }
+  static cudaError_t stage_grid(const StageArgs &a, int g, cudaStream_t s) {
+    ns_update_kernel<CU, PHYS, false><<<g, NT, N::SMEM, s>>>(a);
+    return cudaGetLastError();
+  }
+  static cudaError_t stage(const StageArgs &a, cudaStream_t s) { return stage_grid(a, a.ne, s); }
+  static cudaError_t rhs_nodal(const StageArgs &a, cudaStream_t s) {
+    ns_update_kernel<CU, PHYS, true><<<a.ne, NT, N::SMEM, s>>>(a);
+    return cudaGetLastError();
+  }
+  static int blocks_per_sm() {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ns_update_kernel<CU, PHYS, false>, NT, N::SMEM) !=
+        cudaSuccess) {
+      cudaGetLastError();
+      return 1;
+    }
+    return n > 0 ? n : 1;
+  }
+  static KernelOps ops() {
+    KernelOps o = Base::ops();
+    o.epb = 1; o.nt = NT; o.minb = CF::MINB; o.smem = F::SMEM; o.preferred = 1;
+    o.init = init; o.stage = stage; o.stage_grid = stage_grid; o.blocks_per_sm = blocks_per_sm;
+    o.rhs_nodal = rhs_nodal;
+    o.ns_grad = nullptr; o.ns_visc = flux;
+    o.ns_grad32 = o.ns_visc32 = o.ns_grad32tc = o.ns_visc32tc = nullptr;
+    return o;
+  }
+};
+template <int PHYS, int P, int Q>
+void reg3_ns() {
+  register_ops(PHYS, P + 1, Q, Launch3Ns<PHYS, P + 1, Q>::ops());
 }
 
 template <int PHYS, int P, int Q, int EPB, int MINB, bool MIXED>

@@ -26,8 +26,11 @@ const KernelOps *find_ops(int physics, int L, int Q) {
   std::lock_guard<std::mutex> lk(table_mutex());
   auto it = table().find(std::make_tuple(physics, L, Q));
   if (it == table().end() || it->second.empty()) return nullptr;
-  // the default is the first plain CTA tile (it handles every stage kind and
-  // boundary sides), whatever order the compilation units registered in
+  // the default is the preferred tile, else the first plain CTA tile (both
+  // handle every stage kind and boundary sides), whatever order the
+  // compilation units registered in
+  for (const KernelOps &o : it->second)
+    if (o.preferred) return &o;
   for (const KernelOps &o : it->second)
     if (o.warp == 0) return &o;
   return &it->second.front();
