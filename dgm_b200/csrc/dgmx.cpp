@@ -226,20 +226,21 @@ struct dgmx_domain {
     return e;
   }
   bool ns() const { return prm.physics == DGMX_NS2D || prm.physics == DGMX_NS3D; }
-  // the tile whose viscous kernels and stage kernel run (they go together:
-  // what the viscous kernels leave in Pv is the stage kernel's affair)
-  const KernelOps *ns_ops() const { return visc32 && (visc_tc || !ops->ns_visc32) ? vops : ops; }
-  bool separate_grad() const { return visc32 ? ns_ops()->ns_grad32 != nullptr : ops->ns_grad != nullptr; }
+  // the tile whose viscous kernels run (what they leave in Pv is read by the
+  // stage kernel of the same form)
+  const KernelOps *visc_ops() const {
+    if (!visc32) return ops;
+    return visc_tc ? ops->tensor : (ops->ns_visc32 ? ops : vops);
+  }
+  bool separate_grad() const { return (visc32 ? visc_ops()->ns_grad32 : visc_ops()->ns_grad) != nullptr; }
   cudaError_t ns_grad(const StageArgs &a, bool nodal, cudaStream_t s) const {
     if (!separate_grad()) return cudaSuccess;
-    if (visc32 && visc_tc) return vops->ns_grad32tc(a, nodal, s);
-    return visc32 ? ns_ops()->ns_grad32(a, nodal, s) : ops->ns_grad(a, nodal, s);
+    return visc32 ? visc_ops()->ns_grad32(a, nodal, s) : visc_ops()->ns_grad(a, nodal, s);
   }
   cudaError_t ns_visc(const StageArgs &a, bool nodal, cudaStream_t s) const {
-    if (visc32 && visc_tc) return vops->ns_visc32tc(a, nodal, s);
-    return visc32 ? ns_ops()->ns_visc32(a, nodal, s) : ops->ns_visc(a, nodal, s);
+    return visc32 ? visc_ops()->ns_visc32(a, nodal, s) : visc_ops()->ns_visc(a, nodal, s);
   }
-  int visc_epb() const { return ns_ops()->epb; }
+  int visc_epb() const { return visc_ops()->epb; }
   // the viscous flux kernel over tile list which (0 boundary, 1 interior);
   // no launch for an empty list
   cudaError_t ns_visc_tiles(StageArgs a, int which, cudaStream_t s) const {
@@ -248,8 +249,10 @@ struct dgmx_domain {
     a.vtiles = vtiles + (which == 0 ? 0 : nvt_b);
     return ns_visc(a, false, s);
   }
+  // projected gradients in global memory: tiles with a gradient kernel only
+  cudaError_t alloc_gradients() { return Ghat ? cudaSuccess : dalloc(&Ghat, (size_t)ne * (dim + 1) * dim * ld); }
   bool mixed() const { return prm.precision == DGMX_MIXED; }
-  const KernelOps *stage_ops() const { return mixed() ? ops_m : (ns() ? ns_ops() : ops); }
+  const KernelOps *stage_ops() const { return mixed() ? ops_m : (visc_tc ? ops->tensor : ops); }
 
   void release() {
     if (graph) cudaGraphExecDestroy(graph);
@@ -918,7 +921,7 @@ dgmx_status create_impl(const dgmx_mesh *m, const dgmx_params *p, dgmx_domain **
   if (d->visc32) {
     if (const std::vector<KernelOps> *vs = find_variants(phys, pp + 1, qq))
       for (const KernelOps &o : *vs)
-        if (o.ns_grad32) { d->vops = &o; break; }
+        if (o.ns_visc32) { d->vops = &o; break; }
     if (!d->vops) {
       g_create_error = "no FP32 viscous kernels built for p=" + std::to_string(pp) + ", q=" + std::to_string(qq);
       return DGMX_ERR_UNSUPPORTED;
@@ -1005,7 +1008,7 @@ dgmx_status create_impl(const dgmx_mesh *m, const dgmx_params *p, dgmx_domain **
                              chk(dalloc(&d->Tf[0], d->ntrace()), "alloc T0 (FP32)") &&
                              chk(dalloc(&d->Tf[1], d->ntrace()), "alloc T1 (FP32)") &&
                              chk(dalloc(&d->uref, (size_t)kUrefStride), "alloc reference state"))) &&
-            (!d->ns() || (chk(dalloc(&d->Ghat, (size_t)d->ne * (d->dim + 1) * d->dim * d->ld), "alloc gradients") &&
+            (!d->ns() || ((!d->separate_grad() || chk(d->alloc_gradients(), "alloc gradients")) &&
                           chk(dalloc(&d->Vtr, (size_t)d->nslot * d->nfaces * (d->nf - 1) * d->gf), "alloc viscous traces") &&
                           chk(dalloc(&d->Pv, (size_t)d->ne * d->nf * d->ld), "alloc viscous divergence"))) &&
             (!d->ns() || d->dim != 3 || (chk(dalloc(&d->R0, (size_t)d->ne * d->nf), "alloc hold coefficients") &&
@@ -1548,13 +1551,19 @@ dgmx_status dgmx_time_derivative_device(dgmx_domain *d, const double *U_dev, dou
   cudaSetDevice(d->prm.device);
   StageArgs a = d->base_args();
   a.Xn = U_dev; a.Fn = F_dev;
-  a.Tout = d->T[d->tcur ^ 1];
-  cudaError_t e = d->ops->traces_nodal(a, d->stream);
-  ++d->launches;
-  if (e != cudaSuccess) return d->cuda(e, "nodal trace kernel");
-  dgmx_status xs = exchange(d, fp64_halo(d->T[d->tcur ^ 1], d->nf * d->gf));
-  if (xs != DGMX_OK) return xs;
-  a.Tin = d->T[d->tcur ^ 1];
+  const KernelOps *rhs = d->visc_tc ? d->ops->tensor : d->ops;
+  cudaError_t e = cudaSuccess;
+  dgmx_status xs = DGMX_OK;
+  // the own and neighbour traces, unless the tile interpolates both itself
+  // (ghost slots of a partition hold traces only)
+  if (!rhs->self_traces || d->partitioned()) {
+    a.Tout = d->T[d->tcur ^ 1];
+    e = rhs->traces_nodal(a, d->stream);
+    ++d->launches;
+    if (e != cudaSuccess) return d->cuda(e, "nodal trace kernel");
+    if ((xs = exchange(d, fp64_halo(d->T[d->tcur ^ 1], d->nf * d->gf))) != DGMX_OK) return xs;
+    a.Tin = d->T[d->tcur ^ 1];
+  }
   if (d->prm.physics == DGMX_SHALLOW && d->prm.sw_balance) {
     if (!d->sw_captured) { a.Rcap = d->Rsw; d->sw_captured = true; }
     a.Rsub = d->Rsw;
@@ -1566,7 +1575,7 @@ dgmx_status dgmx_time_derivative_device(dgmx_domain *d, const double *U_dev, dou
     if ((xs = exchange(d, visc_halo(d))) != DGMX_OK) return xs;
   }
   a.R0 = d->hold ? d->R0 : nullptr;
-  e = (d->ns() ? d->ns_ops() : d->ops)->rhs_nodal(a, d->stream);
+  e = rhs->rhs_nodal(a, d->stream);
   ++d->launches;
   if (e != cudaSuccess) return d->cuda(e, "nodal rhs kernel");
   if (d->hold) {
@@ -1574,7 +1583,7 @@ dgmx_status dgmx_time_derivative_device(dgmx_domain *d, const double *U_dev, dou
     if ((xs = hold_stage(d, a, nullptr, F_dev)) != DGMX_OK) return xs;
   }
   // the traces of the current modal register live in T[tcur]; T[tcur^1]
-  // was used as scratch and is rewritten by the next stage.
+  // may have been used as scratch and is rewritten by the next stage.
   return DGMX_OK;
 }
 
@@ -1777,9 +1786,15 @@ dgmx_status dgmx_autotune(dgmx_domain *d, int reps, double *rows, int cap, int *
 
 dgmx_status dgmx_set_tensor_contractions(dgmx_domain *d, int on) {
   if (!d) return DGMX_ERR_ARGUMENT;
-  if (on && (!d->visc32 || !d->vops || !d->vops->ns_grad32tc))
+  if (on && (!d->visc32 || !d->ops->tensor))
     return d->fail(DGMX_ERR_UNSUPPORTED, "tensor-core contractions run in the FP32 viscous form (precision "
                                          "DGMX_MIXED) of Navier-Stokes 3-D at p >= 5");
+  cudaSetDevice(d->prm.device);
+  if (on) {
+    cudaError_t e = d->ops->tensor->init(d->tab);
+    if (e == cudaSuccess) e = d->alloc_gradients();
+    if (e != cudaSuccess) return d->cuda(e, "tensor-core form");
+  }
   d->visc_tc = on != 0;
   if (d->graph) { cudaGraphExecDestroy(d->graph); d->graph = nullptr; }
   return DGMX_OK;

@@ -36,6 +36,7 @@ struct GeomClass {
   double nrm[6][3];     // unit normal of face f in the frame of its master side
   double onrm[6][3];    // this element's own outward unit normal of face f
   double jr[6];         // side Jacobian / element Jacobian on this element's side
+  double tv[6];         // onrm[f] = tv[f] metric[r], r the face's local axis (affine elements)
   double fr[6][15];     // 3-D: face frame of nrm[f]: s (3), t (3), inverse rows (9)
   int master;           // bit f set: this element owns (is master of) face f
   int bc;               // bits 4f..4f+3: boundary type of face f (0: interior)
@@ -303,6 +304,7 @@ struct KernelOps {
   cudaError_t (*traces_modal)(const StageArgs &a, const double *Xm, void *T, cudaStream_t s) = nullptr;
   cudaError_t (*traces_nodal)(const StageArgs &a, cudaStream_t s) = nullptr;
   cudaError_t (*rhs_nodal)(const StageArgs &a, cudaStream_t s) = nullptr;
+  int self_traces = 0;                                 // rhs_nodal without a.Tin interpolates both traces itself
   cudaError_t (*forward)(const StageArgs &a, const double *Un, double *Um, cudaStream_t s) = nullptr;
   cudaError_t (*backward)(const StageArgs &a, const double *Um, double *Un, cudaStream_t s) = nullptr;
   // Navier-Stokes only: lifted gradients, then viscous traces + divergence
@@ -315,10 +317,9 @@ struct KernelOps {
   // uncapped tile of each (physics, L, Q, EPB)
   cudaError_t (*ns_grad32)(const StageArgs &a, bool nodal, cudaStream_t s) = nullptr;
   cudaError_t (*ns_visc32)(const StageArgs &a, bool nodal, cudaStream_t s) = nullptr;
-  // the FP32 viscous kernels with 3xTF32 tensor-core contractions (3-D,
-  // p >= 5)
-  cudaError_t (*ns_grad32tc)(const StageArgs &a, bool nodal, cudaStream_t s) = nullptr;
-  cudaError_t (*ns_visc32tc)(const StageArgs &a, bool nodal, cudaStream_t s) = nullptr;
+  // the tile of the 3xTF32 tensor-core form (3-D, p >= 5): its ns_grad32 and
+  // ns_visc32, and the stage and rhs_nodal that go with them
+  const KernelOps *tensor = nullptr;
 };
 void register_ops(int physics, int L, int Q, const KernelOps &ops);
 const KernelOps *find_ops(int physics, int L, int Q);            // default variant

@@ -6,8 +6,27 @@
 #include "pipeline.cuh"
 #include "form3.cuh"
 #include "stage2.cuh"
+#include "stage2d.cuh"
 
 namespace dgmx {
+
+// Launch of a kernel that calls pdl_wait (kernels.cuh), allowed to start
+// before the kernel ahead of it on the stream has drained.
+template <class... P>
+inline cudaError_t launch_dependent(void (*k)(P...), unsigned grid, int nt, size_t smem, cudaStream_t s,
+                                    const P &...a) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3((unsigned)nt);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, k, a...);
+}
 
 // Every k_*.cu is its own device module with its own copy of the __constant__
 // tables, whose host shadows have internal linkage.  The uploader must have
@@ -76,114 +95,63 @@ struct ViscPairFits<true, CV> {
                                 CV::MINB * (NsCfg<CV, float>::Visc::SMEM + 1024) <= 228 * 1024;
 };
 
-// Whether two CTAs of the FP64 gradient kernel's tile CG fit one SM.
-template <bool NS, class CG>
-struct GradPairFits {
-  static constexpr bool value = false;
-};
-template <class CG>
-struct GradPairFits<true, CG> {
-  static constexpr bool value = 2 * (NsCfg<CG, double>::Grad::SMEM + 1024) <= 228 * 1024;
-};
-
-// Whether two CTAs of the lean FP64 viscous tile CW fit one SM.
-template <bool NS, class CW>
-struct ViscLeanFits {
-  static constexpr bool value = false;
-};
-template <class CW>
-struct ViscLeanFits<true, CW> {
-  static constexpr bool value = NsCfg<CW, double>::Visc::LEAN && 2 * (NsCfg<CW, double>::Visc::SMEM + 1024) <= 228 * 1024;
-};
-
 template <int PHYS, int L, int Q, int EPB, int MINB, bool MIXED = false, int NT_ = 0>
 struct Launch {
   using C = Cfg<PHYS, L, Q, EPB, MINB, MIXED, NT_>;
-  // 3xTF32 tensor-core contractions in the FP32 viscous kernels: 3-D
-  // Navier-Stokes at p >= 5 (1-D operators of at least 7 x 7)
-  static constexpr bool kTensorViscous = PHYS == DGMX_NS3D && L >= 6;
-  // The FP32 viscous kernels' tile.  Above 512 quadrature points one thread
+  // The separate viscous kernels serve the 3xTF32 form of 3-D Navier-Stokes
+  // at p >= 5 (1-D operators of at least 7 x 7).
+  static constexpr bool kVisc32 = PHYS == DGMX_NS3D && L >= 6 && !MIXED && MINB == 0;
+  // Their tile.  Above 512 quadrature points one thread
   // per point (and its registers) leaves one CTA per SM, whose barriers then
   // idle the SM; 256 threads (about three points each) and four CTAs per SM
   // (the traces read from global memory and the lean viscous layout,
   // NsCfg::Grad::TRG and NsCfg::Visc::LEAN, ~50 KB each) let CTAs' barrier
-  // waits overlap the others' work.  At p = 7, q = 9: as fast as 384 x 3 on
-  // the CUDA cores, 15 % faster with the 3xTF32 contractions (64 registers).
+  // waits overlap the others' work (p = 7, q = 9: 15 % faster than 384 x 3).
   using CV2 = Cfg<PHYS, L, Q, EPB, 4, MIXED, 256>;
   static constexpr bool kViscPair = C::QD > 512 && EPB == 1 && ViscPairFits<is_ns(PHYS) && !MIXED, CV2>::value;
   using CV = std::conditional_t<kViscPair, CV2, C>;
-  // The FP64 gradient kernel's tile, the same way: 512 threads and two CTAs
-  // per SM (64 registers), where its shared memory without the staged traces
-  // (read from global memory instead, NsCfg::Grad::TRG) fits twice.
-  using CG2 = Cfg<PHYS, L, Q, EPB, 2, MIXED, 512>;
-  static constexpr bool kGradPair = C::QD > 512 && EPB == 1 && GradPairFits<is_ns(PHYS) && !MIXED, CG2>::value;
-  using CG = std::conditional_t<kGradPair, CG2, C>;
-  // and the FP64 viscous kernel's, with its lean layout (NsCfg::Visc::LEAN)
-  using CW2 = Cfg<PHYS, L, Q, EPB, 2, MIXED, 512>;
-  static constexpr bool kViscLean = C::QD > 512 && EPB == 1 && ViscLeanFits<is_ns(PHYS) && !MIXED, CW2>::value;
-  using CW = std::conditional_t<kViscLean, CW2, C>;
   static dim3 grid(int ne) { return dim3((unsigned)((ne + EPB - 1) / EPB)); }
   static dim3 vgrid(const StageArgs &a) { return a.vtiles ? dim3((unsigned)a.nvtiles) : grid(a.ne); }
-  static cudaError_t init(const Tables1D &t) {
+  // tables, projections and trace kernels (all that another form's tile of
+  // the same (L, Q) takes from this one)
+  static cudaError_t init_aux(const Tables1D &t) {
     cudaError_t e = upload_tables_lq<L, Q, typename C::R>(t);
     if (e != cudaSuccess) return e;
     const int sm = (int)C::SMEM;
-    if ((e = cudaFuncSetAttribute(stage_kernel<C, PHYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
     if ((e = cudaFuncSetAttribute(traces_modal_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
     if constexpr (!MIXED) {
       if ((e = cudaFuncSetAttribute(traces_nodal_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
-      if ((e = cudaFuncSetAttribute(rhs_nodal_kernel<C, PHYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
       if ((e = cudaFuncSetAttribute(forward_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
       if ((e = cudaFuncSetAttribute(backward_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
     }
-    if constexpr (is_ns(PHYS) && !MIXED) {
-      const int sg = (int)NsCfg<CG>::Grad::SMEM, sv = (int)NsCfg<CW>::Visc::SMEM;
-      if ((e = cudaFuncSetAttribute(ns_grad_kernel<CG, PHYS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sg))) return e;
-      if ((e = cudaFuncSetAttribute(ns_grad_kernel<CG, PHYS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sg))) return e;
-      if ((e = cudaFuncSetAttribute(ns_visc_kernel<CW, PHYS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sv))) return e;
-      if ((e = cudaFuncSetAttribute(ns_visc_kernel<CW, PHYS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sv))) return e;
-    }
-    if constexpr (is_ns(PHYS) && !MIXED && MINB == 0) {
-      // the FP32 viscous kernels (one set per (physics, L, Q, EPB): the
-      // uncapped tile carries them) and their FP32 tables
+    return cudaSuccess;
+  }
+  static KernelOps aux() {
+    KernelOps o;
+    o.traces_modal = traces_modal; o.traces_nodal = traces_nodal; o.forward = forward; o.backward = backward;
+    return o;
+  }
+  static cudaError_t init(const Tables1D &t) {
+    cudaError_t e = init_aux(t);
+    if (e != cudaSuccess) return e;
+    const int sm = (int)C::SMEM;
+    if ((e = cudaFuncSetAttribute(stage_kernel<C, PHYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
+    if constexpr (!MIXED)
+      if ((e = cudaFuncSetAttribute(rhs_nodal_kernel<C, PHYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm))) return e;
+    if constexpr (kVisc32) {
+      // the 3xTF32 viscous kernels and their FP32 tables
       using N = NsCfg<CV, float>;
       if ((e = upload_tables_lq<L, Q, float>(t)) != cudaSuccess) return e;
       const int sg = (int)N::Grad::SMEM, sv = (int)N::Visc::SMEM;
-      if ((e = cudaFuncSetAttribute(ns_grad_kernel<CV, PHYS, false, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, sg))) return e;
-      if ((e = cudaFuncSetAttribute(ns_grad_kernel<CV, PHYS, true, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, sg))) return e;
-      if ((e = cudaFuncSetAttribute(ns_visc_kernel<CV, PHYS, false, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, sv))) return e;
-      if ((e = cudaFuncSetAttribute(ns_visc_kernel<CV, PHYS, true, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, sv))) return e;
-      if constexpr (kTensorViscous) {
-        if ((e = cudaFuncSetAttribute(ns_grad_kernel<CV, PHYS, false, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sg))) return e;
-        if ((e = cudaFuncSetAttribute(ns_grad_kernel<CV, PHYS, true, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sg))) return e;
-        if ((e = cudaFuncSetAttribute(ns_visc_kernel<CV, PHYS, false, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sv))) return e;
-        if ((e = cudaFuncSetAttribute(ns_visc_kernel<CV, PHYS, true, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sv))) return e;
-      }
+      if ((e = cudaFuncSetAttribute(ns_grad_kernel<CV, PHYS, false, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sg))) return e;
+      if ((e = cudaFuncSetAttribute(ns_grad_kernel<CV, PHYS, true, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sg))) return e;
+      if ((e = cudaFuncSetAttribute(ns_visc_kernel<CV, PHYS, false, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sv))) return e;
+      if ((e = cudaFuncSetAttribute(ns_visc_kernel<CV, PHYS, true, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sv))) return e;
     }
     return cudaSuccess;
   }
   static cudaError_t ns_grad32(const StageArgs &a, bool nodal, cudaStream_t s) {
-    if constexpr (is_ns(PHYS) && !MIXED && MINB == 0) {
-      using N = NsCfg<CV, float>;
-      if (nodal) ns_grad_kernel<CV, PHYS, true, float><<<grid(a.ne), CV::NT, N::Grad::SMEM, s>>>(a);
-      else ns_grad_kernel<CV, PHYS, false, float><<<grid(a.ne), CV::NT, N::Grad::SMEM, s>>>(a);
-      return cudaGetLastError();
-    } else {
-      return cudaErrorNotSupported;
-    }
-  }
-  static cudaError_t ns_visc32(const StageArgs &a, bool nodal, cudaStream_t s) {
-    if constexpr (is_ns(PHYS) && !MIXED && MINB == 0) {
-      using N = NsCfg<CV, float>;
-      if (nodal) ns_visc_kernel<CV, PHYS, true, float><<<vgrid(a), CV::NT, N::Visc::SMEM, s>>>(a);
-      else ns_visc_kernel<CV, PHYS, false, float><<<vgrid(a), CV::NT, N::Visc::SMEM, s>>>(a);
-      return cudaGetLastError();
-    } else {
-      return cudaErrorNotSupported;
-    }
-  }
-  static cudaError_t ns_grad32tc(const StageArgs &a, bool nodal, cudaStream_t s) {
-    if constexpr (is_ns(PHYS) && !MIXED && MINB == 0 && kTensorViscous) {
+    if constexpr (kVisc32) {
       using N = NsCfg<CV, float>;
       if (nodal) ns_grad_kernel<CV, PHYS, true, float, true><<<grid(a.ne), CV::NT, N::Grad::SMEM, s>>>(a);
       else ns_grad_kernel<CV, PHYS, false, float, true><<<grid(a.ne), CV::NT, N::Grad::SMEM, s>>>(a);
@@ -192,31 +160,11 @@ struct Launch {
       return cudaErrorNotSupported;
     }
   }
-  static cudaError_t ns_visc32tc(const StageArgs &a, bool nodal, cudaStream_t s) {
-    if constexpr (is_ns(PHYS) && !MIXED && MINB == 0 && kTensorViscous) {
+  static cudaError_t ns_visc32(const StageArgs &a, bool nodal, cudaStream_t s) {
+    if constexpr (kVisc32) {
       using N = NsCfg<CV, float>;
       if (nodal) ns_visc_kernel<CV, PHYS, true, float, true><<<vgrid(a), CV::NT, N::Visc::SMEM, s>>>(a);
       else ns_visc_kernel<CV, PHYS, false, float, true><<<vgrid(a), CV::NT, N::Visc::SMEM, s>>>(a);
-      return cudaGetLastError();
-    } else {
-      return cudaErrorNotSupported;
-    }
-  }
-  static cudaError_t ns_grad(const StageArgs &a, bool nodal, cudaStream_t s) {
-    if constexpr (is_ns(PHYS) && !MIXED) {
-      using N = NsCfg<CG>;
-      if (nodal) ns_grad_kernel<CG, PHYS, true><<<grid(a.ne), CG::NT, N::Grad::SMEM, s>>>(a);
-      else ns_grad_kernel<CG, PHYS, false><<<grid(a.ne), CG::NT, N::Grad::SMEM, s>>>(a);
-      return cudaGetLastError();
-    } else {
-      return cudaErrorNotSupported;
-    }
-  }
-  static cudaError_t ns_visc(const StageArgs &a, bool nodal, cudaStream_t s) {
-    if constexpr (is_ns(PHYS) && !MIXED) {
-      using N = NsCfg<CW>;
-      if (nodal) ns_visc_kernel<CW, PHYS, true><<<vgrid(a), CW::NT, N::Visc::SMEM, s>>>(a);
-      else ns_visc_kernel<CW, PHYS, false><<<vgrid(a), CW::NT, N::Visc::SMEM, s>>>(a);
       return cudaGetLastError();
     } else {
       return cudaErrorNotSupported;
@@ -280,11 +228,7 @@ struct Launch {
     o.epb = EPB; o.nt = C::NT; o.smem = C::SMEM; o.minb = MINB; o.mixed = MIXED;
     o.init = init; o.stage = stage; o.traces_modal = traces_modal; o.traces_nodal = traces_nodal;
     o.rhs_nodal = rhs_nodal; o.forward = forward; o.backward = backward;
-    if constexpr (is_ns(PHYS) && !MIXED) { o.ns_grad = ns_grad; o.ns_visc = ns_visc; }
-    if constexpr (is_ns(PHYS) && !MIXED && MINB == 0) { o.ns_grad32 = ns_grad32; o.ns_visc32 = ns_visc32; }
-    if constexpr (is_ns(PHYS) && !MIXED && MINB == 0 && kTensorViscous) {
-      o.ns_grad32tc = ns_grad32tc; o.ns_visc32tc = ns_visc32tc;
-    }
+    if constexpr (kVisc32) { o.ns_grad32 = ns_grad32; o.ns_visc32 = ns_visc32; }
     return o;
   }
 };
@@ -356,12 +300,80 @@ struct PLaunch {
   }
 };
 
+// Threads of a third-form tile: about one per modal row, 64 to 256.
+constexpr int form3_threads(int L) {
+  const int t = (5 * L * L + 31) / 32 * 32;
+  return t < 64 ? 64 : (t > 256 ? 256 : t);
+}
+// CTAs per SM that smem bytes and a cap of r registers per thread allow.
+constexpr int form3_blocks(size_t smem, int nt, int r) {
+  const int per_part = 16384 / (32 * r), by_regs = per_part * 4 / ((nt + 31) / 32);
+  const int by_smem = (int)((228 * 1024) / (smem + 1024));
+  const int b = by_regs < by_smem ? by_regs : by_smem;
+  return b < 1 ? 1 : b;
+}
+
+// Euler 3-D in the third form: every stage kind, boundary sides and the
+// right-hand side on GLL values.  The projections and trace kernels come from
+// the plain tile.
+template <int PHYS, int L, int Q, bool MIXED, int NT = form3_threads(L), int REGS = MIXED ? 72 : 112>
+struct Launch3 {
+  using Base = Launch<PHYS, L, Q, default_epb(3, Q), 0, MIXED>;
+  using C0 = Cfg3<PHYS, L, Q, NT, 0, MIXED>;
+  using C = Cfg3<PHYS, L, Q, NT, form3_blocks(Stage3<C0>::SMEM, NT, REGS), MIXED>;
+  using N = Stage3<C>;
+  static cudaError_t init(const Tables1D &t) {
+    cudaError_t e = Base::init_aux(t);
+    if (e == cudaSuccess) e = upload_tables2_lq<L, Q, typename C::R>(t);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(stage3_kernel<C, PHYS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)N::SMEM);
+    if constexpr (!MIXED)
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(stage3_kernel<C, PHYS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)N::SMEM);
+    return e;
+  }
+  static cudaError_t stage_grid(const StageArgs &a, int g, cudaStream_t s) {
+    return launch_dependent(stage3_kernel<C, PHYS, false>, (unsigned)g, NT, N::SMEM, s, a);
+  }
+  static cudaError_t stage(const StageArgs &a, cudaStream_t s) { return stage_grid(a, a.ne, s); }
+  static cudaError_t rhs_nodal(const StageArgs &a, cudaStream_t s) {
+    if constexpr (!MIXED) {
+      return launch_dependent(stage3_kernel<C, PHYS, true>, (unsigned)a.ne, NT, N::SMEM, s, a);
+    } else {
+      return cudaErrorNotSupported;
+    }
+  }
+  static int blocks_per_sm() {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, stage3_kernel<C, PHYS, false>, NT, N::SMEM) != cudaSuccess) {
+      cudaGetLastError();
+      return 1;
+    }
+    return n > 0 ? n : 1;
+  }
+  static KernelOps ops() {
+    KernelOps o = Base::aux();
+    o.epb = 1; o.nt = NT; o.minb = C::MINB; o.smem = N::SMEM; o.preferred = 1; o.mixed = MIXED;
+    o.init = init; o.stage = stage; o.stage_grid = stage_grid; o.blocks_per_sm = blocks_per_sm;
+    o.rhs_nodal = rhs_nodal;
+    return o;
+  }
+};
+template <int PHYS, int P, int Q, bool MIXED = false>
+void reg3() {
+  const int key = PHYS + (MIXED ? kMixedKey : 0);
+  constexpr int NT = form3_threads(P + 1);
+  register_ops(key, P + 1, Q, Launch3<PHYS, P + 1, Q, MIXED>::ops());
+  register_ops(key, P + 1, Q, Launch3<PHYS, P + 1, Q, MIXED, NT, MIXED ? 56 : 80>::ops());
+}
+
 // The second-form stage kernel (stage2.cuh) for LSRK and right-hand-side
 // stages; other stage kinds, and every other kernel of the handle, come from
-// the plain tile of the same (L, Q).
+// the third-form tile of the same (L, Q).
 template <int PHYS, int L, int Q, int EPB, int NT, int MINB, bool MIXED = false, int VD = 0>
 struct Launch2 {
-  using Base = Launch<PHYS, L, Q, default_epb(3, Q), 0, MIXED>;
+  static_assert(EPB == 1, "the third form's tiles hold one element");
+  using Base = Launch3<PHYS, L, Q, MIXED>;
   using C = Cfg2<PHYS, L, Q, EPB, NT, MINB, MIXED, VD>;
   static cudaError_t init(const Tables1D &t) {
     cudaError_t e = Base::init(t);
@@ -379,17 +391,15 @@ struct Launch2 {
   }
   static cudaError_t stage_grid(const StageArgs &a, int g, cudaStream_t s) {
     if (a.kind != kLSRK && a.kind != kRHS) return Base::stage_grid(a, g, s);
-    stage2_kernel<C, PHYS><<<g, NT, C::SMEM, s>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(stage2_kernel<C, PHYS>, (unsigned)g, NT, C::SMEM, s, a);
   }
   static cudaError_t stage(const StageArgs &a, cudaStream_t s) {
     if (a.kind != kLSRK && a.kind != kRHS) return Base::stage(a, s);
-    stage2_kernel<C, PHYS><<<(unsigned)((a.ne + EPB - 1) / EPB), NT, C::SMEM, s>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(stage2_kernel<C, PHYS>, (unsigned)((a.ne + EPB - 1) / EPB), NT, C::SMEM, s, a);
   }
   static KernelOps ops() {
     KernelOps o = Base::ops();
-    o.epb = EPB; o.nt = NT; o.minb = MINB; o.smem = C::SMEM;
+    o.epb = EPB; o.nt = NT; o.minb = MINB; o.smem = C::SMEM; o.preferred = 0;
     o.init = init; o.stage = stage; o.stage_grid = stage_grid; o.blocks_per_sm = blocks_per_sm;
     o.warp = 3;
     return o;
@@ -450,61 +460,62 @@ void reg2() {
   if constexpr (!MIXED && B72 >= 2 && B72 != B80) reg2_variant<PHYS, P, Q, 1, NTB, B72, MIXED>();
 }
 
-// Threads of a third-form tile: about one per modal row, 64 to 256.
-constexpr int form3_threads(int L) {
-  const int t = (5 * L * L + 31) / 32 * 32;
-  return t < 64 ? 64 : (t > 256 ? 256 : t);
-}
-// CTAs per SM that smem bytes and a cap of r registers per thread allow.
-constexpr int form3_blocks(size_t smem, int nt, int r) {
-  const int per_part = 16384 / (32 * r), by_regs = per_part * 4 / ((nt + 31) / 32);
-  const int by_smem = (int)((228 * 1024) / (smem + 1024));
-  const int b = by_regs < by_smem ? by_regs : by_smem;
-  return b < 1 ? 1 : b;
-}
-
 // Navier-Stokes 3-D in the third form: ns_flux_kernel, then ns_update_kernel
 // as the stage kernel (every stage kind).  The projections and trace kernels
 // come from the plain tile.
-template <int PHYS, int L, int Q>
+//
+// Threads and register caps, measured as flux + update per stage: p = 7 (12^3)
+// flux 256 at 112 with update 256 at 64 registers 232 us, 320 at 96 248, 384
+// at 80 246, update 128 at 96 234; p = 5 (14^3) flux 256 at 80 with update 128
+// at 96 171 us, 192 at 96 187; p = 3 (16^3) flux 96 at 80 with update 64 at 96
+// 90 us, 128 at 96 92.  Above p = 3 an element has more pencils than 256
+// threads take in a round, below p = 7 smaller caps buy more CTAs per SM.
+template <int PHYS, int L, int Q, int NTF = (L < 5 ? form3_threads(L) : (L == 5 ? 160 : 256)), int RF = (L < 8 ? 80 : 112),
+          int NTU = (L < 5 ? 64 : (L < 8 ? 128 : 256)), int RU = (L < 8 ? 96 : 64)>
 struct Launch3Ns {
   using Base = Launch<PHYS, L, Q, default_epb(3, Q), 0>;
-  static constexpr int NT = form3_threads(L);
-  using C0 = Cfg3<PHYS, L, Q, NT, 0, false>;
-  using CF = Cfg3<PHYS, L, Q, NT, form3_blocks(NsFlux<C0>::SMEM, NT, 112), false>;
-  using CU = Cfg3<PHYS, L, Q, NT, form3_blocks(NsUpdate<C0>::SMEM, NT, 80), false>;
+  using C0 = Cfg3<PHYS, L, Q, 64, 0, false>;
+  using CF = Cfg3<PHYS, L, Q, NTF, form3_blocks(NsFlux<C0>::SMEM, NTF, RF), false>;
+  using CU = Cfg3<PHYS, L, Q, NTU, form3_blocks(NsUpdate<C0, false>::SMEM, NTU, RU), false>;
   using F = NsFlux<CF>;
-  using N = NsUpdate<CU>;
+  using CN = Cfg3<PHYS, L, Q, NTU, form3_blocks(NsUpdate<C0, true>::SMEM, NTU, 112), false>;
+  using N = NsUpdate<CU, false>;
+  using NN = NsUpdate<CN, true>;
   static cudaError_t init(const Tables1D &t) {
-    cudaError_t e = Base::init(t);
+    cudaError_t e = Base::init_aux(t);
     if (e == cudaSuccess) e = upload_tables2_lq<L, Q, double>(t);
+    // the FP32 viscous form's
+    if (e == cudaSuccess) e = upload_tables_lq<L, Q, float>(t);
+    if (e == cudaSuccess) e = upload_tables2_lq<L, Q, float>(t);
     auto attr = [&](auto k, size_t smem) {
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     };
-    attr(ns_flux_kernel<CF, PHYS, false>, F::SMEM);
-    attr(ns_flux_kernel<CF, PHYS, true>, F::SMEM);
+    attr(ns_flux_kernel<CF, PHYS, false, false>, F::SMEM);
+    attr(ns_flux_kernel<CF, PHYS, true, false>, F::SMEM);
+    attr(ns_flux_kernel<CF, PHYS, false, true>, F::SMEM);
+    attr(ns_flux_kernel<CF, PHYS, true, true>, F::SMEM);
     attr(ns_update_kernel<CU, PHYS, false>, N::SMEM);
-    attr(ns_update_kernel<CU, PHYS, true>, N::SMEM);
+    attr(ns_update_kernel<CN, PHYS, true>, NN::SMEM);
     return e;
   }
+  template <bool F32>
   static cudaError_t flux(const StageArgs &a, bool nodal, cudaStream_t s) {
     const unsigned g = a.vtiles ? a.nvtiles : a.ne;
-    if (nodal) ns_flux_kernel<CF, PHYS, true><<<g, NT, F::SMEM, s>>>(a);
-    else ns_flux_kernel<CF, PHYS, false><<<g, NT, F::SMEM, s>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(nodal ? ns_flux_kernel<CF, PHYS, true, F32> : ns_flux_kernel<CF, PHYS, false, F32>, g, NTF,
+                            F::SMEM, s, a);
   }
   static cudaError_t stage_grid(const StageArgs &a, int g, cudaStream_t s) {
-    ns_update_kernel<CU, PHYS, false><<<g, NT, N::SMEM, s>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(ns_update_kernel<CU, PHYS, false>, (unsigned)g, NTU, N::SMEM, s, a);
   }
-  static cudaError_t stage(const StageArgs &a, cudaStream_t s) { return stage_grid(a, a.ne, s); }
+  static cudaError_t stage(const StageArgs &a, cudaStream_t s) {
+    return stage_grid(a, a.ne, s);
+  }
   static cudaError_t rhs_nodal(const StageArgs &a, cudaStream_t s) {
-    ns_update_kernel<CU, PHYS, true><<<a.ne, NT, N::SMEM, s>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(ns_update_kernel<CN, PHYS, true>, (unsigned)a.ne, NTU, NN::SMEM, s, a);
   }
   static int blocks_per_sm() {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ns_update_kernel<CU, PHYS, false>, NT, N::SMEM) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ns_update_kernel<CU, PHYS, false>, NTU, N::SMEM) !=
         cudaSuccess) {
       cudaGetLastError();
       return 1;
@@ -512,18 +523,147 @@ struct Launch3Ns {
     return n > 0 ? n : 1;
   }
   static KernelOps ops() {
-    KernelOps o = Base::ops();
-    o.epb = 1; o.nt = NT; o.minb = CF::MINB; o.smem = F::SMEM; o.preferred = 1;
+    KernelOps o = Base::aux();
+    o.epb = 1; o.nt = NTF; o.minb = CF::MINB; o.smem = F::SMEM; o.preferred = 1;
     o.init = init; o.stage = stage; o.stage_grid = stage_grid; o.blocks_per_sm = blocks_per_sm;
     o.rhs_nodal = rhs_nodal;
-    o.ns_grad = nullptr; o.ns_visc = flux;
-    o.ns_grad32 = o.ns_visc32 = o.ns_grad32tc = o.ns_visc32tc = nullptr;
+    o.ns_grad = nullptr; o.ns_visc = flux<false>;
+    o.ns_grad32 = nullptr; o.ns_visc32 = flux<true>;
+    if constexpr (L >= 6) {
+      // 3xTF32: at q = 9 the first-form stage tile runs 512 threads (one per
+      // point, 736, would get 80 registers and spill about 1 KB each)
+      static const KernelOps tensor = Launch<PHYS, L, Q, default_epb(3, Q), 0, false, Q == 9 ? 512 : 0>::ops();
+      o.tensor = &tensor;
+    }
     return o;
   }
 };
 template <int PHYS, int P, int Q>
 void reg3_ns() {
   register_ops(PHYS, P + 1, Q, Launch3Ns<PHYS, P + 1, Q>::ops());
+  register_ops(PHYS, P + 1, Q, Launch3Ns<PHYS, P + 1, Q, (P < 4 ? 128 : 256), (P < 4 ? 96 : 112), 128, 80>::ops());
+}
+
+// Elements per CTA of a 2-D tile: about 128 modal rows.
+constexpr int stage2d_epb(int nf, int L) { return 128 / (nf * L) > 1 ? 128 / (nf * L) : 1; }
+
+// Euler 2-D and shallow water (stage2d.cuh): every stage kind, boundary sides,
+// sources and the right-hand side on GLL values.  The projections and trace
+// kernels come from the plain tile.
+template <int PHYS, int L, int Q, bool MIXED, int EPB = stage2d_epb(phys_nf(PHYS), L), int NT = 128, int MINB = 4>
+struct Launch2D {
+  using Base = Launch<PHYS, L, Q, default_epb(2, Q), 0, MIXED>;
+  using C = CfgD<PHYS, L, Q, EPB, NT, MINB, MIXED>;
+  static cudaError_t init(const Tables1D &t) {
+    cudaError_t e = Base::init_aux(t);
+    if (e == cudaSuccess) e = upload_tables2_lq<L, Q, typename C::R>(t);
+    auto attr = [&](auto k) {
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    };
+    attr(stage2d_kernel<C, PHYS>);
+    if constexpr (!MIXED) {
+      attr(rhs2d_kernel<C, PHYS, false>);
+      attr(rhs2d_kernel<C, PHYS, true>);
+    }
+    return e;
+  }
+  static cudaError_t stage_grid(const StageArgs &a, int g, cudaStream_t s) {
+    return launch_dependent(stage2d_kernel<C, PHYS>, (unsigned)g, NT, C::SMEM, s, a);
+  }
+  static cudaError_t stage(const StageArgs &a, cudaStream_t s) { return stage_grid(a, (a.ne + EPB - 1) / EPB, s); }
+  static cudaError_t rhs_nodal(const StageArgs &a, cudaStream_t s) {
+    if constexpr (!MIXED) {
+      const unsigned g = (a.ne + EPB - 1) / EPB;
+      return launch_dependent(a.Tin ? rhs2d_kernel<C, PHYS, false> : rhs2d_kernel<C, PHYS, true>, g, NT, C::SMEM, s, a);
+    } else {
+      return cudaErrorNotSupported;
+    }
+  }
+  static int blocks_per_sm() {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, stage2d_kernel<C, PHYS>, NT, C::SMEM) != cudaSuccess) {
+      cudaGetLastError();
+      return 1;
+    }
+    return n > 0 ? n : 1;
+  }
+  static KernelOps ops() {
+    KernelOps o = Base::aux();
+    o.epb = EPB; o.nt = NT; o.minb = MINB; o.smem = C::SMEM; o.mixed = MIXED; o.preferred = 1;
+    o.init = init; o.stage = stage; o.stage_grid = stage_grid; o.blocks_per_sm = blocks_per_sm;
+    o.rhs_nodal = rhs_nodal; o.self_traces = !MIXED;
+    return o;
+  }
+};
+
+// Navier-Stokes 2-D: ns2d_flux_kernel, then the face terms and update of
+// stage2d_kernel.
+template <int PHYS, int L, int Q, int EPB = stage2d_epb(4, L), int NT = 128, int MINB = 4>
+struct Launch2DNs {
+  using Base = Launch<PHYS, L, Q, default_epb(2, Q), 0>;
+  using C = CfgD<PHYS, L, Q, EPB, NT, MINB, false>;
+  using N = NsFlux2<C>;
+  static cudaError_t init(const Tables1D &t) {
+    cudaError_t e = Base::init_aux(t);
+    if (e == cudaSuccess) e = upload_tables2_lq<L, Q, double>(t);
+    // the FP32 viscous form's
+    if (e == cudaSuccess) e = upload_tables_lq<L, Q, float>(t);
+    if (e == cudaSuccess) e = upload_tables2_lq<L, Q, float>(t);
+    auto attr = [&](auto k, size_t smem) {
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    };
+    attr(ns2d_flux_kernel<C, PHYS, false, false>, N::SMEM);
+    attr(ns2d_flux_kernel<C, PHYS, true, false>, N::SMEM);
+    attr(ns2d_flux_kernel<C, PHYS, false, true>, N::SMEM);
+    attr(ns2d_flux_kernel<C, PHYS, true, true>, N::SMEM);
+    attr(stage2d_kernel<C, PHYS>, C::SMEM);
+    attr(rhs2d_kernel<C, PHYS, false>, C::SMEM);
+    return e;
+  }
+  template <bool F32>
+  static cudaError_t flux(const StageArgs &a, bool nodal, cudaStream_t s) {
+    const unsigned g = a.vtiles ? a.nvtiles : (a.ne + EPB - 1) / EPB;
+    return launch_dependent(nodal ? ns2d_flux_kernel<C, PHYS, true, F32> : ns2d_flux_kernel<C, PHYS, false, F32>, g, NT,
+                            N::SMEM, s, a);
+  }
+  static cudaError_t stage_grid(const StageArgs &a, int g, cudaStream_t s) {
+    return launch_dependent(stage2d_kernel<C, PHYS>, (unsigned)g, NT, C::SMEM, s, a);
+  }
+  static cudaError_t stage(const StageArgs &a, cudaStream_t s) { return stage_grid(a, (a.ne + EPB - 1) / EPB, s); }
+  static cudaError_t rhs_nodal(const StageArgs &a, cudaStream_t s) {
+    return launch_dependent(rhs2d_kernel<C, PHYS, false>, (unsigned)((a.ne + EPB - 1) / EPB), NT, C::SMEM, s, a);
+  }
+  static int blocks_per_sm() {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, stage2d_kernel<C, PHYS>, NT, C::SMEM) != cudaSuccess) {
+      cudaGetLastError();
+      return 1;
+    }
+    return n > 0 ? n : 1;
+  }
+  static KernelOps ops() {
+    KernelOps o = Base::aux();
+    o.epb = EPB; o.nt = NT; o.minb = MINB; o.smem = N::SMEM; o.preferred = 1;
+    o.init = init; o.stage = stage; o.stage_grid = stage_grid; o.blocks_per_sm = blocks_per_sm;
+    o.rhs_nodal = rhs_nodal;
+    o.ns_visc = flux<false>; o.ns_visc32 = flux<true>;
+    return o;
+  }
+};
+
+// 2-D tiles of one (physics, p, q): 128 threads (the default) and half of it.
+template <int PHYS, int P, int Q, bool MIXED = false>
+void reg2d() {
+  constexpr int E = stage2d_epb(phys_nf(PHYS), P + 1), B = MIXED ? 6 : 4;
+  const int key = PHYS + (MIXED ? kMixedKey : 0);
+  register_ops(key, P + 1, Q, Launch2D<PHYS, P + 1, Q, MIXED, E, 128, B>::ops());
+  register_ops(key, P + 1, Q, Launch2D<PHYS, P + 1, Q, MIXED, (E + 1) / 2, 64, 2 * B>::ops());
+}
+template <int PHYS, int P, int Q>
+void reg2d_ns() {
+  constexpr int E = stage2d_epb(4, P + 1);
+  register_ops(PHYS, P + 1, Q, Launch2DNs<PHYS, P + 1, Q, E, 128, 5>::ops());
+  register_ops(PHYS, P + 1, Q, Launch2DNs<PHYS, P + 1, Q, (E + 1) / 2, 64, 8>::ops());
 }
 
 template <int PHYS, int P, int Q, int EPB, int MINB, bool MIXED>

@@ -67,39 +67,85 @@ struct Cfg3 {
   static constexpr int NG = 15;                         // flux buffers: direction r, field n at 5 r + n
 };
 
-// Geometry of the element a CTA works on, in shared memory.
+// Links and geometry of the element a CTA works on, in shared memory.  The
+// classes are read once, coalesced: a mesh whose vertex coordinates round
+// differently has hundreds of them, more than the L1 left beside the tiles.
 struct Geo3 {
   double metric[9];
-  double tj[6];      // jump scale of face f: J_side/J_el with the sign of n . metric[r]
-  double tv[6];      // normal scale: n = tv metric[r]
+  double tv[6];      // n = tv metric[r] on face f
   double jr[6];
   double nrm[6][3], onrm[6][3];
-  int master, bc;
+  int master, bc, cls;
   FaceLink lnk[6];
 };
-__device__ __forceinline__ int face_ax(int f) { return (f == 0 || f == 5) ? 2 : ((f == 1 || f == 3) ? 1 : 0); }
 
 template <class C>
-__device__ __forceinline__ void f3_load_geo(Geo3 &g, const StageArgs &a, int e, int tid) {
-  const int cl = a.gclass[e];
-  const GeomClass *gc = a.classes + (cl >= 0 ? cl : 0);
-  if (tid < 9) g.metric[tid] = gc->metric[tid];
-  if (tid < 18) {
-    g.nrm[tid / 3][tid % 3] = gc->nrm[tid / 3][tid % 3];
-    g.onrm[tid / 3][tid % 3] = gc->onrm[tid / 3][tid % 3];
-  }
+__device__ __forceinline__ void f3_load_links(Geo3 &g, const StageArgs &a, int e, int tid) {
   if (tid < 6) {
-    const double *m = gc->metric + 3 * face_ax(tid), *n = gc->onrm[tid];
-    const double t = (n[0] * m[0] + n[1] * m[1] + n[2] * m[2]) / (m[0] * m[0] + m[1] * m[1] + m[2] * m[2]);
-    g.tv[tid] = t;
-    g.tj[tid] = t * gc->jr[tid];
-    g.jr[tid] = gc->jr[tid];
-    g.lnk[tid] = a.links[(size_t)e * 6 + tid];
+    const FaceLink lk = a.links[(size_t)e * 6 + tid];
+    g.lnk[tid] = lk;
+    if (tid == 0) g.cls = lk.cls >= 0 ? lk.cls : 0;
   }
-  if (tid == 0) { g.master = gc->master; g.bc = gc->bc; }
+}
+// after a barrier
+template <class C>
+__device__ __forceinline__ void f3_load_geo(Geo3 &g, const StageArgs &a, int tid) {
+  const GeomClass *gc = a.classes + g.cls;
+  for (int w = tid; w < 58; w += C::NT) {
+    if (w < 9) g.metric[w] = gc->metric[w];
+    else if (w < 15) g.tv[w - 9] = gc->tv[w - 9];
+    else if (w < 21) g.jr[w - 15] = gc->jr[w - 15];
+    else if (w < 39) (&g.nrm[0][0])[w - 21] = (&gc->nrm[0][0])[w - 21];
+    else if (w < 57) (&g.onrm[0][0])[w - 39] = (&gc->onrm[0][0])[w - 39];
+    else { g.master = gc->master; g.bc = gc->bc; }
+  }
+}
+
+// Asks `bytes` at p into L2 (hints: nothing is moved into the SM and nothing
+// waits).
+template <int NT>
+__device__ __forceinline__ void prefetch_span(const void *p, int bytes, int tid) {
+  for (int l = tid; l * 128 < bytes; l += NT) prefetch_l2_lines(p, bytes, l);
+}
+// The element that starts on this SM slot when this one ends: CTAs start in
+// block order, so about (SMs x CTAs per SM) further on.
+template <class C>
+__device__ __forceinline__ int element_ahead(const StageArgs &a, int e) {
+  unsigned nsm;
+  asm("mov.u32 %0, %%nsmid;" : "=r"(nsm));
+  const int n = e + (int)nsm * C::MINB;
+  return n < a.ne ? n : -1;
+}
+
+// Asks the neighbours' face blocks of `vals` values per face (Tr: [e][face])
+// into L2.
+template <class C, class T>
+__device__ __forceinline__ void prefetch_neighbours(const Geo3 &g, const T *Tr, int vals, int tid) {
+  const int lines = (vals * (int)sizeof(T) + 127) / 128;
+  for (int w = tid; w < 6 * lines; w += C::NT) {
+    const FaceLink lk = g.lnk[w / lines];
+    prefetch_l2_lines(Tr + ((size_t)lk.elem * 6 + lk.face) * vals, vals * (int)sizeof(T), w % lines);
+  }
 }
 
 // ---- pencil operators --------------------------------------------------------
+// Two FP32 values that go through the same operator: a pair fills the slot of
+// one FP64 value, so the FP32 viscous form keeps the FP64 layout (and its
+// bank pattern) with half the buffers, loads and pencils.
+struct F2 {
+  float x, y;
+  F2() = default;
+  __device__ __forceinline__ F2(float v) : x(v), y(v) {}
+  __device__ __forceinline__ F2(float a, float b) : x(a), y(b) {}
+};
+using ::fma;   // beside the overload for pairs
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) { return F2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return F2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ F2 fma(float c, F2 v, F2 a) { return F2(fmaf(c, v.x, a.x), fmaf(c, v.y, a.y)); }
+template <class T> struct CoefOf { using type = T; };
+template <> struct CoefOf<F2> { using type = float; };
+template <class T> using coef_t = typename CoefOf<T>::type;
+
 // Even-odd folding of a pencil of N values: s[i] = v[i] + v[N-1-i] (and the
 // middle value at N/2 when N is odd), d[i] = v[i] - v[N-1-i].
 template <int N, class T>
@@ -117,7 +163,7 @@ __device__ __forceinline__ void eo_project(const T (&s)[(Q + 1) / 2], const T (&
     const bool sym = (a % 2 == 0) != DER;
 #pragma unroll
     for (int i = 0; i < (sym ? (Q + 1) / 2 : Q / 2); ++i)
-      acc[a] = fma(DER ? cE2<T, L, Q>[a * Q + i] : cBw<T, L, Q>[a * Q + i], sym ? s[i] : d[i], acc[a]);
+      acc[a] = fma(DER ? cE2<coef_t<T>, L, Q>[a * Q + i] : cBw<coef_t<T>, L, Q>[a * Q + i], sym ? s[i] : d[i], acc[a]);
   }
 }
 // out[i] = sum_a B[a][i] v[a]
@@ -127,10 +173,10 @@ __device__ __forceinline__ void eo_expand(const T (&v)[L], T (&out)[Q]) {
   for (int i = 0; i < (Q + 1) / 2; ++i) {
     T e = T(0), o = T(0);
 #pragma unroll
-    for (int a = 0; a < L; a += 2) e = fma(cB<T, L, Q>[a * Q + i], v[a], e);
+    for (int a = 0; a < L; a += 2) e = fma(cB<coef_t<T>, L, Q>[a * Q + i], v[a], e);
     if (i == Q / 2) { out[i] = e; continue; }   // odd modes vanish in the middle
 #pragma unroll
-    for (int a = 1; a < L; a += 2) o = fma(cB<T, L, Q>[a * Q + i], v[a], o);
+    for (int a = 1; a < L; a += 2) o = fma(cB<coef_t<T>, L, Q>[a * Q + i], v[a], o);
     out[i] = e + o;
     out[Q - 1 - i] = e - o;
   }
@@ -300,7 +346,7 @@ __device__ __forceinline__ void f3_lift_rows(T *X, int nblk, int tid) {
     for (int b = 0; b < L; ++b) {
       T acc = T(0);
 #pragma unroll
-      for (int h = 0; h < G; ++h) acc = fma(cBwG<T, L, Q>[b * G + h], v[h], acc);
+      for (int h = 0; h < G; ++h) acc = fma(cBwG<coef_t<T>, L, Q>[b * G + h], v[h], acc);
       z[b] = acc;
     }
     st_pencil<L>(p, 1, z);
@@ -317,7 +363,7 @@ __device__ __forceinline__ void f3_lift_cols(const T *X, T *Y, int nblk, int tid
     for (int b = 0; b < L; ++b) {
       T acc = T(0);
 #pragma unroll
-      for (int g = 0; g < G; ++g) acc = fma(cBwG<T, L, Q>[b * G + g], v[g], acc);
+      for (int g = 0; g < G; ++g) acc = fma(cBwG<coef_t<T>, L, Q>[b * G + g], v[g], acc);
       z[b] = acc;
     }
     st_pencil<L>(Y + o, C::PF, z);
@@ -345,6 +391,13 @@ __device__ __forceinline__ void f3_faces(typename C::R *X, const Geo3 &g, const 
     T Uo[5], Un[5], D[5];
 #pragma unroll
     for (int k = 0; k < NF; ++k) { Uo[k] = to[k * GF]; Un[k] = tn[k * GF]; }
+    T Va[4];
+    if constexpr (is_ns(PHYS)) {
+      const T *vo = a.V + ((size_t)e * 6 + f) * (NF - 1) * GF + q;
+      const T *vn = a.V + ((size_t)lk.elem * 6 + lk.face) * (NF - 1) * GF + gn;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) Va[k] = vo[k * GF] + vn[k * GF];
+    }
     T *eo = X + f * NF * C::XLS + (q / G) * C::PF + q % G;
     const T jr = T(g.jr[f]);
     const T nm[3] = {T(g.nrm[f][0]), T(g.nrm[f][1]), T(g.nrm[f][2])};
@@ -353,8 +406,7 @@ __device__ __forceinline__ void f3_faces(typename C::R *X, const Geo3 &g, const 
       T UL[5], UR[5], FR[5];
 #pragma unroll
       for (int k = 0; k < NF; ++k) { UL[k] = master ? Uo[k] : Un[k]; UR[k] = master ? Un[k] : Uo[k]; }
-      const int cl = a.gclass[e];
-      ok = face_flux_pert<PHYS, T>(*ref, UL, UR, nm, T(a.gamma), a.flux, D, FR, a.classes[cl >= 0 ? cl : 0].fr[f]);
+      ok = face_flux_pert<PHYS, T>(*ref, UL, UR, nm, T(a.gamma), a.flux, D, FR, a.classes[g.cls].fr[f]);
 #pragma unroll
       for (int k = 0; k < NF; ++k) eo[k * C::XLS] = (master ? D[k] : FR[k] - D[k]) * jr;
     } else {
@@ -365,12 +417,9 @@ __device__ __forceinline__ void f3_faces(typename C::R *X, const Geo3 &g, const 
       for (int k = 0; k < NF; ++k) { UL[k] = master ? Uo[k] : Un[k]; UR[k] = master ? Un[k] : Uo[k]; }
       ok = face_jump_vec3<T>(UL, UR, nm, T(a.gamma), a.flux, master, D);
       if constexpr (is_ns(PHYS)) {
-        if (!bt) {
-          const double *vo = a.V + ((size_t)e * 6 + f) * (NF - 1) * GF + q;
-          const double *vn = a.V + ((size_t)lk.elem * 6 + lk.face) * (NF - 1) * GF + gn;
+        if (!bt)
 #pragma unroll
-          for (int k = 1; k < NF; ++k) D[k] = fma(0.5, vo[(k - 1) * GF] + vn[(k - 1) * GF], D[k]);
-        }
+          for (int k = 1; k < NF; ++k) D[k] = fma(0.5, Va[k - 1], D[k]);
       }
 #pragma unroll
       for (int k = 0; k < NF; ++k) eo[k * C::XLS] = D[k] * jr;
@@ -408,121 +457,107 @@ __device__ __forceinline__ void f3_add_faces(const T *XL, int nblk, int n, int a
   }
 }
 
-// ---- stage update of one modal row -----------------------------------------------
-// Every stage kind; the row of the next state that the traces are taken of
-// comes back in nx.
+// ---- stage update -----------------------------------------------------------------
+// One mode: the projected right-hand side q through stage kind `kind` from
+// the evaluated state x, u = Ut (LSRK) or U (the other kinds) and acc = A
+// (RK4); returns the next state and leaves what is stored in u and acc.
+__device__ __forceinline__ double f3_stage_value(const StageArgs &a, double dt, double q, double x, double &u,
+                                                 double &acc) {
+  switch (a.kind) {
+    case kLSRK: u = fma(-dt, q, a.c0 * u); return fma(a.c1, u, x);
+    case kTVD0: return fma(-dt, q, x);
+    case kTVD1:
+    case kTVD2: return a.kind == kTVD1 ? fma(a.c0, u, a.c1 * fma(-dt, q, x)) : fma(a.c1, fma(-dt, q, x), a.c0 * u);
+    case kRK40: acc = a.c1 * q; return fma(a.c0, q, x);
+    case kRK41: acc = fma(a.c1, q, acc); return fma(a.c0, q, u);
+    case kRK43: return fma(a.c0, fma(a.c1, q, acc), u);
+    default: acc = q; return x;   // kRHS
+  }
+}
+
+// The whole element: right-hand side rows in UB (field stride sn, planes sa,
+// rows sb), plus the volume part `vol` in global memory when given; the next
+// state, which the traces are taken of, replaces it.  Consecutive threads
+// take consecutive modes, V at a time (2 where modal blocks are even): with a
+// row per thread, 64 bytes apart, this interval took 18 k of the
+// Navier-Stokes update kernel's 47 k cycles per element at p = 7, coalesced
+// 11 k of 35 k (two groups of loads in flight per thread measured no faster).
 template <class C>
-__device__ __forceinline__ void f3_update_row(const StageArgs &a, int e, int n, int ab, const typename C::R (&Rr)[C::L],
-                                              typename C::R (&nx)[C::L]) {
-  constexpr int L = C::L;
-  const size_t gi = (((size_t)e * C::NF + n) * L * L + ab) * L;
+__device__ __forceinline__ void f3_update_all(typename C::R *UB, int sn, int sa, int sb, const double *vol,
+                                              const StageArgs &a, int e, int tid) {
+  using T = typename C::R;
+  constexpr int L = C::L, LD = C::LD, V = L % 2 == 0 ? 2 : 1, W = C::NF * LD / V;
   const double dt = a.dts ? a.dts[solve_of(a, e)] : a.dt;
-  double x[L];
-  ld_row<L>(a.X + gi, x);
-  if constexpr (C::MIXED) {
-    const double ref0 = ab == 0 ? a.uref[kUrefStride * solve_of(a, e) + 5 + n] : 0.0;
-    if (a.kind == kRHS) {
+  const size_t base = (size_t)e * C::NF * LD;
+  const bool lsrk = a.kind == kLSRK;
+  const bool need_u = a.kind != kTVD0 && a.kind != kRK40 && a.kind != kRHS;
+  const bool need_a = a.kind == kRK41 || a.kind == kRK43;
+  // where the next state and the accumulator go
+  double *dst = (lsrk || a.kind == kTVD2 || a.kind == kRK43) ? a.U : (a.kind == kRHS ? nullptr : a.Ut);
+  const bool put_a = a.kind == kRK40 || a.kind == kRK41 || a.kind == kRHS;
+  for (int w = tid; w < W; w += C::NT) {
+    const int m = w * V, n = m / LD, r = m - n * LD, ab = r / L, c = r - ab * L;
+    T *p = UB + n * sn + (ab / L) * sa + (ab % L) * sb + c;
+    const size_t gi = base + m;
+    double x[V];
+    T u[V];
+    ld_row<V>(a.X + gi, x);
+    if constexpr (C::MIXED) {
+      const double ref0 = r == 0 ? a.uref[kUrefStride * solve_of(a, e) + 5 + n] : 0.0;
+      if (lsrk) ld_row<V>(a.Utf + gi, u);
+      double un[V];
 #pragma unroll
-      for (int c = 0; c < L; ++c) { a.A[gi + c] = Rr[c]; nx[c] = float(c == 0 ? x[c] - ref0 : x[c]); }
-      return;
-    }
-    float ut[L];
-    double u[L];
-    ld_row<L>(a.Utf + gi, ut);
-    const float c0 = float(a.c0), mdt = -float(dt);
-#pragma unroll
-    for (int c = 0; c < L; ++c) {
-      ut[c] = fmaf(mdt, Rr[c], c0 * ut[c]);
-      u[c] = fma(a.c1, double(ut[c]), x[c]);
-      nx[c] = float(c == 0 ? u[c] - ref0 : u[c]);
-    }
-    st_row<L>(a.Utf + gi, ut);
-    st_row<L>(a.U + gi, u);
-  } else {
-    if (a.R0 && ab == 0) a.R0[(size_t)e * C::NF + n] = Rr[0];   // bulk-flow hold
-    if (a.kind == kLSRK) {
-      double ut[L];
-      ld_row<L>(a.Ut + gi, ut);
-#pragma unroll
-      for (int c = 0; c < L; ++c) {
-        ut[c] = fma(-dt, Rr[c], a.c0 * ut[c]);
-        nx[c] = fma(a.c1, ut[c], x[c]);
+      for (int k = 0; k < V; ++k) {
+        const float q = p[k];
+        if (lsrk) {
+          u[k] = fmaf(-float(dt), q, float(a.c0) * u[k]);
+          un[k] = fma(a.c1, double(u[k]), x[k]);
+        } else {
+          a.A[gi + k] = q;
+          un[k] = x[k];
+        }
+        p[k] = float(k == 0 ? un[k] - ref0 : un[k]);
       }
-      st_row<L>(a.Ut + gi, ut);
-      st_row<L>(a.U + gi, nx);
-      return;
-    }
-    double u[L], acc[L];
-    switch (a.kind) {
-      case kTVD0:
+      if (lsrk) { st_row<V>(a.Utf + gi, u); st_row<V>(a.U + gi, un); }
+    } else {
+      double acc[V], v[V], nx[V];
+      if (need_u) ld_row<V>((lsrk ? a.Ut : a.U) + gi, u);
+      if (vol) ld_row<V>(vol + gi, v);
+      if (need_a) ld_row<V>(a.A + gi, acc);
 #pragma unroll
-        for (int c = 0; c < L; ++c) nx[c] = fma(-dt, Rr[c], x[c]);
-        st_row<L>(a.Ut + gi, nx);
-        break;
-      case kTVD1:
-        ld_row<L>(a.U + gi, u);
-#pragma unroll
-        for (int c = 0; c < L; ++c) nx[c] = fma(a.c0, u[c], a.c1 * fma(-dt, Rr[c], x[c]));
-        st_row<L>(a.Ut + gi, nx);
-        break;
-      case kTVD2:
-        ld_row<L>(a.U + gi, u);
-#pragma unroll
-        for (int c = 0; c < L; ++c) nx[c] = fma(a.c1, fma(-dt, Rr[c], x[c]), a.c0 * u[c]);
-        st_row<L>(a.U + gi, nx);
-        break;
-      case kRK40:
-#pragma unroll
-        for (int c = 0; c < L; ++c) { nx[c] = fma(a.c0, Rr[c], x[c]); acc[c] = a.c1 * Rr[c]; }
-        st_row<L>(a.Ut + gi, nx);
-        st_row<L>(a.A + gi, acc);
-        break;
-      case kRK41:
-        ld_row<L>(a.U + gi, u);
-        ld_row<L>(a.A + gi, acc);
-#pragma unroll
-        for (int c = 0; c < L; ++c) { nx[c] = fma(a.c0, Rr[c], u[c]); acc[c] = fma(a.c1, Rr[c], acc[c]); }
-        st_row<L>(a.Ut + gi, nx);
-        st_row<L>(a.A + gi, acc);
-        break;
-      case kRK43:
-        ld_row<L>(a.U + gi, u);
-        ld_row<L>(a.A + gi, acc);
-#pragma unroll
-        for (int c = 0; c < L; ++c) nx[c] = fma(a.c0, fma(a.c1, Rr[c], acc[c]), u[c]);
-        st_row<L>(a.U + gi, nx);
-        break;
-      default:   // kRHS
-#pragma unroll
-        for (int c = 0; c < L; ++c) { acc[c] = Rr[c]; nx[c] = x[c]; }
-        st_row<L>(a.A + gi, acc);
-        break;
+      for (int k = 0; k < V; ++k) {
+        const double q = vol ? p[k] + v[k] : p[k];
+        if (a.R0 && r + k == 0) a.R0[(size_t)e * C::NF + n] = q;   // bulk-flow hold
+        nx[k] = f3_stage_value(a, dt, q, x[k], u[k], acc[k]);
+        p[k] = nx[k];
+      }
+      if (lsrk) st_row<V>(a.Ut + gi, u);
+      if (dst) st_row<V>(dst + gi, nx);
+      if (put_a) st_row<V>(a.A + gi, acc);
     }
   }
 }
 
 // ---- next traces --------------------------------------------------------------------
-// The next modal rows sit in buffers UB (rows of pitch SJ, planes of SI);
-// their end values along c were written by the update.  Ends along b (faces
-// 1, 3) and a (faces 4, 2) -> FP [f][n][a'][b'], rows of PL.
+// End values of the next modal block (field stride sn, planes sa, rows sb)
+// along a (faces 4, 2), b (1, 3) and c (0, 5) -> FP [f][n][a'][b'].
 template <class C, class T>
-__device__ __forceinline__ void f3_ends(const T *UB, T *FP, int tid) {
+__device__ __forceinline__ void f3_ends(const T *UB, int sn, int sa, int sb, T *FP, int tid) {
   constexpr int NF = C::NF, L = C::L, Q = C::Q, PL = C::PL, N = NF * L * L, PB = NF * C::FPS;
-  for (int w = tid; w < 2 * N; w += C::NT) {
+  for (int w = tid; w < 3 * N; w += C::NT) {
     const int ax = w / N, r = w - ax * N, n = r / (L * L), xy = r - n * L * L, x = xy / L, y = xy - x * L;
+    const T *p = UB + n * sn + (ax == 0 ? x * sb + y : (ax == 1 ? x * sa + y : x * sa + y * sb));
+    const int st = ax == 0 ? sa : (ax == 1 ? sb : 1);
     T lo = T(0), hi = T(0);
-    const T *ub = UB + n * C::BS;
-    T *fp = FP + n * C::FPS + x * PL + y;
-    const T *p = ax == 0 ? ub + x * C::SI + y : ub + x * C::SJ + y;
-    const int st = ax == 0 ? C::SJ : C::SI;
 #pragma unroll
     for (int b = 0; b < L; ++b) {
       const T v = p[b * st];
       lo = fma(cEnd<T, L, Q>[b], v, lo);
       hi = fma(cEnd<T, L, Q>[L + b], v, hi);
     }
-    fp[(ax == 0 ? 1 : 4) * PB] = lo;
-    fp[(ax == 0 ? 3 : 2) * PB] = hi;
+    T *fp = FP + n * C::FPS + x * PL + y;
+    fp[(ax == 0 ? 4 : (ax == 1 ? 1 : 0)) * PB] = lo;
+    fp[(ax == 0 ? 2 : (ax == 1 ? 3 : 5)) * PB] = hi;
   }
 }
 // W1[f][n][g][b'] = sum_a' Bg[a'][g] FP[f][n][a'][b'], then the trace rows.
@@ -559,21 +594,6 @@ __device__ __forceinline__ void f3_traces_b(const T *W1, T *Tout, int e, int tid
     st_row<G>(Tout + (size_t)e * C::NFACE * C::NF * C::GF + w * G, out);
   }
 }
-// End values along c of one next row: faces 0 and 5.
-template <class C, class T>
-__device__ __forceinline__ void f3_ends_c(const T (&nx)[C::L], T *FP, int n, int aa, int bb) {
-  constexpr int L = C::L, Q = C::Q;
-  T f0 = T(0), f5 = T(0);
-#pragma unroll
-  for (int c = 0; c < L; ++c) {
-    f0 = fma(cEnd<T, L, Q>[c], nx[c], f0);
-    f5 = fma(cEnd<T, L, Q>[L + c], nx[c], f5);
-  }
-  T *fp = FP + n * C::FPS + aa * C::PL + bb;
-  fp[0] = f0;
-  fp[5 * C::NF * C::FPS] = f5;
-}
-
 // GLL values from modal rows already expanded along k and j, to Field layout.
 template <class C>
 __device__ __forceinline__ void f3_store_nodal(const double *buf, const StageArgs &a, int e, int tid) {
@@ -588,6 +608,148 @@ __device__ __forceinline__ void f3_store_nodal(const double *buf, const StageArg
   });
 }
 
+// ---------------------------------------------------------------------- Euler
+// Contravariant fluxes G_r = metric[r] . F(U) at the points: state buffers
+// 0..4 -> flux buffers 5 r + n, in place point by point.  The mixed form
+// evaluates F(Ub + u') - F(Ub) (volume_flux_pert, kernels.cuh).
+template <class C>
+__device__ __forceinline__ void f3_point_fluxes(typename C::R *G, const Geo3 &g, const RefState<typename C::R> *ref,
+                                                const StageArgs &a, int tid) {
+  using T = typename C::R;
+  constexpr int Q = C::Q, BS = C::BS;
+  const T gm1 = T(a.gamma) - T(1.0);
+  T m[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) m[k] = T(g.metric[k]);
+  for (int w = tid; w < Q * Q * Q; w += C::NT) {
+    const int i = w / (Q * Q), jk = w - i * Q * Q, j = jk / Q, k = jk - j * Q;
+    T *p = G + i * C::SI + j * C::SJ + k;
+    T U[5];
+#pragma unroll
+    for (int n = 0; n < 5; ++n) U[n] = p[n * BS];
+    if constexpr (C::MIXED) {
+      const RefState<T> &b = *ref;
+      const T ir = p_rcp(b.r + U[0]);
+      const T mx = b.m[0] + U[1], my = b.m[1] + U[2], mz = b.m[2] + U[3];
+      const T ux = (U[1] - b.u[0] * U[0]) * ir, uy = (U[2] - b.u[1] * U[0]) * ir, uz = (U[3] - b.u[2] * U[0]) * ir;
+      T sd = T(0);
+      sd = fma(U[1], b.u[0], sd); sd = fma(mx, ux, sd);
+      sd = fma(U[2], b.u[1], sd); sd = fma(my, uy, sd);
+      sd = fma(U[3], b.u[2], sd); sd = fma(mz, uz, sd);
+      const T pp = gm1 * fma(T(-0.5), sd, U[4]);
+      const T Hp = U[4] + pp, H = b.H + Hp;
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const T m0 = m[3 * r], m1 = m[3 * r + 1], m2 = m[3 * r + 2];
+        const T Vb = m0 * b.u[0] + m1 * b.u[1] + m2 * b.u[2], Vp = m0 * ux + m1 * uy + m2 * uz;
+        T *o = p + 5 * r * BS;
+        o[0] = m0 * U[1] + m1 * U[2] + m2 * U[3];
+        o[BS] = fma(U[1], Vb, fma(mx, Vp, pp * m0));
+        o[2 * BS] = fma(U[2], Vb, fma(my, Vp, pp * m1));
+        o[3 * BS] = fma(U[3], Vb, fma(mz, Vp, pp * m2));
+        o[4 * BS] = fma(Hp, Vb, H * Vp);
+      }
+    } else {
+      const T ir = T(1.0) / U[0];
+      const T u = U[1] * ir, v = U[2] * ir, ww = U[3] * ir;
+      const T pr = gm1 * fma(T(-0.5), fma(U[3], ww, fma(U[2], v, U[1] * u)), U[4]);
+      const T Ep = U[4] + pr;
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        const T m0 = m[3 * r], m1 = m[3 * r + 1], m2 = m[3 * r + 2];
+        const T V = fma(m2, ww, fma(m1, v, m0 * u));
+        T *o = p + 5 * r * BS;
+        o[0] = U[0] * V;
+        o[BS] = fma(U[1], V, pr * m0);
+        o[2 * BS] = fma(U[2], V, pr * m1);
+        o[3 * BS] = fma(U[3], V, pr * m2);
+        o[4 * BS] = Ep * V;
+      }
+    }
+  }
+}
+
+// One fused stage (or, NODAL, one right-hand side on GLL values): 15 flux
+// buffers and the face terms in shared memory.  The right-hand side rows go
+// back to buffers 0..4, whose rows the k pass has just read; the end planes
+// FP take the place of the face terms, the traces' first pass W1 buffers 5...
+template <class C>
+struct Stage3 {
+  static constexpr int O_X = C::NG * C::BS;
+  static constexpr size_t DATA = ((size_t)(O_X + C::S_XL) * sizeof(typename C::R) + 15) / 16 * 16;
+  static constexpr size_t SMEM = DATA + (sizeof(Geo3) + 15) / 16 * 16 + (C::MIXED ? sizeof(RefState<float>) : 0);
+  static_assert(C::S_FP <= C::S_XL && C::S_W1 <= 10 * C::BS, "end planes and trace rows fit the dead regions");
+};
+template <class C, int PHYS, bool NODAL>
+__global__ void __launch_bounds__(C::NT, C::MINB) stage3_kernel(StageArgs a) {
+  using T = typename C::R;
+  using N = Stage3<C>;
+  constexpr int L = C::L, BS = C::BS, SI = C::SI, SJ = C::SJ, GF = C::GF;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T *U = reinterpret_cast<T *>(smem_raw), *X = U + N::O_X, *W1 = U + 5 * BS;
+  Geo3 &g = *reinterpret_cast<Geo3 *>(smem_raw + N::DATA);
+  RefState<T> *ref = reinterpret_cast<RefState<T> *>(smem_raw + N::DATA + (sizeof(Geo3) + 15) / 16 * 16);
+  const int tid = threadIdx.x;
+  pdl_release();
+  const int ntile = a.tiles ? *a.ntiles : a.ne;
+  for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
+    const int e = a.tiles ? a.tiles[t] : t;
+    if (t != (int)blockIdx.x) __syncthreads();
+    f3_load_links<C>(g, a, e, tid);
+    pdl_wait();
+    if constexpr (C::MIXED) {
+      if (tid == 0) *ref = *reinterpret_cast<const RefState<T> *>(a.uref + kUrefStride * solve_of(a, e) + 10);
+    }
+    if constexpr (NODAL) f3_state_nodal<C>(U, a, e, tid); else f3_state_k<C>(U, a, e, tid);
+    if (const int n = element_ahead<C>(a, e); n >= 0 && !a.tiles) {
+      if constexpr (!NODAL) prefetch_span<C::NT>(a.X + (size_t)n * 5 * C::LD, 5 * C::LD * 8, tid);
+      prefetch_span<C::NT>(trace_in<C>(a) + (size_t)n * 30 * GF, 30 * GF * (int)sizeof(T), tid);
+    }
+    __syncthreads();
+    f3_load_geo<C>(g, a, tid);
+    prefetch_neighbours<C>(g, trace_in<C>(a), 5 * GF, tid);
+    if constexpr (!NODAL) f3_expand_j<C>(U, 5, tid);
+    __syncthreads();
+    f3_faces<C, PHYS>(X, g, ref, a, e, tid);
+    if constexpr (!NODAL) f3_expand_i<C>(U, 5, tid);
+    __syncthreads();
+    f3_lift_rows<C>(X, 30, tid);
+    f3_point_fluxes<C>(U, g, ref, a, tid);
+    __syncthreads();
+    f3_lift_cols<C>(X, X, 30, tid);
+    f3_div_i<C>(U, tid);
+    __syncthreads();
+    f3_div_j<C>(U, tid);
+    __syncthreads();
+    pencils_k<C>(5, tid, [&](int n, int o, int aa, int bb) {
+      T R[L];
+      f3_div_k_row<C>(U, n, o, R);
+      f3_add_faces<C>(X, 5, n, aa, bb, R);
+      if constexpr (NODAL) {
+        T v[C::Q];
+        eo_expand<L, C::Q>(R, v);
+        st_pencil<C::Q>(U + n * BS + o, 1, v);
+      } else {
+        st_pencil<L>(U + n * BS + o, 1, R);
+      }
+    });
+    __syncthreads();
+    if constexpr (NODAL) {
+      f3_expand_j<C>(U, 5, tid);
+      __syncthreads();
+      f3_store_nodal<C>(U, a, e, tid);
+    } else {
+      f3_update_all<C>(U, BS, SI, SJ, nullptr, a, e, tid);
+      __syncthreads();
+      f3_ends<C>(U, BS, SI, SJ, X, tid);
+      __syncthreads();
+      f3_traces_a<C>(X, W1, tid);
+      __syncthreads();
+      f3_traces_b<C>(W1, trace_out<C>(a), e, tid);
+    }
+  }
+}
+
 // ------------------------------------------------------------------ Navier-Stokes
 // Shared memory of ns_flux_kernel: 15 buffers, [0, 5) the primitive state
 // (density, velocity, internal energy), [5, 15) the gradient work W; then all
@@ -600,7 +762,6 @@ struct NsFlux {
   static constexpr int O_W = 5 * C::BS, O_X = 15 * C::BS;
   static constexpr size_t DATA = (size_t)(15 * C::BS + S_X) * sizeof(double);
   static constexpr size_t SMEM = DATA + (sizeof(Geo3) + 15) / 16 * 16;
-  static_assert(24 * C::XLS <= 10 * C::BS, "the jumps fit the work buffers");
   // the energy gradient's first pass takes the part of X whose jumps
   // (velocity) are consumed by then as one more scratch buffer
   static_assert(18 * C::XLS >= (C::L - 1) * C::SI + C::Q * C::SJ, "scratch buffer of the energy gradient");
@@ -608,7 +769,9 @@ struct NsFlux {
 
 // (q_own + q_nbr)/2 - q_own of the primitive variables at the side Gauss
 // points, times the face's jump scale, into blocks [c][f].
-template <class C>
+// FP32 form: formed in FP64, then rounded, components in pairs (u, v), (w, e)
+// in blocks [pair][f].
+template <class C, bool F32>
 __device__ __forceinline__ void ns3_jumps(double *J, const Geo3 &g, const StageArgs &a, int e, int tid) {
   constexpr int NF = C::NF, GF = C::GF, G = C::G;
   for (int w = tid; w < 6 * GF; w += C::NT) {
@@ -623,19 +786,24 @@ __device__ __forceinline__ void ns3_jumps(double *J, const Geo3 &g, const StageA
     if (bt) ghost_state<3, NF>(a.bckind[bt], a.bcpar[bt], Uo, g.onrm[f], true, Un);
     primitive<3>(Uo, qo);
     primitive<3>(Un, qn);
-    double *o = J + f * C::XLS + (q / G) * C::PF + q % G;
-    const double t = 0.5 * g.tj[f];
+    const int o = f * C::XLS + (q / G) * C::PF + q % G;
+    const double t = 0.5 * g.tv[f] * g.jr[f];
+    if constexpr (F32) {
+      F2 *J2 = reinterpret_cast<F2 *>(J) + o;
+      J2[0] = F2(float(t * (qn[0] - qo[0])), float(t * (qn[1] - qo[1])));
+      J2[6 * C::XLS] = F2(float(t * (qn[2] - qo[2])), float(t * (qn[3] - qo[3])));
+    } else {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) o[c * 6 * C::XLS] = t * (qn[c] - qo[c]);
+      for (int c = 0; c < 4; ++c) J[o + c * 6 * C::XLS] = t * (qn[c] - qo[c]);
+    }
   }
 }
 
 // Gradient passes of one scalar: i pass, v -> (E_i v, P_i v).
-template <class C>
-__device__ __forceinline__ void ns3_grad_i(const double *q, double *de, double *pr) {
+template <class C, class T>
+__device__ __forceinline__ void ns3_grad_i(const T (&v)[C::Q], T *de, T *pr) {
   constexpr int L = C::L, Q = C::Q;
-  double v[Q], s[(Q + 1) / 2], d[Q / 2], o[L];
-  ld_pencil<Q>(q, C::SI, v);
+  T s[(Q + 1) / 2], d[Q / 2], o[L];
   eo_fold<Q>(v, s, d);
   zero<L>(o);
   eo_project<L, Q, true>(s, d, o);
@@ -645,10 +813,10 @@ __device__ __forceinline__ void ns3_grad_i(const double *q, double *de, double *
   st_pencil<L>(pr, C::SI, o);
 }
 // j pass: (E_i v, P_i v) -> (P_j E_i v, E_j P_i v, P_j P_i v)
-template <class C>
-__device__ __forceinline__ void ns3_grad_j(const double *de, const double *pr, double *o0, double *o1, double *o2) {
+template <class C, class T>
+__device__ __forceinline__ void ns3_grad_j(const T *de, const T *pr, T *o0, T *o1, T *o2) {
   constexpr int L = C::L, Q = C::Q;
-  double v[Q], s[(Q + 1) / 2], d[Q / 2], o[L];
+  T v[Q], s[(Q + 1) / 2], d[Q / 2], o[L];
   ld_pencil<Q>(de, C::SJ, v);
   eo_fold<Q>(v, s, d);
   zero<L>(o);
@@ -665,11 +833,12 @@ __device__ __forceinline__ void ns3_grad_j(const double *de, const double *pr, d
 }
 // k pass of row (a, b): the projected derivatives along the local axes with
 // the lifted jumps, then the chain rule: z[d] = sum_r metric[r][d] Z_r, in z.
-template <class C>
-__device__ __forceinline__ void ns3_grad_k(const double *w0, const double *X, const double *met, int aa, int bb,
-                                           double (&z)[3][C::L]) {
+template <class C, class T>
+__device__ __forceinline__ void ns3_grad_k(const T *w0, const T *X, const double *met, int aa, int bb,
+                                           T (&z)[3][C::L]) {
   constexpr int L = C::L, Q = C::Q, PF = C::PF, XLS = C::XLS;
-  double v[Q], s[(Q + 1) / 2], d[Q / 2];
+  using K = coef_t<T>;
+  T v[Q], s[(Q + 1) / 2], d[Q / 2];
 #pragma unroll
   for (int r = 0; r < 3; ++r) {
     ld_pencil<Q>(w0 + r * C::BS, 1, v);
@@ -677,25 +846,32 @@ __device__ __forceinline__ void ns3_grad_k(const double *w0, const double *X, co
     zero<L>(z[r]);
     if (r == 2) eo_project<L, Q, true>(s, d, z[r]); else eo_project<L, Q, false>(s, d, z[r]);
   }
-  const double xk0 = X[aa * PF + bb], xk1 = X[5 * XLS + aa * PF + bb];
-  const double *xj0 = X + XLS + aa * PF, *xj1 = X + 3 * XLS + aa * PF;
-  const double *xi0 = X + 4 * XLS + bb * PF, *xi1 = X + 2 * XLS + bb * PF;
-  const double eb0 = end_value<double, L, Q>(0, bb), eb1 = end_value<double, L, Q>(1, bb);
-  const double ea0 = end_value<double, L, Q>(0, aa), ea1 = end_value<double, L, Q>(1, aa);
+  const T xk0 = X[aa * PF + bb], xk1 = X[5 * XLS + aa * PF + bb];
+  const T *xj0 = X + XLS + aa * PF, *xj1 = X + 3 * XLS + aa * PF;
+  const T *xi0 = X + 4 * XLS + bb * PF, *xi1 = X + 2 * XLS + bb * PF;
+  const K eb0 = end_value<K, L, Q>(0, bb), eb1 = end_value<K, L, Q>(1, bb);
+  const K ea0 = end_value<K, L, Q>(0, aa), ea1 = end_value<K, L, Q>(1, aa);
+  K m[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) m[k] = K(met[k]);
 #pragma unroll
   for (int c = 0; c < L; ++c) {
-    const double z0 = fma(ea1, xi1[c], fma(ea0, xi0[c], z[0][c]));
-    const double z1 = fma(eb1, xj1[c], fma(eb0, xj0[c], z[1][c]));
-    const double z2 = fma(cEnd<double, L, Q>[L + c], xk1, fma(cEnd<double, L, Q>[c], xk0, z[2][c]));
+    const T z0 = fma(ea1, xi1[c], fma(ea0, xi0[c], z[0][c]));
+    const T z1 = fma(eb1, xj1[c], fma(eb0, xj0[c], z[1][c]));
+    const T z2 = fma(cEnd<K, L, Q>[L + c], xk1, fma(cEnd<K, L, Q>[c], xk0, z[2][c]));
 #pragma unroll
-    for (int k = 0; k < 3; ++k) z[k][c] = fma(met[6 + k], z2, fma(met[3 + k], z1, met[k] * z0));
+    for (int k = 0; k < 3; ++k) z[k][c] = fma(m[6 + k], z2, fma(m[3 + k], z1, fma(m[k], z0, T(0))));
   }
 }
 
 // One element: state, projected gradients, stresses, volume flux, its
 // projected divergence (a.Pv, [e][n][L^3]) and the viscous normal-flux
-// traces (a.V).  NODAL: the state comes from GLL values (a.Xn).
-template <class C, int PHYS, bool NODAL>
+// traces (a.V).  NODAL: the state comes from GLL values (a.Xn).  F32: the
+// gradients and stresses in FP32 (precision = DGMX_MIXED); the primitive
+// variables are formed in FP64 and rounded, the internal energy as its
+// difference from the element's first point (a constant the gradient does
+// not see: e ~ 1/(gamma (gamma-1) Ma^2) against variations of O(1)).
+template <class C, int PHYS, bool NODAL, bool F32>
 __global__ void __launch_bounds__(C::NT, C::MINB) ns_flux_kernel(StageArgs a) {
   using N = NsFlux<C>;
   constexpr int L = C::L, Q = C::Q, G = C::G, GF = C::GF, BS = C::BS, SI = C::SI, SJ = C::SJ, NT = C::NT;
@@ -703,17 +879,25 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns_flux_kernel(StageArgs a) {
   double *U = reinterpret_cast<double *>(smem_raw), *W = U + N::O_W, *X = U + N::O_X;
   Geo3 &g = *reinterpret_cast<Geo3 *>(smem_raw + N::DATA);
   const int tid = threadIdx.x, e = a.vtiles ? a.vtiles[blockIdx.x] : (int)blockIdx.x;
-  f3_load_geo<C>(g, a, e, tid);
-  __syncthreads();
+  // links and geometry arrive behind the state's first passes
+  pdl_release();
+  f3_load_links<C>(g, a, e, tid);
+  pdl_wait();
   if constexpr (NODAL) f3_state_nodal<C>(U, a, e, tid); else f3_state_k<C>(U, a, e, tid);
-  ns3_jumps<C>(W, g, a, e, tid);
+  if (const int n = element_ahead<C>(a, e); n >= 0) {
+    if constexpr (!NODAL) prefetch_span<NT>(a.X + (size_t)n * 5 * C::LD, 5 * C::LD * 8, tid);
+    prefetch_span<NT>(a.Tin + (size_t)n * 30 * GF, 30 * GF * 8, tid);
+  }
   __syncthreads();
+  f3_load_geo<C>(g, a, tid);
+  prefetch_neighbours<C>(g, a.Tin, 5 * GF, tid);
   if constexpr (!NODAL) f3_expand_j<C>(U, 5, tid);
-  f3_lift_rows<C>(W, 24, tid);
   __syncthreads();
+  ns3_jumps<C, F32>(X, g, a, e, tid);
   if constexpr (!NODAL) f3_expand_i<C>(U, 5, tid);
-  f3_lift_cols<C>(W, X, 24, tid);
   __syncthreads();
+  if constexpr (F32) f3_lift_rows<C>(reinterpret_cast<F2 *>(X), 12, tid);
+  else f3_lift_rows<C>(X, 24, tid);
   // density, velocity, internal energy in place
   for (int w = tid; w < Q * Q * Q; w += NT) {
     const int i = w / (Q * Q), jk = w - i * Q * Q, j = jk / Q, k = jk - j * Q;
@@ -728,63 +912,122 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns_flux_kernel(StageArgs a) {
     for (int n = 0; n < 4; ++n) p[(n + 1) * BS] = q[n];
   }
   __syncthreads();
-  // velocity gradient: component c in W[3c .. 3c+2]
-  pencils_i<C>(3, tid, [&](int c, int jk) {
-    ns3_grad_i<C>(U + (1 + c) * BS + jk, W + 3 * c * BS + jk, W + (3 * c + 1) * BS + jk);
-  });
-  __syncthreads();
-  pencils_j<C>(3, tid, [&](int c, int o, int, int) {
-    double *w = W + 3 * c * BS + o;
-    ns3_grad_j<C>(w, w + BS, w, w + BS, w + 2 * BS);
-  });
-  __syncthreads();
-  pencils_k<C>(3, tid, [&](int c, int o, int aa, int bb) {
-    double *w = W + 3 * c * BS + o;
-    double z[3][L];
-    ns3_grad_k<C>(w, X + c * 6 * C::XLS, g.metric, aa, bb, z);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) st_pencil<L>(w + d * BS, 1, z[d]);
-  });
-  __syncthreads();
-  // stresses (modal, linear in the gradient) into W[0..5]; the energy
-  // gradient's i pass into W[9] and the velocity jumps' part of X
-  double *A0 = X;
-  for (int w = tid; w < L * L * L; w += NT) {
-    const int i = w / (L * L), jk = w - i * L * L, j = jk / L, k = jk - j * L;
-    double *p = W + i * SI + j * SJ + k;
-    double t[6];
-    viscous_stress<3, double>(p, BS, a.vis, t);
-#pragma unroll
-    for (int n = 0; n < 6; ++n) p[n * BS] = t[n];
-  }
-  pencils_i<C>(1, tid, [&](int, int jk) { ns3_grad_i<C>(U + 4 * BS + jk, W + 9 * BS + jk, A0 + jk); });
-  __syncthreads();
-  pencils_j<C>(1, tid, [&](int, int o, int, int) {
-    double *w = W + 6 * BS + o;
-    ns3_grad_j<C>(W + 9 * BS + o, A0 + o, w, w + BS, w + 2 * BS);
-  });
-  f3_expand_k<C>(W, 6, tid);
-  __syncthreads();
   const double kap = a.gamma / a.Pr * a.vis;
-  pencils_k<C>(1, tid, [&](int, int o, int aa, int bb) {
-    double *w = W + 6 * BS + o;
-    double z[3][L], u[Q];
-    ns3_grad_k<C>(w, X + 18 * C::XLS, g.metric, aa, bb, z);
+  if constexpr (F32) {
+    F2 *W2 = reinterpret_cast<F2 *>(W), *X2 = reinterpret_cast<F2 *>(X);
+    f3_lift_cols<C>(X2, X2, 12, tid);
+    // gradient of the pairs (u, v) and (w, e), pair c in W2[3c .. 3c+2]
+    const double eref = U[4 * BS];
+    pencils_i<C>(2, tid, [&](int c, int jk) {
+      F2 v[Q];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
+      for (int i = 0; i < Q; ++i) {
+        const double *p = U + (1 + 2 * c) * BS + jk + i * SI;
+        v[i] = F2(float(p[0]), float(c == 0 ? p[BS] : p[BS] - eref));
+      }
+      ns3_grad_i<C>(v, W2 + 3 * c * BS + jk, W2 + (3 * c + 1) * BS + jk);
+    });
+    __syncthreads();
+    pencils_j<C>(2, tid, [&](int c, int o, int, int) {
+      F2 *w = W2 + 3 * c * BS + o;
+      ns3_grad_j<C>(w, w + BS, w, w + BS, w + 2 * BS);
+    });
+    __syncthreads();
+    pencils_k<C>(2, tid, [&](int c, int o, int aa, int bb) {
+      F2 *w = W2 + 3 * c * BS + o;
+      F2 z[3][L];
+      ns3_grad_k<C>(w, X2 + c * 6 * C::XLS, g.metric, aa, bb, z);
 #pragma unroll
-      for (int c = 0; c < L; ++c) z[d][c] *= kap;
-      eo_expand<L, Q>(z[d], u);
-      st_pencil<Q>(w + d * BS, 1, u);
+      for (int d = 0; d < 3; ++d) st_pencil<L>(w + d * BS, 1, z[d]);
+    });
+    __syncthreads();
+    // stresses and heat flux (modal) as pairs (t11, t12), (t13, t22),
+    // (t23, t33), (hx, hy), (hz, 0)
+    for (int w = tid; w < L * L * L; w += NT) {
+      const int i = w / (L * L), jk = w - i * L * L, j = jk / L, k = jk - j * L;
+      F2 *p = W2 + i * SI + j * SJ + k;
+      F2 q[6];
+#pragma unroll
+      for (int n = 0; n < 6; ++n) q[n] = p[n * BS];
+      const float gr[9] = {q[0].x, q[1].x, q[2].x, q[0].y, q[1].y, q[2].y, q[3].x, q[4].x, q[5].x};
+      const float kf = float(kap);
+      float t[6];
+      viscous_stress<3, float>(gr, 1, float(a.vis), t);
+      p[0] = F2(t[0], t[1]); p[BS] = F2(t[2], t[3]); p[2 * BS] = F2(t[4], t[5]);
+      p[3 * BS] = F2(kf * q[3].y, kf * q[4].y); p[4 * BS] = F2(kf * q[5].y, 0.0f);
     }
-  });
-  f3_expand_j<C>(W, 6, tid);
-  __syncthreads();
-  f3_expand_j<C>(W + 6 * BS, 3, tid);
-  f3_expand_i<C>(W, 6, tid);
-  __syncthreads();
-  f3_expand_i<C>(W + 6 * BS, 3, tid);
-  __syncthreads();
+    __syncthreads();
+    f3_expand_k<C>(W2, 5, tid);
+    __syncthreads();
+    f3_expand_j<C>(W2, 5, tid);
+    __syncthreads();
+    f3_expand_i<C>(W2, 5, tid);
+    __syncthreads();
+  } else {
+    f3_lift_cols<C>(X, X, 24, tid);
+    // velocity gradient: component c in W[3c .. 3c+2]
+    pencils_i<C>(3, tid, [&](int c, int jk) {
+      double v[Q];
+      ld_pencil<Q>(U + (1 + c) * BS + jk, SI, v);
+      ns3_grad_i<C>(v, W + 3 * c * BS + jk, W + (3 * c + 1) * BS + jk);
+    });
+    __syncthreads();
+    pencils_j<C>(3, tid, [&](int c, int o, int, int) {
+      double *w = W + 3 * c * BS + o;
+      ns3_grad_j<C>(w, w + BS, w, w + BS, w + 2 * BS);
+    });
+    __syncthreads();
+    pencils_k<C>(3, tid, [&](int c, int o, int aa, int bb) {
+      double *w = W + 3 * c * BS + o;
+      double z[3][L];
+      ns3_grad_k<C>(w, X + c * 6 * C::XLS, g.metric, aa, bb, z);
+  #pragma unroll
+      for (int d = 0; d < 3; ++d) st_pencil<L>(w + d * BS, 1, z[d]);
+    });
+    __syncthreads();
+    // stresses (modal, linear in the gradient) into W[0..5]; the energy
+    // gradient's i pass into W[9] and the velocity jumps' part of X
+    double *A0 = X;
+    for (int w = tid; w < L * L * L; w += NT) {
+      const int i = w / (L * L), jk = w - i * L * L, j = jk / L, k = jk - j * L;
+      double *p = W + i * SI + j * SJ + k;
+      double t[6];
+      viscous_stress<3, double>(p, BS, a.vis, t);
+  #pragma unroll
+      for (int n = 0; n < 6; ++n) p[n * BS] = t[n];
+    }
+    pencils_i<C>(1, tid, [&](int, int jk) {
+      double v[Q];
+      ld_pencil<Q>(U + 4 * BS + jk, SI, v);
+      ns3_grad_i<C>(v, W + 9 * BS + jk, A0 + jk);
+    });
+    __syncthreads();
+    pencils_j<C>(1, tid, [&](int, int o, int, int) {
+      double *w = W + 6 * BS + o;
+      ns3_grad_j<C>(W + 9 * BS + o, A0 + o, w, w + BS, w + 2 * BS);
+    });
+    f3_expand_k<C>(W, 6, tid);
+    __syncthreads();
+    pencils_k<C>(1, tid, [&](int, int o, int aa, int bb) {
+      double *w = W + 6 * BS + o;
+      double z[3][L], u[Q];
+      ns3_grad_k<C>(w, X + 18 * C::XLS, g.metric, aa, bb, z);
+  #pragma unroll
+      for (int d = 0; d < 3; ++d) {
+  #pragma unroll
+        for (int c = 0; c < L; ++c) z[d][c] *= kap;
+        eo_expand<L, Q>(z[d], u);
+        st_pencil<Q>(w + d * BS, 1, u);
+      }
+    });
+    f3_expand_j<C>(W, 6, tid);
+    __syncthreads();
+    f3_expand_j<C>(W + 6 * BS, 3, tid);
+    f3_expand_i<C>(W, 6, tid);
+    __syncthreads();
+    f3_expand_i<C>(W + 6 * BS, 3, tid);
+    __syncthreads();
+  }
   // contravariant flux G_r = metric[r] . (F(U) - g) at the points, and the
   // viscous normal flux g . n on the face points
   {
@@ -796,11 +1039,23 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns_flux_kernel(StageArgs a) {
       const int i = w / (Q * Q), jk = w - i * Q * Q, j = jk / Q, k = jk - j * Q;
       double *p = U + i * SI + j * SJ + k;
       const double rho = p[0], u = p[BS], v = p[2 * BS], ww = p[3 * BS], ei = p[4 * BS];
-      const double *t = p + 5 * BS;
-      const double t11 = t[0], t12 = t[BS], t13 = t[2 * BS], t22 = t[3 * BS], t23 = t[4 * BS], t33 = t[5 * BS];
-      const double qx = fma(t13, ww, fma(t12, v, fma(t11, u, t[6 * BS])));
-      const double qy = fma(t23, ww, fma(t22, v, fma(t12, u, t[7 * BS])));
-      const double qz = fma(t33, ww, fma(t23, v, fma(t13, u, t[8 * BS])));
+      double t[9];   // t11, t12, t13, t22, t23, t33, heat flux
+      if constexpr (F32) {
+        const F2 *q = reinterpret_cast<const F2 *>(p + 5 * BS);
+#pragma unroll
+        for (int n = 0; n < 5; ++n) {
+          const F2 z = q[n * BS];
+          t[2 * n] = z.x;
+          if (n < 4) t[2 * n + 1] = z.y;
+        }
+      } else {
+#pragma unroll
+        for (int n = 0; n < 9; ++n) t[n] = p[(5 + n) * BS];
+      }
+      const double t11 = t[0], t12 = t[1], t13 = t[2], t22 = t[3], t23 = t[4], t33 = t[5];
+      const double qx = fma(t13, ww, fma(t12, v, fma(t11, u, t[6])));
+      const double qy = fma(t23, ww, fma(t22, v, fma(t12, u, t[7])));
+      const double qz = fma(t33, ww, fma(t23, v, fma(t13, u, t[8])));
       const double pr = gm1 * rho * ei;
       const double H = fma(rho, fma(0.5, fma(ww, ww, fma(v, v, u * u)), ei), pr);   // E + p
 #pragma unroll
@@ -867,25 +1122,42 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns_flux_kernel(StageArgs a) {
 // Face terms (inviscid and viscous) of one element, the stage update from
 // the volume part ns_flux_kernel left in a.Pv, and the next traces.  NODAL:
 // the projected right-hand side goes to GLL values (a.Fn) instead.
-template <class C>
+// Shared memory: the right-hand side and then the next state UB, whose place
+// the traces' first pass W1 takes; the face terms XL, whose place the end
+// planes FP take.
+template <class C, bool NODAL>
 struct NsUpdate {
-  static constexpr int O_X = 5 * C::BS, S_X = cmax(C::S_XL, C::S_W1), O_FP = O_X + S_X;   // W1 follows XL
-  static constexpr size_t DATA = (size_t)(O_FP + C::S_FP) * sizeof(double);
+  static constexpr int SB = NODAL ? C::SJ : C::PL, SA = NODAL ? C::SI : C::L * C::PL;
+  static constexpr int SN = NODAL ? C::BS : C::L * C::L * C::PL;
+  static constexpr int S_UB = cmax(5 * SN, C::S_W1), O_X = S_UB, S_X = cmax(C::S_XL, C::S_FP);
+  static constexpr size_t DATA = (size_t)(O_X + S_X) * sizeof(double);
   static constexpr size_t SMEM = DATA + (sizeof(Geo3) + 15) / 16 * 16;
 };
 template <class C, int PHYS, bool NODAL>
 __global__ void __launch_bounds__(C::NT, C::MINB) ns_update_kernel(StageArgs a) {
-  using N = NsUpdate<C>;
-  constexpr int L = C::L;
+  using N = NsUpdate<C, NODAL>;
+  constexpr int L = C::L, GF = C::GF;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double *UB = reinterpret_cast<double *>(smem_raw), *X = UB + N::O_X, *FP = UB + N::O_FP;
+  double *UB = reinterpret_cast<double *>(smem_raw), *X = UB + N::O_X;
   Geo3 &g = *reinterpret_cast<Geo3 *>(smem_raw + N::DATA);
   const int tid = threadIdx.x;
-  const int ntile = a.tiles ? *a.ntiles : (int)gridDim.x;
+  pdl_release();
+  const int ntile = a.tiles ? *a.ntiles : a.ne;
   for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
     const int e = a.tiles ? a.tiles[t] : t;
     if (t != (int)blockIdx.x) __syncthreads();
-    f3_load_geo<C>(g, a, e, tid);
+    f3_load_links<C>(g, a, e, tid);
+    pdl_wait();
+    // read five intervals on
+    prefetch_span<C::NT>(a.Pv + (size_t)e * 5 * C::LD, 5 * C::LD * 8, tid);
+    if constexpr (!NODAL) {
+      prefetch_span<C::NT>(a.X + (size_t)e * 5 * C::LD, 5 * C::LD * 8, tid);
+      prefetch_span<C::NT>(a.Ut + (size_t)e * 5 * C::LD, 5 * C::LD * 8, tid);
+    }
+    __syncthreads();
+    f3_load_geo<C>(g, a, tid);
+    prefetch_neighbours<C>(g, a.Tin, 5 * GF, tid);
+    prefetch_neighbours<C>(g, a.V, 4 * GF, tid);
     __syncthreads();
     f3_faces<C, PHYS>(X, g, nullptr, a, e, tid);
     __syncthreads();
@@ -893,32 +1165,35 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns_update_kernel(StageArgs a) 
     __syncthreads();
     f3_lift_cols<C>(X, X, 30, tid);
     __syncthreads();
-    pencils_k<C>(5, tid, [&](int n, int o, int aa, int bb) {
-      double R[L], nx[L];
-      ld_row<L>(a.Pv + ((((size_t)e * 5 + n) * L + aa) * L + bb) * L, R);
+    for (int w = tid; w < 5 * L * L; w += C::NT) {
+      const int n = w / (L * L), ab = w - n * L * L, aa = ab / L, bb = ab - aa * L;
+      double R[L];
+      zero<L>(R);
+      if constexpr (NODAL) ld_row<L>(a.Pv + ((size_t)e * 5 * L * L + w) * L, R);
       f3_add_faces<C>(X, 5, n, aa, bb, R);
+      double *u = UB + n * N::SN + aa * N::SA + bb * N::SB;
       if constexpr (NODAL) {
-        if (a.R0 && aa == 0 && bb == 0) a.R0[(size_t)e * 5 + n] = R[0];
-        double u[C::Q];
-        eo_expand<L, C::Q>(R, u);
-        st_pencil<C::Q>(UB + n * C::BS + o, 1, u);
+        if (a.R0 && ab == 0) a.R0[(size_t)e * 5 + n] = R[0];
+        double v[C::Q];
+        eo_expand<L, C::Q>(R, v);
+        st_pencil<C::Q>(u, 1, v);
       } else {
-        f3_update_row<C>(a, e, n, aa * L + bb, R, nx);
-        st_pencil<L>(UB + n * C::BS + o, 1, nx);
-        f3_ends_c<C>(nx, FP, n, aa, bb);
+        st_pencil<L>(u, 1, R);
       }
-    });
+    }
     __syncthreads();
     if constexpr (NODAL) {
       f3_expand_j<C>(UB, 5, tid);
       __syncthreads();
       f3_store_nodal<C>(UB, a, e, tid);
     } else {
-      f3_ends<C>(UB, FP, tid);
+      f3_update_all<C>(UB, N::SN, N::SA, N::SB, a.Pv, a, e, tid);
       __syncthreads();
-      f3_traces_a<C>(FP, X, tid);
+      f3_ends<C>(UB, N::SN, N::SA, N::SB, X, tid);
       __syncthreads();
-      f3_traces_b<C>(X, a.Tout, e, tid);
+      f3_traces_a<C>(X, UB, tid);
+      __syncthreads();
+      f3_traces_b<C>(UB, a.Tout, e, tid);
     }
   }
 }

@@ -5,7 +5,7 @@
 // stage.  Here the 2-D arenas (Euler 2-D and shallow water, p = 1..7,
 // q = p + 2) share ONE launch per LSRK stage: the kernel walks a device-side
 // list of (arena, tile) work items and runs, for each, the fused stage body
-// (stage_tile, stage.cuh) compiled for that arena's (physics, p, q) at a
+// (stage2d_tile, stage2d.cuh) compiled for that arena's (physics, p, q) at a
 // common launch shape of 128 threads per CTA.  The body of a work item is a
 // CTA-uniform branch, so a launch mixes orders freely; per element the
 // arithmetic is that of the body alone (each pencil's operations and their
@@ -19,16 +19,15 @@ namespace dgmx {
 
 constexpr int kFusedBodies = 14;   // Euler 2-D p = 1..7, shallow water p = 1..7
 constexpr int kFusedThreads = 128;
-// CTAs per SM the register allocation is held to (the bodies of the largest
-// orders spill a little at this cap; the small orders gain the occupancy)
-constexpr int kFusedMinBlocks64 = 7, kFusedMinBlocksMixed = 8;
+// CTAs per SM the register allocation is held to
+constexpr int kFusedMinBlocks64 = 4, kFusedMinBlocksMixed = 5;
 
 template <bool MIXED, int B>
 struct FusedCfg {
   static constexpr int PHYS = B < 7 ? DGMX_EULER2D : DGMX_SHALLOW;
   static constexpr int P = B % 7 + 1, L = P + 1, Q = P + 2;
-  static constexpr int EPB = default_epb(2, Q);
-  using C = Cfg<PHYS, L, Q, EPB, 0, MIXED, kFusedThreads>;
+  static constexpr int EPB = stage2d_epb(phys_nf(PHYS), L);
+  using C = CfgD<PHYS, L, Q, EPB, kFusedThreads, 0, MIXED>;
 };
 
 template <bool MIXED, int B = 0>
@@ -47,8 +46,8 @@ __device__ __forceinline__ void fused_dispatch(int body, unsigned char *raw, con
   if constexpr (B < kFusedBodies) {
     if (body == B) {
       using F = FusedCfg<MIXED, B>;
-      Smem<typename F::C> sm(raw);
-      stage_tile<typename F::C, F::PHYS>(sm, a, tile * F::EPB, tid);
+      SmemD<typename F::C> sm(raw);
+      stage2d_tile<typename F::C, F::PHYS>(sm, a, tile * F::EPB, tid);
     } else {
       fused_dispatch<MIXED, B + 1>(body, raw, a, tile, tid);
     }
@@ -62,6 +61,7 @@ __global__ void __launch_bounds__(kFusedThreads, MIXED ? kFusedMinBlocksMixed : 
                                                                        const int *bodies, const int2 *items,
                                                                        const int *nitems, int stage) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pdl_release();
   const int n = *nitems;
   for (int t = blockIdx.x; t < n; t += gridDim.x) {
     if (t != (int)blockIdx.x) __syncthreads();
@@ -76,7 +76,9 @@ template <bool MIXED, int B = 0>
 static cudaError_t fused_upload() {
   if constexpr (B < 7) {
     using F = FusedCfg<MIXED, B>;
-    const cudaError_t e = upload_tables_lq<F::L, F::Q, typename F::C::R>(make_tables(F::L, F::Q, F::Q - 1));
+    const Tables1D t = make_tables(F::L, F::Q, F::Q - 1);
+    cudaError_t e = upload_tables_lq<F::L, F::Q, typename F::C::R>(t);
+    if (e == cudaSuccess) e = upload_tables2_lq<F::L, F::Q, typename F::C::R>(t);
     if (e != cudaSuccess) return e;
     return fused_upload<MIXED, B + 1>();
   } else {
@@ -109,9 +111,8 @@ struct FusedHost {
   }
   static cudaError_t launch(const StageArgs *args, int narena, const int *bodies, const int2 *items,
                             const int *nitems, int stage, int grid, cudaStream_t s) {
-    fused_stage_kernel<MIXED><<<grid, kFusedThreads, fused_smem<MIXED>(), s>>>(args, narena, bodies, items,
-                                                                               nitems, stage);
-    return cudaGetLastError();
+    return launch_dependent(fused_stage_kernel<MIXED>, (unsigned)grid, kFusedThreads, fused_smem<MIXED>(), s, args,
+                            narena, bodies, items, nitems, stage);
   }
 };
 

@@ -9,6 +9,15 @@
 
 namespace dgmx {
 
+// Programmatic dependent launch.  A stage's kernel may be launched while the
+// one before it on the stream still runs (launch_dependent below): it lets the
+// next one in when all its blocks have started (pdl_release), and reads what
+// earlier kernels wrote only after pdl_wait, which returns once they have
+// completed and their stores are visible.  Between the two it may read mesh
+// data, which no kernel writes.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 template <int B, int E>
 struct Pow { static constexpr int v = B * Pow<B, E - 1>::v; };
 template <int B>

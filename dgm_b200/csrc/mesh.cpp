@@ -272,6 +272,10 @@ bool build_mesh(const dgmx_mesh &m, const Tables1D &t, HostMesh &out, std::strin
       for (int k = 0; k < 3; ++k) c.nrm[s][k] = n[k];
       for (int k = 0; k < 3; ++k) c.onrm[s][k] = geo[e].nrm[s][k];
       c.jr[s] = geo[e].jr[s];
+      // local axis of side s: 3-D 0,5 -> k, 1,3 -> j, 2,4 -> i; 2-D 0,2 -> j, 1,3 -> i
+      const int ax = dim == 3 ? (s == 0 || s == 5 ? 2 : (s == 1 || s == 3 ? 1 : 0)) : (s % 2 == 0 ? 1 : 0);
+      const double *mt = c.metric + 3 * ax, *on = c.onrm[s];
+      c.tv[s] = (on[0] * mt[0] + on[1] * mt[1] + on[2] * mt[2]) / (mt[0] * mt[0] + mt[1] * mt[1] + mt[2] * mt[2]);
       if (dim == 3) face_frame(c.nrm[s], c.fr[s]);
       if (S.master) c.master |= 1 << s;
     }

@@ -788,6 +788,7 @@ __device__ __forceinline__ void s2_prefetch(const StageArgs &a, int tile, int ne
 template <class C, int PHYS>
 __device__ __forceinline__ void stage2_tile(const Smem2<C> &sm, const StageArgs &a, int e0, int tid) {
   s2_load<C>(sm, a, e0, tid);
+  pdl_wait();
   __syncthreads();
   s2_interval1<C, PHYS>(sm, a, e0, tid);
   __syncthreads();
@@ -814,6 +815,7 @@ template <class C, int PHYS>
 __global__ void __launch_bounds__(C::NT, C::MINB) stage2_kernel(StageArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem2<C> sm(smem_raw);
+  pdl_release();
   const int ntile = a.tiles ? *a.ntiles : (int)gridDim.x;
   // One tile per CTA: the CTAs resident at once are about (SMs x CTAs per SM)
   // and start in block order, so the tile that many blocks ahead starts

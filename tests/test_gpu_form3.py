@@ -43,3 +43,94 @@ def test_navier_stokes_3d_every_order(p, q, inttype):
     D.advance(dt, 2)
     assert rel(D.state(), P.state()) < 1e-12
     D.close()
+
+
+@pytest.mark.parametrize("inttype", [14, 4, 3])
+@pytest.mark.parametrize("flux", ["laxfriedrichs", "roe"])
+@pytest.mark.parametrize("p,q", ORDERS)
+def test_euler_3d_every_order(p, q, flux, inttype):
+    """The third-form stage tile (the default) and the right-hand side on
+    GLL values."""
+    import dgm_b200
+    n = (3, 2, 2) if p < 6 else (2, 1, 2)
+    m = rotated_box(3, n, 0.0, 2 * np.pi, p, q, seed=p)
+    P = oracle.Problem(m, oracle.EULER3D, flux=flux)
+    D = dgm_b200.Domain(m, dgm_b200.EULER3D, flux=flux, inttype=inttype)
+    x, y, z = P.coords()
+    f = ics.taylor_green(x, y, z, Ma=0.3)
+    U0 = P.project(f)   # at q = p+1 projecting twice is not projecting once
+    F_o, F_g = P.rhs(U0), D.time_derivative(U0)
+    scale = np.sqrt((F_o ** 2).sum()) + np.sqrt((U0 ** 2).sum())
+    assert np.sqrt(((F_g - F_o) ** 2).sum()) / scale < 1e-12
+    P.set_state(U0)
+    D.set_state(f)
+    dt = 0.02 / (p + 1) ** 2
+    assert P.advance(inttype, dt, 2) == 0
+    D.advance(dt, 2)
+    assert rel(D.state(), P.state()) < 1e-12
+    D.close()
+
+
+ORDERS_2D = [(p, q) for p in range(1, 9) for q in (p + 1, p + 2)]
+
+
+@pytest.mark.parametrize("phys", ["euler2d", "ns2d", "shallow"])
+@pytest.mark.parametrize("inttype", [14, 4, 3])
+@pytest.mark.parametrize("p,q", ORDERS_2D)
+def test_2d_every_order(p, q, inttype, phys):
+    """Every 2-D tile on a ragged, randomly rotated mesh (more elements than
+    one CTA holds, not a multiple of it), and the right-hand side on GLL
+    values (one launch, traces interpolated in it)."""
+    import dgm_b200
+    code = {"euler2d": 1, "ns2d": 2, "shallow": 30}[phys]
+    m = rotated_box(2, (7, 5), -5.0, 5.0, p, q, seed=p)
+    flux, vis = ("laxfriedrichs", 0.0) if phys == "shallow" else ("roe", 0.02 if phys == "ns2d" else 0.0)
+    P = oracle.Problem(m, code, flux=flux, vis=vis)
+    if phys == "shallow":
+        P.set_sw_balance(False)
+    x, y, _ = P.coords()
+    f = ics.gaussian_bump(x, y, w=2.0) if phys == "shallow" else ics.isentropic_vortex(x, y, beta=2.0, period=(10.0, 10.0))
+    U0 = P.project(f)
+    dt = 0.01 / (p + 1) ** 2
+    F_o = P.rhs(U0)
+    P.set_state(U0)
+    assert P.advance(inttype, dt, 2) == 0
+    D = dgm_b200.Domain(m, code, flux=flux, inttype=inttype, vis=vis, sw_balance=False)
+    scale = np.sqrt((F_o ** 2).sum()) + np.sqrt((U0 ** 2).sum())
+    for k in range(D.variant_count()):
+        D.set_variant(k)
+        assert np.sqrt(((D.time_derivative(U0) - F_o) ** 2).sum()) / scale < 1e-12
+        D.set_state(f)
+        D.advance(dt, 2)
+        assert rel(D.state(), P.state()) < 1e-12
+    D.close()
+
+
+@pytest.mark.parametrize("phys,p", [("euler2d", 1), ("euler2d", 4), ("euler2d", 8), ("shallow", 3), ("shallow", 8),
+                                    ("euler3d", 1), ("euler3d", 4), ("euler3d", 7)])
+def test_mixed_form_every_tile(phys, p):
+    """The FP32 form of the same tiles: 1e-6 of the FP64 oracle, the bar of
+    the mixed form's other tests."""
+    import dgm_b200
+    code, dim = {"euler2d": (1, 2), "shallow": (30, 2), "euler3d": (8, 3)}[phys]
+    n = (7, 5) if dim == 2 else (3, 2, 2)
+    lo, hi = (-5.0, 5.0) if dim == 2 else (0.0, 2 * np.pi)
+    m = rotated_box(dim, n, lo, hi, p, 0, seed=p)
+    flux = "laxfriedrichs" if phys == "shallow" else "roe"
+    P = oracle.Problem(m, code, flux=flux)
+    if phys == "shallow":
+        P.set_sw_balance(False)
+    x, y, z = P.coords()
+    f = (ics.gaussian_bump(x, y, w=2.0) if phys == "shallow" else
+         ics.isentropic_vortex(x, y, beta=2.0, period=(10.0, 10.0)) if dim == 2 else ics.taylor_green(x, y, z, Ma=0.3))
+    U0 = P.project(f)
+    dt = 0.01 / (p + 1) ** 2
+    P.set_state(U0)
+    assert P.advance(14, dt, 2) == 0
+    D = dgm_b200.Domain(m, code, flux=flux, precision=dgm_b200.MIXED, sw_balance=False)
+    for k in range(D.variant_count()):
+        D.set_variant(k)
+        D.set_state(f)
+        D.advance(dt, 2)
+        assert rel(D.state(), P.state()) < 1e-6
+    D.close()
