@@ -917,7 +917,8 @@ dgmx_status create_impl(const dgmx_mesh *m, const dgmx_params *p, dgmx_domain **
       return DGMX_ERR_UNSUPPORTED;
     }
   }
-  d->ops = find_ops(phys, pp + 1, qq);
+  const bool plain = bspec && !bspec->sides.empty();
+  d->ops = default_ops(phys, pp + 1, qq, m->ne, plain);
   if (d->visc32) {
     if (const std::vector<KernelOps> *vs = find_variants(phys, pp + 1, qq))
       for (const KernelOps &o : *vs)
@@ -928,7 +929,7 @@ dgmx_status create_impl(const dgmx_mesh *m, const dgmx_params *p, dgmx_domain **
     }
   }
   if (d->ops && d->prm.precision == DGMX_MIXED) {
-    d->ops_m = find_ops(phys + kMixedKey, pp + 1, qq);
+    d->ops_m = default_ops(phys + kMixedKey, pp + 1, qq, m->ne, plain);
     if (!d->ops_m) {
       g_create_error = "no mixed-precision kernels built for p=" + std::to_string(pp) + ", q=" + std::to_string(qq);
       return DGMX_ERR_UNSUPPORTED;

@@ -293,7 +293,10 @@ constexpr int kMixedKey = 1000;
 struct KernelOps {
   int epb = 0, nt = 0, minb = 0, mixed = 0;
   int warp = 0;                                        // kind: 0 CTA tile, 2 prefetching persistent kernel
-  int preferred = 0;                                   // the default tile of its (physics, L, Q) when set
+  // default choice (default_ops): the tile preferred most, except that one
+  // with small >= elements goes first (a mesh that one wave of its CTAs holds
+  // gains from more threads and registers per element, not from occupancy)
+  int preferred = 0, small = 0;
   size_t smem = 0;
   cudaError_t (*init)(const Tables1D &t) = nullptr;   // tables + smem attributes, current device
   cudaError_t (*stage)(const StageArgs &a, cudaStream_t s) = nullptr;
@@ -322,7 +325,9 @@ struct KernelOps {
   const KernelOps *tensor = nullptr;
 };
 void register_ops(int physics, int L, int Q, const KernelOps &ops);
-const KernelOps *find_ops(int physics, int L, int Q);            // default variant
+// The default tile for a mesh of ne elements; plain: one that handles
+// boundary sides (kind 0).
+const KernelOps *default_ops(int physics, int L, int Q, int ne, bool plain);
 const std::vector<KernelOps> *find_variants(int physics, int L, int Q);
 void list_ops(std::vector<std::vector<int>> &out);
 

@@ -379,7 +379,20 @@ struct Launch2 {
     cudaError_t e = Base::init(t);
     if (e != cudaSuccess) return e;
     if ((e = upload_tables2_lq<L, Q, typename C::R>(t)) != cudaSuccess) return e;
+    if constexpr (NODAL2)
+      if ((e = cudaFuncSetAttribute(rhs2_kernel<C, PHYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM)) != cudaSuccess)
+        return e;
     return cudaFuncSetAttribute(stage2_kernel<C, PHYS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+  }
+  // right-hand side on GLL values in this form where its stage is the default
+  static constexpr bool NODAL2 = !MIXED && L <= 5 && (5 * L * L <= NT);
+  static cudaError_t rhs_nodal(const StageArgs &a, cudaStream_t s) {
+    if constexpr (NODAL2) {
+      rhs2_kernel<C, PHYS><<<(unsigned)a.ne, NT, C::SMEM, s>>>(a);
+      return cudaGetLastError();
+    } else {
+      return cudaErrorNotSupported;
+    }
   }
   static int blocks_per_sm() {
     int n = 0;
@@ -400,6 +413,7 @@ struct Launch2 {
   static KernelOps ops() {
     KernelOps o = Base::ops();
     o.epb = EPB; o.nt = NT; o.minb = MINB; o.smem = C::SMEM; o.preferred = 0;
+    if constexpr (NODAL2) o.rhs_nodal = rhs_nodal;
     o.init = init; o.stage = stage; o.stage_grid = stage_grid; o.blocks_per_sm = blocks_per_sm;
     o.warp = 3;
     return o;
@@ -407,11 +421,16 @@ struct Launch2 {
 };
 
 template <int PHYS, int P, int Q, int EPB, int NT, int MINB, bool MIXED, int VD = 0>
-void reg2_variant() {
+void reg2_variant(int preferred = 0, int small = 0) {
   using C = Cfg2<PHYS, P + 1, Q, EPB, NT, MINB, MIXED, VD>;
   if constexpr (C::SMEM <= 227 * 1024 && (MINB == 0 || (65536 / (NT * MINB) >= 40 &&
                                                         (int)((228 * 1024) / (C::SMEM + 1024)) >= MINB)))
-    register_ops(PHYS + (MIXED ? kMixedKey : 0), P + 1, Q, Launch2<PHYS, P + 1, Q, EPB, NT, MINB, MIXED, VD>::ops());
+  {
+    KernelOps o = Launch2<PHYS, P + 1, Q, EPB, NT, MINB, MIXED, VD>::ops();
+    o.preferred = preferred;
+    o.small = small;
+    register_ops(PHYS + (MIXED ? kMixedKey : 0), P + 1, Q, o);
+  }
 }
 
 // CTAs per SM of NT threads that a cap of R registers per thread allows: a
@@ -441,11 +460,16 @@ void reg2() {
   constexpr int B96 = blocks_for_regs<CB>(NTB, 96), B80 = blocks_for_regs<CB>(NTB, 80);
   constexpr int B64 = blocks_for_regs<CB>(NTB, 64), A64 = blocks_for_regs<CA>(NTA, 64);
   reg2_variant<PHYS, P, Q, 1, NTA, 0, MIXED>();
-  reg2_variant<PHYS, P, Q, 1, NTB, 0, MIXED>();
-  if constexpr (B96 >= 2) reg2_variant<PHYS, P, Q, 1, NTB, B96, MIXED>();
+  // up to p = 4 the default (p = 3, 32^3: FP64 260 us against the third form's
+  // 315, FP32 201 against 215; p = 2, 20^3: 39 against 54; above, the third
+  // form's tile is faster); a mesh of one wave takes the uncapped tile (p = 3,
+  // 8^3: 7.4 us against 11 to 12 for the capped ones)
+  constexpr int PREF = P <= 4 ? 2 : 0, ONE_WAVE = P <= 4 ? 4 * 148 : 0;
+  reg2_variant<PHYS, P, Q, 1, NTB, 0, MIXED>(0, MIXED ? 0 : ONE_WAVE);
+  if constexpr (B96 >= 2) reg2_variant<PHYS, P, Q, 1, NTB, B96, MIXED>(0, MIXED ? ONE_WAVE : 0);
   if constexpr (A96 >= 2) reg2_variant<PHYS, P, Q, 1, NTA, A96, MIXED>();
   if constexpr (B80 >= 2 && B80 != B96) reg2_variant<PHYS, P, Q, 1, NTB, B80, MIXED>();
-  if constexpr (A80 >= 2 && A80 != A96) reg2_variant<PHYS, P, Q, 1, NTA, A80, MIXED>();
+  if constexpr (A80 >= 2 && A80 != A96) reg2_variant<PHYS, P, Q, 1, NTA, A80, MIXED>(MIXED ? 0 : PREF);
   if constexpr (MIXED && B64 >= 2 && B64 != B80) reg2_variant<PHYS, P, Q, 1, NTB, B64, MIXED>();
   // FP32 with the volume's three directions spread over three warps
   if constexpr (MIXED && A80 >= 2) reg2_variant<PHYS, P, Q, 1, NTA, A80, MIXED, 1>();
@@ -453,7 +477,7 @@ void reg2() {
   if constexpr (MIXED && A64 >= 2 && A64 != A80) reg2_variant<PHYS, P, Q, 1, NTA, A64, MIXED, 1>();
   constexpr int A56 = blocks_for_regs<CA>(NTA, 56);
   if constexpr (MIXED && B64 >= 2 && B64 != B80) reg2_variant<PHYS, P, Q, 1, NTB, B64, MIXED, 1>();
-  if constexpr (MIXED && A56 >= 2 && A56 != A64) reg2_variant<PHYS, P, Q, 1, NTA, A56, MIXED, 1>();
+  if constexpr (MIXED && A56 >= 2 && A56 != A64) reg2_variant<PHYS, P, Q, 1, NTA, A56, MIXED, 1>(PREF);
   // FP64 at 72 registers: one more CTA per SM for a few dozen bytes of spills
   constexpr int A72 = blocks_for_regs<CA>(NTA, 72), B72 = blocks_for_regs<CB>(NTB, 72);
   if constexpr (!MIXED && A72 >= 2 && A72 != A80) reg2_variant<PHYS, P, Q, 1, NTA, A72, MIXED>();
@@ -541,7 +565,10 @@ struct Launch3Ns {
 template <int PHYS, int P, int Q>
 void reg3_ns() {
   register_ops(PHYS, P + 1, Q, Launch3Ns<PHYS, P + 1, Q>::ops());
-  register_ops(PHYS, P + 1, Q, Launch3Ns<PHYS, P + 1, Q, (P < 4 ? 128 : 256), (P < 4 ? 96 : 112), 128, 80>::ops());
+  // p = 3: 512 elements 21 us against 29, 4096 elements 95 against 94
+  KernelOps o = Launch3Ns<PHYS, P + 1, Q, (P < 4 ? 128 : 256), (P < 4 ? 96 : 112), 128, 80>::ops();
+  if (P < 4) o.small = 2048;
+  register_ops(PHYS, P + 1, Q, o);
 }
 
 // Elements per CTA of a 2-D tile: about 128 modal rows.

@@ -22,18 +22,17 @@ void register_ops(int physics, int L, int Q, const KernelOps &ops) {
   table()[std::make_tuple(physics, L, Q)].push_back(ops);
 }
 
-const KernelOps *find_ops(int physics, int L, int Q) {
+const KernelOps *default_ops(int physics, int L, int Q, int ne, bool plain) {
   std::lock_guard<std::mutex> lk(table_mutex());
   auto it = table().find(std::make_tuple(physics, L, Q));
-  if (it == table().end() || it->second.empty()) return nullptr;
-  // the default is the preferred tile, else the first plain CTA tile (both
-  // handle every stage kind and boundary sides), whatever order the
-  // compilation units registered in
-  for (const KernelOps &o : it->second)
-    if (o.preferred) return &o;
-  for (const KernelOps &o : it->second)
-    if (o.warp == 0) return &o;
-  return &it->second.front();
+  if (it == table().end()) return nullptr;
+  const KernelOps *best = nullptr;
+  for (const KernelOps &o : it->second) {
+    if (plain && o.warp != 0) continue;
+    if (o.small >= ne) return &o;
+    if (!best || o.preferred > best->preferred) best = &o;
+  }
+  return best;
 }
 
 const std::vector<KernelOps> *find_variants(int physics, int L, int Q) {

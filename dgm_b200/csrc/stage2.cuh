@@ -38,13 +38,9 @@
 // other stage kinds run the plain kernel of the same (L, Q)).
 #pragma once
 
-#include "stage.cuh"
+#include "pencil.cuh"
 
 namespace dgmx {
-
-// Tables of the second form (constant memory, per working type and (L, Q)).
-template <class T, int L, int Q> __constant__ T cE2[L * Q];          // E[a][j] = sum_i B[a][i] w_i D[i][j]
-template <class T, int L, int Q> __constant__ T cBwG[L * (Q - 1)];   // BwG[a][g] = sum_i B[a][i] w_i G2GL[i][g]
 
 template <int PHYS, int L_, int Q_, int EPB_, int NT_, int MINB_, bool MIXED_, int VDIRS_ = 0>
 struct Cfg2 {
@@ -292,14 +288,11 @@ __device__ __forceinline__ void s2_backward_k_row(const Smem2<C> &sm, const Stag
   }
   // planes of NF L Q = 4 (mod 16) values at p = 3: this pass's (n a, b) rows
   // and the j pass's contiguous reads both fall on distinct banks
-  T *dst = sm.slot(s) + C::O_T1 + (r % L) * (NF * L * Q) + (r / L) * Q;
+  T x[L], u[Q];
 #pragma unroll
-  for (int k = 0; k < Q; ++k) {
-    T acc = T(0);
-#pragma unroll
-    for (int c = 0; c < L; ++c) acc = fma(cB<T, L, Q>[c * Q + k], T(v[c]), acc);
-    dst[k] = acc;
-  }
+  for (int c = 0; c < L; ++c) x[c] = T(v[c]);
+  eo_expand<L, Q>(x, u);
+  st_pencil<Q>(sm.slot(s) + C::O_T1 + (r % L) * (NF * L * Q) + (r / L) * Q, 1, u);
 }
 
 template <class C, int PHYS>
@@ -350,17 +343,10 @@ __device__ __forceinline__ void s2_backward_j_pencil(const Smem2<C> &sm, int w) 
   constexpr int NF = C::NF, L = C::L, Q = C::Q, N = NF * L * Q;
   const int s = w / N, r = w - s * N;   // r = (n*L + a)*Q + k
   const T *src = sm.slot(s) + C::O_T1 + r;
-  T v[L];
-#pragma unroll
-  for (int b = 0; b < L; ++b) v[b] = src[b * N];
-  T *dst = sm.slot(s) + C::O_T2 + r;
-#pragma unroll
-  for (int j = 0; j < Q; ++j) {
-    T acc = T(0);
-#pragma unroll
-    for (int b = 0; b < L; ++b) acc = fma(cB<T, L, Q>[b * Q + j], v[b], acc);
-    dst[j * C::XJ] = acc;
-  }
+  T v[L], u[Q];
+  ld_pencil<L>(src, N, v);
+  eo_expand<L, Q>(v, u);
+  st_pencil<Q>(sm.slot(s) + C::O_T2 + r, C::XJ, u);
 }
 
 template <class C>
@@ -378,17 +364,10 @@ __device__ __forceinline__ void s2_backward_i(const Smem2<C> &sm, int tid) {
   for (int w = tid; w < EPB * N; w += C::NT) {
     const int s = w / N, r = w - s * N, n = r / (Q * Q), jk = r - n * Q * Q, j = jk / Q, k = jk - j * Q;
     const T *src = sm.slot(s) + C::O_T2 + j * C::XJ + n * L * Q + k;
-    T v[L];
-#pragma unroll
-    for (int a = 0; a < L; ++a) v[a] = src[a * Q];
-    T *dst = sm.slot(s) + C::O_UN + n * Q * Q * Q + jk;
-#pragma unroll
-    for (int i = 0; i < Q; ++i) {
-      T acc = T(0);
-#pragma unroll
-      for (int a = 0; a < L; ++a) acc = fma(cB<T, L, Q>[a * Q + i], v[a], acc);
-      dst[i * Q * Q] = acc;
-    }
+    T v[L], u[Q];
+    ld_pencil<L>(src, Q, v);
+    eo_expand<L, Q>(v, u);
+    st_pencil<Q>(sm.slot(s) + C::O_UN + n * Q * Q * Q + jk, Q * Q, u);
   }
 }
 
@@ -420,8 +399,8 @@ __device__ __forceinline__ void s2_volume_column(const Smem2<C> &sm, const Stage
     for (int n = 0; n < NF; ++n)
 #pragma unroll
       for (int b = 0; b < L; ++b) acc[r][n][b] = T(0);
-#pragma unroll
-  for (int i = 0; i < Q; ++i) {
+  // contravariant fluxes of one point of the column
+  auto point = [&](int i, T (&Gr)[NR][5]) {
     T U[5];
 #pragma unroll
     for (int n = 0; n < NF; ++n) U[n] = un[(n * Q + i) * Q * Q];
@@ -441,17 +420,11 @@ __device__ __forceinline__ void s2_volume_column(const Smem2<C> &sm, const Stage
         const T m0 = met[r][0], m1 = met[r][1], m2 = met[r][2];
         const T Vb = m0 * b.u[0] + m1 * b.u[1] + m2 * b.u[2];       // reference contravariant velocity
         const T Vp = m0 * upx + m1 * upy + m2 * upz;                 // its perturbation
-        T Gr[5];
-        Gr[0] = m0 * U[1] + m1 * U[2] + m2 * U[3];
-        Gr[1] = fma(U[1], Vb, fma(mx, Vp, pp * m0));
-        Gr[2] = fma(U[2], Vb, fma(my, Vp, pp * m1));
-        Gr[3] = fma(U[3], Vb, fma(mz, Vp, pp * m2));
-        Gr[4] = fma(Hp, Vb, H * Vp);
-#pragma unroll
-        for (int n = 0; n < NF; ++n)
-#pragma unroll
-          for (int bb = 0; bb < L; ++bb)
-            acc[r][n][bb] = fma(R0 + r == 0 ? cE2<T, L, Q>[bb * Q + i] : cBw<T, L, Q>[bb * Q + i], Gr[n], acc[r][n][bb]);
+        Gr[r][0] = m0 * U[1] + m1 * U[2] + m2 * U[3];
+        Gr[r][1] = fma(U[1], Vb, fma(mx, Vp, pp * m0));
+        Gr[r][2] = fma(U[2], Vb, fma(my, Vp, pp * m1));
+        Gr[r][3] = fma(U[3], Vb, fma(mz, Vp, pp * m2));
+        Gr[r][4] = fma(Hp, Vb, H * Vp);
       }
     } else {
       const T ir = T(1.0) / U[0];
@@ -466,19 +439,34 @@ __device__ __forceinline__ void s2_volume_column(const Smem2<C> &sm, const Stage
       for (int r = 0; r < NR; ++r) {
         const T m0 = met[r][0], m1 = met[r][1], m2 = met[r][2];
         const T V = fma(m2, ww, fma(m1, v, m0 * u));
-        T Gr[5];
-        Gr[0] = U[0] * V;
-        Gr[1] = fma(U[1], V, p * m0);
-        Gr[2] = fma(U[2], V, p * m1);
-        Gr[3] = fma(U[3], V, p * m2);
-        Gr[4] = Ep * V;
-#pragma unroll
-        for (int n = 0; n < NF; ++n)
-#pragma unroll
-          for (int bb = 0; bb < L; ++bb)
-            acc[r][n][bb] = fma(R0 + r == 0 ? cE2<T, L, Q>[bb * Q + i] : cBw<T, L, Q>[bb * Q + i], Gr[n], acc[r][n][bb]);
+        Gr[r][0] = U[0] * V;
+        Gr[r][1] = fma(U[1], V, p * m0);
+        Gr[r][2] = fma(U[2], V, p * m1);
+        Gr[r][3] = fma(U[3], V, p * m2);
+        Gr[r][4] = Ep * V;
       }
     }
+  };
+  // the two points i and Q-1-i of a column share their coefficients (pencil.cuh)
+#pragma unroll
+  for (int i = 0; i < (Q + 1) / 2; ++i) {
+    const bool mid = 2 * i + 1 == Q;
+    T Gp[NR][5], Gm[NR][5];
+    point(i, Gp);
+    if (!mid) point(Q - 1 - i, Gm);
+#pragma unroll
+    for (int r = 0; r < NR; ++r)
+#pragma unroll
+      for (int n = 0; n < NF; ++n) {
+        const T sum = mid ? Gp[r][n] : Gp[r][n] + Gm[r][n], dif = mid ? T(0) : Gp[r][n] - Gm[r][n];
+#pragma unroll
+        for (int bb = 0; bb < L; ++bb) {
+          const bool sym = (bb % 2 == 0) != (R0 + r == 0);
+          if (mid && !sym) continue;
+          acc[r][n][bb] = fma(R0 + r == 0 ? cE2<T, L, Q>[bb * Q + i] : cBw<T, L, Q>[bb * Q + i], sym ? sum : dif,
+                              acc[r][n][bb]);
+        }
+      }
   }
   const int j = jk / Q, k = jk - j * Q;
   T *dst = sm.slot(s) + C::O_X + j * C::XJ + k;
@@ -520,30 +508,62 @@ __device__ __forceinline__ void s2_pass_j(const Smem2<C> &sm, int tid) {
   for (int w = tid; w < EPB * N; w += C::NT) {
     const int s = w / N, r = w - s * N;   // r = (n*L + a)*Q + k
     const T *x = sm.slot(s) + C::O_X + r;   // a warp reads contiguous values
-    T x0[Q], x1[Q], x2[Q];
-#pragma unroll
-    for (int j = 0; j < Q; ++j) {
-      x0[j] = x[j * C::XJ];
-      x1[j] = x[(C::S_X1 + 1) + j * C::XJ];
-      x2[j] = x[2 * (C::S_X1 + 1) + j * C::XJ];
-    }
+    T v[Q], sf[(Q + 1) / 2], df[Q / 2], o[L];
     T *y = sm.slot(s) + C::O_Y + r;
-#pragma unroll
-    for (int b = 0; b < L; ++b) {
-      T y0 = T(0), y2 = T(0);
-#pragma unroll
-      for (int j = 0; j < Q; ++j) {
-        y0 = fma(cBw<T, L, Q>[b * Q + j], x0[j], y0);
-        y0 = fma(cE2<T, L, Q>[b * Q + j], x1[j], y0);
-        y2 = fma(cBw<T, L, Q>[b * Q + j], x2[j], y2);
-      }
-      y[b * N] = y0;
-      y[(C::S_Y1 + 1) + b * N] = y2;
-    }
+    zero<L>(o);
+    ld_pencil<Q>(x, C::XJ, v);
+    eo_fold<Q>(v, sf, df);
+    eo_project<L, Q, false>(sf, df, o);
+    ld_pencil<Q>(x + (C::S_X1 + 1), C::XJ, v);
+    eo_fold<Q>(v, sf, df);
+    eo_project<L, Q, true>(sf, df, o);
+    st_pencil<L>(y, N, o);
+    zero<L>(o);
+    ld_pencil<Q>(x + 2 * (C::S_X1 + 1), C::XJ, v);
+    eo_fold<Q>(v, sf, df);
+    eo_project<L, Q, false>(sf, df, o);
+    st_pencil<L>(y + (C::S_Y1 + 1), N, o);
   }
 }
 
 // ---- interval 6: k-axis pass, face terms, update, next modal block ---------
+// Row (n, a, b) of the projected right-hand side: the k pass and the face terms.
+template <class C>
+__device__ __forceinline__ void s2_rhs_row(const typename C::R *sl, int n, int aa, int bb, typename C::R (&R)[C::L]) {
+  using T = typename C::R;
+  constexpr int NF = C::NF, L = C::L, Q = C::Q, PL = C::PL;
+  // R[c] = sum_k P[c][k] Y0[k] + E[c][k] Y2[k]
+  const T *y = sl + C::O_Y + bb * (NF * L * Q) + (n * L + aa) * Q;
+  T v[Q], sf[(Q + 1) / 2], df[Q / 2];
+  zero<L>(R);
+  ld_pencil<Q>(y, 1, v);
+  eo_fold<Q>(v, sf, df);
+  eo_project<L, Q, false>(sf, df, R);
+  ld_pencil<Q>(y + (C::S_Y1 + 1), 1, v);
+  eo_fold<Q>(v, sf, df);
+  eo_project<L, Q, true>(sf, df, R);
+  // face terms: k faces (0: k=0, 5: k=Q-1) plane (a, b); j faces (1: j=0,
+  // 3: j=Q-1) plane (a, c); i faces (4: i=0, 2: i=Q-1) plane (b, c)
+  const T *xl = sl + C::O_XL;
+  constexpr int FB = NF * C::XLS;   // one face's block
+  const T xk0 = xl[0 * FB + n * C::XLS + aa * PL + bb], xk1 = xl[5 * FB + n * C::XLS + aa * PL + bb];
+  const T *xj0 = xl + 1 * FB + n * C::XLS + aa * PL, *xj1 = xl + 3 * FB + n * C::XLS + aa * PL;
+  const T *xi0 = xl + 4 * FB + n * C::XLS + bb * PL, *xi1 = xl + 2 * FB + n * C::XLS + bb * PL;
+  const T eb0 = end_value<T, L, Q>(0, bb), eb1 = end_value<T, L, Q>(1, bb);
+  const T ea0 = end_value<T, L, Q>(0, aa), ea1 = end_value<T, L, Q>(1, aa);
+#pragma unroll
+  for (int c = 0; c < L; ++c) {
+    T acc = R[c];
+    acc = fma(cEnd<T, L, Q>[c], xk0, acc);
+    acc = fma(cEnd<T, L, Q>[L + c], xk1, acc);
+    acc = fma(eb0, xj0[c], acc);
+    acc = fma(eb1, xj1[c], acc);
+    acc = fma(ea0, xi0[c], acc);
+    acc = fma(ea1, xi1[c], acc);
+    R[c] = acc;
+  }
+}
+
 template <class C, int PHYS>
 __device__ __forceinline__ void s2_update(const Smem2<C> &sm, const StageArgs &a, int tid) {
   using T = typename C::R;
@@ -553,37 +573,8 @@ __device__ __forceinline__ void s2_update(const Smem2<C> &sm, const StageArgs &a
     const int s = w / N, r = w - s * N, n = r / (L * L), ab = r - n * L * L, aa = ab / L, bb = ab - aa * L;
     const int e = sm.eid[s];
     T *sl = sm.slot(s);
-    // R[c] = sum_k P[c][k] Y0[k] + E[c][k] Y2[k]
-    const T *y = sl + C::O_Y + bb * (NF * L * Q) + (n * L + aa) * Q;
-    T y0[Q], y2[Q];
-#pragma unroll
-    for (int k = 0; k < Q; ++k) { y0[k] = y[k]; y2[k] = y[(C::S_Y1 + 1) + k]; }
-    // face terms: k faces (0: k=0, 5: k=Q-1) plane (a, b); j faces (1: j=0,
-    // 3: j=Q-1) plane (a, c); i faces (4: i=0, 2: i=Q-1) plane (b, c)
-    const T *xl = sl + C::O_XL;
-    constexpr int FB = NF * C::XLS;   // one face's block
-    const T xk0 = xl[0 * FB + n * C::XLS + aa * PL + bb], xk1 = xl[5 * FB + n * C::XLS + aa * PL + bb];
-    const T *xj0 = xl + 1 * FB + n * C::XLS + aa * PL, *xj1 = xl + 3 * FB + n * C::XLS + aa * PL;
-    const T *xi0 = xl + 4 * FB + n * C::XLS + bb * PL, *xi1 = xl + 2 * FB + n * C::XLS + bb * PL;
-    const T eb0 = end_value<T, L, Q>(0, bb), eb1 = end_value<T, L, Q>(1, bb);
-    const T ea0 = end_value<T, L, Q>(0, aa), ea1 = end_value<T, L, Q>(1, aa);
     T R[L];
-#pragma unroll
-    for (int c = 0; c < L; ++c) {
-      T acc = T(0);
-#pragma unroll
-      for (int k = 0; k < Q; ++k) {
-        acc = fma(cBw<T, L, Q>[c * Q + k], y0[k], acc);
-        acc = fma(cE2<T, L, Q>[c * Q + k], y2[k], acc);
-      }
-      acc = fma(cEnd<T, L, Q>[c], xk0, acc);
-      acc = fma(cEnd<T, L, Q>[L + c], xk1, acc);
-      acc = fma(eb0, xj0[c], acc);
-      acc = fma(eb1, xj1[c], acc);
-      acc = fma(ea0, xi0[c], acc);
-      acc = fma(ea1, xi1[c], acc);
-      R[c] = acc;
-    }
+    s2_rhs_row<C>(sl, n, aa, bb, R);
     // The state the right-hand side was evaluated on (X; X = U for LSRK)
     // is read back from global memory: its shared copy is dead by now.
     T *ub = sl + C::O_UB + r * PL;
@@ -833,6 +824,58 @@ __global__ void __launch_bounds__(C::NT, C::MINB) stage2_kernel(StageArgs a) {
     // 292 to 279 us in FP64 and from 233 to 238 us in the FP32 form
     if constexpr (!C::MIXED) s2_prefetch<C>(a, tile, next, threadIdx.x);
     stage2_tile<C, PHYS>(sm, a, tile * C::EPB, threadIdx.x);
+  }
+}
+
+// Domain::time_derivative on GLL values with the same passes: the state comes
+// from a.Xn instead of modal rows, and the projected right-hand side goes back
+// to GLL values (a.Fn) through the backward passes.  Traces from a.Tin.
+template <class C, int PHYS>
+__global__ void __launch_bounds__(C::NT, C::MINB) rhs2_kernel(StageArgs a) {
+  constexpr int NF = C::NF, L = C::L, Q = C::Q, QD = C::QD, N = NF * L * L;
+  static_assert(!C::MIXED && C::EPB == 1, "FP64, one element per CTA");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Smem2<C> sm(smem_raw);
+  const int tid = threadIdx.x, e = blockIdx.x;
+  double *sl = sm.slot(0);
+  s2_load<C>(sm, a, e, tid);
+  for (int l = tid; l < NF * ((QD * 8 + 127) / 128); l += C::NT) {   // read three intervals on
+    const int n = l % NF;
+    prefetch_l2_lines(a.Xn + ((size_t)n * a.ne + e) * QD, QD * 8, l / NF);
+  }
+  __syncthreads();
+  for (int w = tid; w < C::NFACE * C::GF; w += C::NT) s2_face_point<C, PHYS>(sm, a, e, w);
+  __syncthreads();
+  for (int w = tid; w < C::NFACE * NF; w += C::NT) s2_lift<C>(sm, w);
+  __syncthreads();   // the nodal values take the place of the face terms
+  for (int w = tid; w < NF * QD; w += C::NT) {
+    const int n = w / QD;
+    sl[C::O_UN + w] = a.Xn[((size_t)n * a.ne + e) * QD + (w - n * QD)];
+  }
+  __syncthreads();
+  s2_volume<C, PHYS>(sm, a, tid);
+  __syncthreads();
+  s2_pass_j<C>(sm, tid);
+  __syncthreads();
+  // one row per thread, held over the barrier: T1 takes the place of what the
+  // rows are made from
+  static_assert(N <= C::NT, "one thread per modal row");
+  double R[L];
+  if (tid < N) s2_rhs_row<C>(sl, tid / (L * L), tid / L % L, tid % L, R);
+  __syncthreads();
+  if (tid < N) {   // row (n L + a) L + b, as s2_backward_k_row
+    double u[Q];
+    eo_expand<L, Q>(R, u);
+    st_pencil<Q>(sl + C::O_T1 + (tid % L) * (NF * L * Q) + (tid / L) * Q, 1, u);
+  }
+  __syncthreads();
+  for (int w = tid; w < NF * L * Q; w += C::NT) s2_backward_j_pencil<C>(sm, w);
+  __syncthreads();
+  s2_backward_i<C>(sm, tid);
+  __syncthreads();
+  for (int w = tid; w < NF * QD; w += C::NT) {
+    const int n = w / QD;
+    a.Fn[((size_t)n * a.ne + e) * QD + (w - n * QD)] = sl[C::O_UN + w];
   }
 }
 

@@ -443,8 +443,10 @@ __device__ __forceinline__ void sd_front(const SmemD<C> &sm, const StageArgs &a,
   sd_load<C>(sm, a, e0, tid);
   pdl_wait();
   for (int w = tid; w < C::EPB * 4 * C::G; w += NT) sd_face_point<C, PHYS, SELF>(sm, a, e0, w);
+  // from the last thread down: a tile with threads enough for both does the
+  // rows beside the face points
   if constexpr (!NODAL && !is_ns(PHYS))
-    for (int w = tid; w < C::EPB * C::NF * C::L; w += NT) sd_state_row<C>(sm, a, e0, w);
+    for (int w = NT - 1 - tid; w < C::EPB * C::NF * C::L; w += NT) sd_state_row<C>(sm, a, e0, w);
   __syncthreads();
   if constexpr (!is_ns(PHYS)) for (int w = tid; w < 2 * NC; w += NT) {
     const int c = w < NC ? w : w - NC, s = c / C::Q, j = c - s * C::Q;
