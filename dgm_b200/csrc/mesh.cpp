@@ -2,11 +2,13 @@
 // affine geometry and geometry classes; readers for DGM's input files.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <fstream>
 #include <map>
 #include <sstream>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "dgmx_internal.hpp"
@@ -148,6 +150,15 @@ bool build_mesh(const dgmx_mesh &m, const Tables1D &t, HostMesh &out, std::strin
   out.J.resize(ne);
   const size_t qd = dim == 2 ? (size_t)Q * Q : (size_t)Q * Q * Q;
   out.cx.assign(qd * ne, 0.0); out.cy.assign(qd * ne, 0.0); out.cz.assign(qd * ne, 0.0);
+  // weights of an element's vertices in its GLL points, the same for all
+  std::vector<double> wt(qd * nv);
+  for (size_t i = 0; i < qd; ++i) {
+    const int ix[3] = {dim == 2 ? (int)i / Q : (int)i / (Q * Q), dim == 2 ? (int)i % Q : (int)i / Q % Q, (int)i % Q};
+    static const int va[8] = {0, 1, 1, 0, 0, 1, 1, 0}, vb[8] = {0, 0, 1, 1, 0, 0, 1, 1}, vc[8] = {0, 0, 0, 0, 1, 1, 1, 1};
+    auto half = [&](int d, int hi) { return hi ? 0.5 * (1.0 + t.z[ix[d]]) : 0.5 * (1.0 - t.z[ix[d]]); };
+    for (int v = 0; v < nv; ++v)
+      wt[i * nv + v] = dim == 2 ? half(0, va[v]) * half(1, vb[v]) : half(0, va[v]) * half(1, vb[v]) * half(2, vc[v]);
+  }
   for (int e = 0; e < ne; ++e) {
     ElemGeo &g = geo[e];
     std::memset(&g, 0, sizeof(g));
@@ -169,16 +180,13 @@ bool build_mesh(const dgmx_mesh &m, const Tables1D &t, HostMesh &out, std::strin
         const double tx = (s == 0 || s == 2) ? xr : xs, ty = (s == 0 || s == 2) ? yr : ys;
         g.jr[s] = std::sqrt(tx * tx + ty * ty) / J;
       }
-      for (int i = 0; i < Q; ++i)
-        for (int j = 0; j < Q; ++j) {
-          const double pa0 = 0.5 * (1.0 - t.z[i]), pa1 = 0.5 * (1.0 + t.z[i]);
-          const double pb0 = 0.5 * (1.0 - t.z[j]), pb1 = 0.5 * (1.0 + t.z[j]);
-          const double w[4] = {pa0 * pb0, pa1 * pb0, pa1 * pb1, pa0 * pb1};
-          double x = 0, y = 0;
-          for (int v = 0; v < 4; ++v) { x += X(e, v, 0) * w[v]; y += X(e, v, 1) * w[v]; }
-          out.cx[(size_t)e * qd + i * Q + j] = x;
-          out.cy[(size_t)e * qd + i * Q + j] = y;
-        }
+      for (size_t i = 0; i < qd; ++i) {
+        const double *w = &wt[i * 4];
+        double x = 0, y = 0;
+        for (int v = 0; v < 4; ++v) { x += X(e, v, 0) * w[v]; y += X(e, v, 1) * w[v]; }
+        out.cx[(size_t)e * qd + i] = x;
+        out.cy[(size_t)e * qd + i] = y;
+      }
     } else {
       double d[3][3];  // d[c][0]=x_r-ish: d[c][k] = (X(v_k) - X(v_0))/2 for k = r,s,t
       const int vk[3] = {1, 3, 4};
@@ -206,22 +214,13 @@ bool build_mesh(const dgmx_mesh &m, const Tables1D &t, HostMesh &out, std::strin
         const double cx = u[1] * v[2] - u[2] * v[1], cy = u[2] * v[0] - u[0] * v[2], cz = u[0] * v[1] - u[1] * v[0];
         g.jr[s] = std::sqrt(cx * cx + cy * cy + cz * cz) / J;
       }
-      for (int i = 0; i < Q; ++i)
-        for (int j = 0; j < Q; ++j)
-          for (int k = 0; k < Q; ++k) {
-            const double pa[2] = {0.5 * (1.0 - t.z[i]), 0.5 * (1.0 + t.z[i])};
-            const double pb[2] = {0.5 * (1.0 - t.z[j]), 0.5 * (1.0 + t.z[j])};
-            const double pc[2] = {0.5 * (1.0 - t.z[k]), 0.5 * (1.0 + t.z[k])};
-            static const int va[8] = {0, 1, 1, 0, 0, 1, 1, 0}, vb[8] = {0, 0, 1, 1, 0, 0, 1, 1},
-                             vc[8] = {0, 0, 0, 0, 1, 1, 1, 1};
-            double x = 0, y = 0, z = 0;
-            for (int v = 0; v < 8; ++v) {
-              const double w = pa[va[v]] * pb[vb[v]] * pc[vc[v]];
-              x += X(e, v, 0) * w; y += X(e, v, 1) * w; z += X(e, v, 2) * w;
-            }
-            const size_t q = (size_t)e * qd + (i * Q + j) * Q + k;
-            out.cx[q] = x; out.cy[q] = y; out.cz[q] = z;
-          }
+      for (size_t i = 0; i < qd; ++i) {
+        const double *w = &wt[i * 8];
+        double x = 0, y = 0, z = 0;
+        for (int v = 0; v < 8; ++v) { x += X(e, v, 0) * w[v]; y += X(e, v, 1) * w[v]; z += X(e, v, 2) * w[v]; }
+        const size_t q = (size_t)e * qd + i;
+        out.cx[q] = x; out.cy[q] = y; out.cz[q] = z;
+      }
     }
     out.J[e] = g.J;
   }
@@ -231,25 +230,29 @@ bool build_mesh(const dgmx_mesh &m, const Tables1D &t, HostMesh &out, std::strin
   out.perm.clear();
   std::map<std::vector<int>, int> perm_ids;
   const int n1 = t.G, n2 = dim == 2 ? 1 : t.G;
+  int by_flags[16];
+  std::fill(by_flags, by_flags + 16, -1);
   for (int e = 0; e < ne; ++e)
     for (int s = 0; s < nfaces; ++s) {
       const SideInfo &S = side[(size_t)e * nfaces + s];
-      std::vector<int> p(gf);
-      if (S.master) {
-        // master point side_map(S, q) pairs with the slave's point q
-        for (int q = 0; q < gf; ++q) p[side_map(dim, S, n1, n2, q)] = q;
-      } else {
-        const SideInfo &M = side[(size_t)S.le * nfaces + S.ls];
-        for (int q = 0; q < gf; ++q) p[q] = side_map(dim, M, n1, n2, q);
-      }
-      auto it = perm_ids.find(p);
-      int off;
-      if (it == perm_ids.end()) {
-        off = (int)out.perm.size();
-        out.perm.insert(out.perm.end(), p.begin(), p.end());
-        perm_ids[p] = off;
-      } else {
-        off = it->second;
+      // a permutation is set by the master's flags and the side's role
+      const SideInfo &M = S.master ? S : side[(size_t)S.le * nfaces + S.ls];
+      int &off = by_flags[(S.master ? 8 : 0) | (M.flip_a ? 4 : 0) | (M.flip_b ? 2 : 0) | (M.transp ? 1 : 0)];
+      if (off < 0) {
+        std::vector<int> p(gf);
+        // master point side_map(M, q) pairs with the slave's point q
+        for (int q = 0; q < gf; ++q) {
+          const int g = side_map(dim, M, n1, n2, q);
+          if (S.master) p[g] = q; else p[q] = g;
+        }
+        auto it = perm_ids.find(p);
+        if (it == perm_ids.end()) {
+          off = (int)out.perm.size();
+          out.perm.insert(out.perm.end(), p.begin(), p.end());
+          perm_ids[p] = off;
+        } else {
+          off = it->second;
+        }
       }
       // a boundary side points at itself (identity order); its neighbour
       // state is made from its own trace
@@ -257,7 +260,7 @@ bool build_mesh(const dgmx_mesh &m, const Tables1D &t, HostMesh &out, std::strin
     }
 
   // --- geometry classes
-  std::map<std::string, int> class_ids;
+  std::unordered_map<std::string, int> class_ids;
   out.gclass.resize(ne);
   out.classes.clear();
   for (int e = 0; e < ne; ++e) {
@@ -272,16 +275,20 @@ bool build_mesh(const dgmx_mesh &m, const Tables1D &t, HostMesh &out, std::strin
       for (int k = 0; k < 3; ++k) c.nrm[s][k] = n[k];
       for (int k = 0; k < 3; ++k) c.onrm[s][k] = geo[e].nrm[s][k];
       c.jr[s] = geo[e].jr[s];
-      // local axis of side s: 3-D 0,5 -> k, 1,3 -> j, 2,4 -> i; 2-D 0,2 -> j, 1,3 -> i
-      const int ax = dim == 3 ? (s == 0 || s == 5 ? 2 : (s == 1 || s == 3 ? 1 : 0)) : (s % 2 == 0 ? 1 : 0);
-      const double *mt = c.metric + 3 * ax, *on = c.onrm[s];
-      c.tv[s] = (on[0] * mt[0] + on[1] * mt[1] + on[2] * mt[2]) / (mt[0] * mt[0] + mt[1] * mt[1] + mt[2] * mt[2]);
-      if (dim == 3) face_frame(c.nrm[s], c.fr[s]);
       if (S.master) c.master |= 1 << s;
     }
-    std::string key(reinterpret_cast<const char *>(&c), sizeof(c));
+    // the face frames and scales follow from what stands before them
+    std::string key(reinterpret_cast<const char *>(&c), offsetof(GeomClass, tv));
+    key.append(reinterpret_cast<const char *>(&c.master), 2 * sizeof(int));
     auto it = class_ids.find(key);
     if (it == class_ids.end()) {
+      for (int s = 0; s < nfaces; ++s) {
+        // local axis of side s: 3-D 0,5 -> k, 1,3 -> j, 2,4 -> i; 2-D 0,2 -> j, 1,3 -> i
+        const int ax = dim == 3 ? (s == 0 || s == 5 ? 2 : (s == 1 || s == 3 ? 1 : 0)) : (s % 2 == 0 ? 1 : 0);
+        const double *mt = c.metric + 3 * ax, *on = c.onrm[s];
+        c.tv[s] = (on[0] * mt[0] + on[1] * mt[1] + on[2] * mt[2]) / (mt[0] * mt[0] + mt[1] * mt[1] + mt[2] * mt[2]);
+        if (dim == 3) face_frame(c.nrm[s], c.fr[s]);
+      }
       const int id = (int)out.classes.size();
       out.classes.push_back(c);
       class_ids[key] = id;

@@ -553,26 +553,24 @@ dgmx_status add_impl(dgmx_pool *P, const dgmx_mesh *m, int phys, const double *U
     cmap[c] = nid;
     new_classes.push_back(hm.classes[c]);
   }
-  std::map<int, int> pmap;   // solve's perm offset -> arena offset
+  std::vector<int> pmap(hm.perm.size() / a.gf, -1);   // solve's permutation -> arena offset
   std::vector<int> new_perm;
   std::map<std::vector<int>, int> new_perm_keys;
-  for (const FaceLink &lk : hm.links) {
-    if (pmap.count(lk.perm)) continue;
-    std::vector<int> key(hm.perm.begin() + lk.perm, hm.perm.begin() + lk.perm + a.gf);
-    int off;
+  for (size_t k = 0; k < pmap.size(); ++k) {
+    std::vector<int> key(hm.perm.begin() + k * a.gf, hm.perm.begin() + (k + 1) * a.gf);
     auto it = a.perm_index.find(key);
     auto jt = new_perm_keys.find(key);
     if (it != a.perm_index.end()) {
-      off = it->second;
+      pmap[k] = it->second;
     } else if (jt != new_perm_keys.end()) {
-      off = jt->second;
+      pmap[k] = jt->second;
     } else {
-      off = (int)(a.perm_h.size() + new_perm.size());
+      const int off = (int)(a.perm_h.size() + new_perm.size());
       if (off + a.gf > a.perm_cap) return P->fail(DGMX_ERR_MEMORY, "too many face permutations in one arena");
       new_perm.insert(new_perm.end(), key.begin(), key.end());
       new_perm_keys[key] = off;
+      pmap[k] = off;
     }
-    pmap[lk.perm] = off;
   }
   if ((st = ensure_scratch(P, nodal)) != DGMX_OK) return st;
   int e0 = 0;
@@ -592,14 +590,14 @@ dgmx_status add_impl(dgmx_pool *P, const dgmx_mesh *m, int phys, const double *U
     for (int f = 0; f < a.nfaces; ++f) {
       FaceLink lk = hm.links[(size_t)e * a.nfaces + f];
       lk.elem += e0;
-      lk.perm = pmap[lk.perm];
+      lk.perm = pmap[lk.perm / a.gf];
       lks[(size_t)e * a.nfaces + f] = lk;
     }
     lks[(size_t)e * a.nfaces].cls = gcl[e];
   }
   // reference state of the mixed form: the J- and GLL-weighted mean of U0
   double ref[kUrefStride] = {};
-  {
+  if (a.mixed) {
     std::vector<double> wq(a.qd);
     for (int i = 0; i < a.qd; ++i) {
       const int ix = i % a.Q, iy = (i / a.Q) % a.Q, iz = i / (a.Q * a.Q);
@@ -629,8 +627,10 @@ dgmx_status add_impl(dgmx_pool *P, const dgmx_mesh *m, int phys, const double *U
   up(a.gclass + e0, gcl.data(), sizeof(int) * nalloc);
   up(a.esolve + e0, es.data(), sizeof(int) * nalloc);
   up(a.links + (size_t)e0 * a.nfaces, lks.data(), sizeof(FaceLink) * lks.size());
-  std::memcpy(a.uref_pin + (size_t)kUrefStride * slot, ref, sizeof(ref));
-  up(a.uref + (size_t)kUrefStride * slot, a.uref_pin + (size_t)kUrefStride * slot, sizeof(ref));
+  if (a.mixed) {
+    std::memcpy(a.uref_pin + (size_t)kUrefStride * slot, ref, sizeof(ref));
+    up(a.uref + (size_t)kUrefStride * slot, a.uref_pin + (size_t)kUrefStride * slot, sizeof(ref));
+  }
   up(P->scratch, U0, sizeof(double) * nodal);
   // projection of U0 into the range, zero second register, traces
   StageArgs s = arena_args(P, a);
