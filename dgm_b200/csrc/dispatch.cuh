@@ -678,13 +678,19 @@ struct Launch2DNs {
   }
 };
 
-// 2-D tiles of one (physics, p, q): 128 threads (the default) and half of it.
+// 2-D tiles of one (physics, p, q): 128 threads (the default) and half of it,
+// and 256, where every interval's tasks run side by side, for a mesh of one
+// CTA per SM or less (16 x 16, p = 4: 6.5 us a stage against 7.4).
 template <int PHYS, int P, int Q, bool MIXED = false>
 void reg2d() {
   constexpr int E = stage2d_epb(phys_nf(PHYS), P + 1), B = MIXED ? 6 : 4;
   const int key = PHYS + (MIXED ? kMixedKey : 0);
   register_ops(key, P + 1, Q, Launch2D<PHYS, P + 1, Q, MIXED, E, 128, B>::ops());
   register_ops(key, P + 1, Q, Launch2D<PHYS, P + 1, Q, MIXED, (E + 1) / 2, 64, 2 * B>::ops());
+  KernelOps o = Launch2D<PHYS, P + 1, Q, MIXED, E, 256, 1>::ops();
+  o.preferred = 0;
+  o.small = 148 * E;
+  register_ops(key, P + 1, Q, o);
 }
 template <int PHYS, int P, int Q>
 void reg2d_ns() {
