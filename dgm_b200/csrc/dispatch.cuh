@@ -143,18 +143,18 @@ struct Launch {
       using N = NsCfg<CV, float>;
       if ((e = upload_tables_lq<L, Q, float>(t)) != cudaSuccess) return e;
       const int sg = (int)N::Grad::SMEM, sv = (int)N::Visc::SMEM;
-      if ((e = cudaFuncSetAttribute(ns_grad_kernel<CV, PHYS, false, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sg))) return e;
-      if ((e = cudaFuncSetAttribute(ns_grad_kernel<CV, PHYS, true, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sg))) return e;
-      if ((e = cudaFuncSetAttribute(ns_visc_kernel<CV, PHYS, false, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sv))) return e;
-      if ((e = cudaFuncSetAttribute(ns_visc_kernel<CV, PHYS, true, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sv))) return e;
+      if ((e = cudaFuncSetAttribute(ns_grad_kernel<CV, PHYS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sg))) return e;
+      if ((e = cudaFuncSetAttribute(ns_grad_kernel<CV, PHYS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sg))) return e;
+      if ((e = cudaFuncSetAttribute(ns_visc_kernel<CV, PHYS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sv))) return e;
+      if ((e = cudaFuncSetAttribute(ns_visc_kernel<CV, PHYS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sv))) return e;
     }
     return cudaSuccess;
   }
   static cudaError_t ns_grad32(const StageArgs &a, bool nodal, cudaStream_t s) {
     if constexpr (kVisc32) {
       using N = NsCfg<CV, float>;
-      if (nodal) ns_grad_kernel<CV, PHYS, true, float, true><<<grid(a.ne), CV::NT, N::Grad::SMEM, s>>>(a);
-      else ns_grad_kernel<CV, PHYS, false, float, true><<<grid(a.ne), CV::NT, N::Grad::SMEM, s>>>(a);
+      if (nodal) ns_grad_kernel<CV, PHYS, true><<<grid(a.ne), CV::NT, N::Grad::SMEM, s>>>(a);
+      else ns_grad_kernel<CV, PHYS, false><<<grid(a.ne), CV::NT, N::Grad::SMEM, s>>>(a);
       return cudaGetLastError();
     } else {
       return cudaErrorNotSupported;
@@ -163,8 +163,8 @@ struct Launch {
   static cudaError_t ns_visc32(const StageArgs &a, bool nodal, cudaStream_t s) {
     if constexpr (kVisc32) {
       using N = NsCfg<CV, float>;
-      if (nodal) ns_visc_kernel<CV, PHYS, true, float, true><<<vgrid(a), CV::NT, N::Visc::SMEM, s>>>(a);
-      else ns_visc_kernel<CV, PHYS, false, float, true><<<vgrid(a), CV::NT, N::Visc::SMEM, s>>>(a);
+      if (nodal) ns_visc_kernel<CV, PHYS, true><<<vgrid(a), CV::NT, N::Visc::SMEM, s>>>(a);
+      else ns_visc_kernel<CV, PHYS, false><<<vgrid(a), CV::NT, N::Visc::SMEM, s>>>(a);
       return cudaGetLastError();
     } else {
       return cudaErrorNotSupported;
@@ -706,57 +706,6 @@ void reg_pipe() {
   if constexpr (PP::OK && PP::SMEM <= 227 * 1024 && (MINB == 0 || 65536 / (C::NT * MINB) >= 48)) {
     if constexpr (MINB == 0 || (228 * 1024) / (PP::SMEM + 1024) >= MINB)
       register_ops(PHYS + (MIXED ? kMixedKey : 0), P + 1, Q, PLaunch<PHYS, P + 1, Q, EPB, MINB, MIXED>::ops());
-  }
-}
-
-
-
-
-// CTAs per SM that the shared memory of one tile allows (228 KB per SM,
-// 1 KB reserved per CTA).
-template <class C>
-constexpr int smem_blocks() { return (int)((228 * 1024) / (C::SMEM + 1024)); }
-
-// Navier-Stokes tiles also need their viscous kernels to fit shared memory.
-template <int PHYS, class C>
-constexpr bool ns_fits() {
-  if constexpr (is_ns(PHYS)) return NsCfg<C>::Grad::SMEM <= 227 * 1024 && NsCfg<C>::Visc::SMEM <= 227 * 1024;
-  else return true;
-}
-
-// Register variant (EPB, MINB) when it is distinct and sensible: the
-// register cap 64K/(NT*MINB) stays >= 48 and the tile fits shared memory.
-template <int PHYS, int P, int Q, int EPB, int MINB, bool MIXED, int NT = 0>
-void reg_variant() {
-  using C = Cfg<PHYS, P + 1, Q, EPB, MINB, MIXED, NT>;
-  if constexpr (ns_fits<PHYS, C>() && (MINB == 0 || (65536 / (C::NT * MINB) >= 48 && smem_blocks<C>() >= MINB))) {
-    register_ops(PHYS + (MIXED ? kMixedKey : 0), P + 1, Q, Launch<PHYS, P + 1, Q, EPB, MINB, MIXED, NT>::ops());
-  }
-}
-
-
-// Tile variants for (physics, p, q): the default packing without and with a
-// register cap at the shared-memory occupancy, and twice the packing.  The
-// first registered variant is the default; dgmx_autotune picks among all.
-template <int PHYS, int P, int Q, bool MIXED = false>
-void reg() {
-  constexpr int E1 = default_epb(phys_dim(PHYS), Q);
-  using C1 = Cfg<PHYS, P + 1, Q, E1, 0, MIXED>;
-  constexpr int B1 = smem_blocks<C1>() > 8 ? 8 : smem_blocks<C1>();
-  reg_variant<PHYS, P, Q, E1, 0, MIXED>();
-  if constexpr (B1 >= 2) reg_variant<PHYS, P, Q, E1, B1, MIXED>();
-  if constexpr (B1 >= 4) reg_variant<PHYS, P, Q, E1, (B1 * 3) / 4, MIXED>();
-  constexpr int E2 = 2 * E1;
-  if constexpr (Cfg<PHYS, P + 1, Q, E2, 0, MIXED>::NT <= 1024 && Cfg<PHYS, P + 1, Q, E2, 0, MIXED>::SMEM <= 200 * 1024) {
-    using C2 = Cfg<PHYS, P + 1, Q, E2, 0, MIXED>;
-    constexpr int B2 = smem_blocks<C2>() > 8 ? 8 : smem_blocks<C2>();
-    if constexpr (B2 >= 2) reg_variant<PHYS, P, Q, E2, B2, MIXED>();
-  }
-  if constexpr (Pipe<C1>::OK) {
-    constexpr int PB = (int)((228 * 1024) / (Pipe<C1>::SMEM + 1024)) > 8 ? 8 : (int)((228 * 1024) / (Pipe<C1>::SMEM + 1024));
-    reg_pipe<PHYS, P, Q, E1, 0, MIXED>();
-    if constexpr (PB >= 2) reg_pipe<PHYS, P, Q, E1, PB, MIXED>();
-    if constexpr (PB >= 4) reg_pipe<PHYS, P, Q, E1, (PB * 3) / 4, MIXED>();
   }
 }
 

@@ -1,8 +1,8 @@
-// Navier-Stokes (BR1) viscous kernels for sm_100a, FP64.
+// Navier-Stokes 3-D (BR1): the separate viscous kernels of the 3xTF32 option
+// (dgmx_set_tensor_contractions, p >= 5), FP32 with tensor-core contractions.
 //
-// The viscous part of Navier_Stokes[3d]::diffusion (src/Navier_Stokes3d.cpp:
-// 182-391, src/Navier_Stokes.cpp:113-252) needs two face exchanges per
-// stage, so it runs as two launches before the fused stage kernel:
+// The viscous part of Navier_Stokes3d::diffusion (src/Navier_Stokes3d.cpp:
+// 182-391) runs as two launches before the first-form stage kernel:
 //   ns_grad_kernel : primitive traces (src/Euler3d.cpp:1162-1199), BR1
 //     averages (src/Domain.cpp:1883-1937, '+'), collocation gradients of
 //     u, v, w, e, the lift of ({{q}} - q) n J, and the L2 projection of each
@@ -15,6 +15,8 @@
 // The stage kernel then adds the viscous lift ('-' averages of the traces)
 // and subtracts the projected divergence (projection is linear, so
 // proj(conv) - proj(div g + lift) equals the reference's single projection).
+// The other forms are ns_flux_kernel (form3.cuh) and ns2d_flux_kernel
+// (stage2d.cuh), which also use primitive, viscous_stress and heat_flux.
 #pragma once
 
 #include "stage.cuh"
@@ -23,13 +25,12 @@ namespace dgmx {
 
 constexpr bool is_ns(int p) { return p == DGMX_NS2D || p == DGMX_NS3D; }
 
-// A contraction of the viscous kernels: with TC, FP32 data and an operator
-// of at least 5 x 5, on the tensor cores (contract_tc, 3xTF32); otherwise
-// on the CUDA cores (contract).
-template <bool TC, int I0, int I1, int I2, int AX, int K, int N, class M, bool ACC, class T, int IS0 = -1,
+// A contraction of the viscous kernels: an operator of at least 5 x 5 on the
+// tensor cores (contract_tc, 3xTF32), a smaller one on the CUDA cores.
+template <int I0, int I1, int I2, int AX, int K, int N, class M, bool ACC, class T, int IS0 = -1,
           int IS1 = -1, int OS0 = -1, int OS1 = -1>
 __device__ __forceinline__ void vcontract(const T *in, T *out, int nbatch, int sin, int sout, int tid, int nthr) {
-  if constexpr (TC && std::is_same<T, float>::value && K >= 5 && N >= 5)
+  if constexpr (K >= 5 && N >= 5)
     contract_tc<I0, I1, I2, AX, K, N, M, ACC, IS0, IS1, OS0, OS1>(in, out, nbatch, sin, sout, tid, nthr);
   else
     contract<I0, I1, I2, AX, K, N, M, ACC, T, IS0, IS1, OS0, OS1>(in, out, nbatch, sin, sout, tid, nthr);
@@ -41,7 +42,7 @@ __device__ __forceinline__ void vcontract(const T *in, T *out, int nbatch, int s
 template <class V>
 constexpr size_t ns_data_bytes(int values) { return ((size_t)values * sizeof(V) + 7) & ~(size_t)7; }
 
-template <class C, class V = double>
+template <class C, class V = float>
 struct NsCfg {
   static constexpr int DIM = C::DIM, NF = C::NF, L = C::L, Q = C::Q, G = C::G;
   static constexpr int EPB = C::EPB, NFACE = C::NFACE, NT = C::NT;
@@ -189,16 +190,16 @@ __device__ __forceinline__ void load_nbr_traces(V *E2, const double *T, const Fa
 
 // G2GL of NB face-major arrays [f][slot][b][GF] and accumulation with the
 // inverse end weights into dst [slot][b][QD] (faces in increasing order).
-template <class C, int NB, class V, bool TC = false>
+template <class C, int NB, class V>
 __device__ __forceinline__ void lift_batch(const V *Fg, V *LFc, V *S, V *dst, int tid) {
   constexpr int DIM = C::DIM, L = C::L, Q = C::Q, G = C::G, EPB = C::EPB, QD = C::QD, QF = C::QF;
   constexpr int NBT = C::NFACE * EPB * NB;
   if constexpr (DIM == 3) {
-    vcontract<TC, G, G, 1, 0, G, Q, MatG2GL<L, Q, V>, false>(Fg, S, NBT, G * G, Q * G, tid, C::NT);
+    vcontract<G, G, 1, 0, G, Q, MatG2GL<L, Q, V>, false>(Fg, S, NBT, G * G, Q * G, tid, C::NT);
     __syncthreads();
-    vcontract<TC, Q, G, 1, 1, G, Q, MatG2GL<L, Q, V>, false>(S, LFc, NBT, Q * G, Q * Q, tid, C::NT);
+    vcontract<Q, G, 1, 1, G, Q, MatG2GL<L, Q, V>, false>(S, LFc, NBT, Q * G, Q * Q, tid, C::NT);
   } else {
-    vcontract<TC, G, 1, 1, 0, G, Q, MatG2GL<L, Q, V>, false>(Fg, LFc, NBT, G, Q, tid, C::NT);
+    vcontract<G, 1, 1, 0, G, Q, MatG2GL<L, Q, V>, false>(Fg, LFc, NBT, G, Q, tid, C::NT);
   }
   __syncthreads();
   const V w0 = V(1.0) / cW<V, L, Q>[0], w1 = V(1.0) / cW<V, L, Q>[Q - 1];
@@ -229,7 +230,7 @@ __device__ __forceinline__ void lift_batch(const V *Fg, V *LFc, V *S, V *dst, in
 
 // w-weighted projection of NB arrays [slot][b][QD] (weighted in place) to
 // modal dst [slot][b][LD].
-template <class C, int NB, class V, bool TC = false>
+template <class C, int NB, class V>
 __device__ __forceinline__ void forward_batch(V *src, V *dst, V *S1, V *S2, int tid) {
   constexpr int DIM = C::DIM, L = C::L, Q = C::Q, QD = C::QD, LD = C::LD, NBT = C::EPB * NB;
   for (int w = tid; w < NBT * QD; w += C::NT) {
@@ -241,33 +242,33 @@ __device__ __forceinline__ void forward_batch(V *src, V *dst, V *S1, V *S2, int 
   }
   __syncthreads();
   if constexpr (DIM == 3) {
-    vcontract<TC, Q, Q, Q, 0, Q, L, MatBt<L, Q, V>, false>(src, S1, NBT, QD, L * Q * Q, tid, C::NT);
+    vcontract<Q, Q, Q, 0, Q, L, MatBt<L, Q, V>, false>(src, S1, NBT, QD, L * Q * Q, tid, C::NT);
     __syncthreads();
-    vcontract<TC, L, Q, Q, 1, Q, L, MatBt<L, Q, V>, false>(S1, S2, NBT, L * Q * Q, L * L * Q, tid, C::NT);
+    vcontract<L, Q, Q, 1, Q, L, MatBt<L, Q, V>, false>(S1, S2, NBT, L * Q * Q, L * L * Q, tid, C::NT);
     __syncthreads();
-    vcontract<TC, L, L, Q, 2, Q, L, MatBt<L, Q, V>, false>(S2, dst, NBT, L * L * Q, LD, tid, C::NT);
+    vcontract<L, L, Q, 2, Q, L, MatBt<L, Q, V>, false>(S2, dst, NBT, L * L * Q, LD, tid, C::NT);
   } else {
-    vcontract<TC, Q, Q, 1, 0, Q, L, MatBt<L, Q, V>, false>(src, S1, NBT, QD, L * Q, tid, C::NT);
+    vcontract<Q, Q, 1, 0, Q, L, MatBt<L, Q, V>, false>(src, S1, NBT, QD, L * Q, tid, C::NT);
     __syncthreads();
-    vcontract<TC, L, Q, 1, 1, Q, L, MatBt<L, Q, V>, false>(S1, dst, NBT, L * Q, LD, tid, C::NT);
+    vcontract<L, Q, 1, 1, Q, L, MatBt<L, Q, V>, false>(S1, dst, NBT, L * Q, LD, tid, C::NT);
   }
   __syncthreads();
 }
 
 // modal [slot][b][LD] -> GLL [slot][b][QD]
-template <class C, int NB, class V, bool TC = false>
+template <class C, int NB, class V>
 __device__ __forceinline__ void backward_batch(const V *src, V *dst, V *S1, V *S2, int tid) {
   constexpr int L = C::L, Q = C::Q, NBT = C::EPB * NB;
   if constexpr (C::DIM == 3) {
-    vcontract<TC, L, L, L, 0, L, Q, MatB<L, Q, V>, false>(src, S1, NBT, C::LD, Q * L * L, tid, C::NT);
+    vcontract<L, L, L, 0, L, Q, MatB<L, Q, V>, false>(src, S1, NBT, C::LD, Q * L * L, tid, C::NT);
     __syncthreads();
-    vcontract<TC, Q, L, L, 1, L, Q, MatB<L, Q, V>, false>(S1, S2, NBT, Q * L * L, Q * Q * L, tid, C::NT);
+    vcontract<Q, L, L, 1, L, Q, MatB<L, Q, V>, false>(S1, S2, NBT, Q * L * L, Q * Q * L, tid, C::NT);
     __syncthreads();
-    vcontract<TC, Q, Q, L, 2, L, Q, MatB<L, Q, V>, false>(S2, dst, NBT, Q * Q * L, C::QD, tid, C::NT);
+    vcontract<Q, Q, L, 2, L, Q, MatB<L, Q, V>, false>(S2, dst, NBT, Q * Q * L, C::QD, tid, C::NT);
   } else {
-    vcontract<TC, L, L, 1, 0, L, Q, MatB<L, Q, V>, false>(src, S1, NBT, C::LD, Q * L, tid, C::NT);
+    vcontract<L, L, 1, 0, L, Q, MatB<L, Q, V>, false>(src, S1, NBT, C::LD, Q * L, tid, C::NT);
     __syncthreads();
-    vcontract<TC, Q, L, 1, 1, L, Q, MatB<L, Q, V>, false>(S1, dst, NBT, Q * L, C::QD, tid, C::NT);
+    vcontract<Q, L, 1, 1, L, Q, MatB<L, Q, V>, false>(S1, dst, NBT, Q * L, C::QD, tid, C::NT);
   }
   __syncthreads();
 }
@@ -358,10 +359,10 @@ __device__ __forceinline__ void load_state_shifted(float *dst, double *Rs, const
 }
 
 // ---------------------------------------------------------------- gradients
-// V: working type (double, or float for the FP32 viscous form); inputs and
-// outputs in global memory stay double.
-template <class C, int PHYS, bool NODAL, class V = double, bool TC = false>
-__global__ void __launch_bounds__(C::NT, NsCfg<C, V>::GRAD_MINB) ns_grad_kernel(StageArgs a) {
+// The working type is float; inputs and outputs in global memory stay double.
+template <class C, int PHYS, bool NODAL>
+__global__ void __launch_bounds__(C::NT, NsCfg<C, float>::GRAD_MINB) ns_grad_kernel(StageArgs a) {
+  using V = float;
   using N = NsCfg<C, V>;
   using R = typename N::Grad;
   constexpr int DIM = C::DIM, NF = C::NF, Q = C::Q, L = C::L, EPB = C::EPB, QD = C::QD, GF = C::GF;
@@ -379,23 +380,17 @@ __global__ void __launch_bounds__(C::NT, NsCfg<C, V>::GRAD_MINB) ns_grad_kernel(
   int *eid = reinterpret_cast<int *>(lnk + EPB * NFACE);
   const int tid = threadIdx.x, e0 = blockIdx.x * EPB;
   load_geo_slots<C>(geo, lnk, eid, a, e0, tid);
-  if constexpr (R::F32) {
-    load_state_shifted<C>(NODAL ? B : A, Rs, NODAL ? a.Xn : a.X, NODAL, e0, a.ne, tid);
-  } else if constexpr (NODAL) {
-    load_nodal_v<C>(B, a.Xn, e0, a.ne, tid);
-  } else {
-    load_modal_v<C>(A, a.X, e0, a.ne, tid);
-  }
+  load_state_shifted<C>(NODAL ? B : A, Rs, NODAL ? a.Xn : a.X, NODAL, e0, a.ne, tid);
   if constexpr (!R::TRG) load_own_traces_v<C>(E, a.Tin, e0, a.ne, tid);
   __syncthreads();
   if constexpr (!R::TRG) load_nbr_traces<C>(E2, a.Tin, lnk, eid, geo, a, tid);
   if constexpr (!NODAL) {
     __syncthreads();
     if constexpr (N::NB1 == NF) {
-      backward_batch<C, NF, V, TC>(A, B, S1, S2, tid);
+      backward_batch<C, NF, V>(A, B, S1, S2, tid);
     } else {   // one slot: fields [0, NB1) then [NB1, NF)
-      backward_batch<C, N::NB1, V, TC>(A, B, S1, S2, tid);
-      backward_batch<C, NF - N::NB1, V, TC>(A + N::NB1 * LD, B + N::NB1 * QD, S1, S2, tid);
+      backward_batch<C, N::NB1, V>(A, B, S1, S2, tid);
+      backward_batch<C, NF - N::NB1, V>(A + N::NB1 * LD, B + N::NB1 * QD, S1, S2, tid);
     }
   }
   __syncthreads();
@@ -403,31 +398,23 @@ __global__ void __launch_bounds__(C::NT, NsCfg<C, V>::GRAD_MINB) ns_grad_kernel(
     // primitive component c at the GLL points
     for (int w = tid; w < EPB * QD; w += C::NT) {
       const int s = w / QD, p = w - s * QD;
-      if constexpr (R::F32) {
-        // B holds rho' = rho - rb, the momenta and E' = E - Eb; with
-        // rho = rb + rho', E/rho - Eb/rb = (E' rb - Eb rho') / (rb rho), so
-        // e - Eb/rb (a per-element constant shift, invisible to the gradient)
-        // is formed from O(Ma^2) terms
-        const V rb = V(Rs[2 * s]), Eb = V(Rs[2 * s + 1]);
-        const V rp = B[(s * NF) * QD + p], r = rb + rp;
-        if (c < DIM) {
-          Qc[w] = B[(s * NF + 1 + c) * QD + p] / r;
-        } else {
-          V k = V(0.0);
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) {
-            const V u = B[(s * NF + 1 + d) * QD + p] / r;
-            k = fma(u, u, k);
-          }
-          const V Ep = B[(s * NF + NF - 1) * QD + p];
-          Qc[w] = fma(V(-0.5), k, (Ep * rb - Eb * rp) / (rb * r));
-        }
+      // B holds rho' = rho - rb, the momenta and E' = E - Eb; with
+      // rho = rb + rho', E/rho - Eb/rb = (E' rb - Eb rho') / (rb rho), so
+      // e - Eb/rb (a per-element constant shift, invisible to the gradient)
+      // is formed from O(Ma^2) terms
+      const V rb = V(Rs[2 * s]), Eb = V(Rs[2 * s + 1]);
+      const V rp = B[(s * NF) * QD + p], r = rb + rp;
+      if (c < DIM) {
+        Qc[w] = B[(s * NF + 1 + c) * QD + p] / r;
       } else {
-        V U[5], q[4];
+        V k = V(0.0);
 #pragma unroll
-        for (int n = 0; n < NF; ++n) U[n] = B[(s * NF + n) * QD + p];
-        primitive<DIM>(U, q);
-        Qc[w] = q[c];
+        for (int d = 0; d < DIM; ++d) {
+          const V u = B[(s * NF + 1 + d) * QD + p] / r;
+          k = fma(u, u, k);
+        }
+        const V Ep = B[(s * NF + NF - 1) * QD + p];
+        Qc[w] = fma(V(-0.5), k, (Ep * rb - Eb * rp) / (rb * r));
       }
     }
     // lift inputs ({{q_c}} - q_c) J n_d per face point, master-frame average
@@ -474,10 +461,10 @@ __global__ void __launch_bounds__(C::NT, NsCfg<C, V>::GRAD_MINB) ns_grad_kernel(
     __syncthreads();
     // collocation derivatives along r, s, t
     using Sh = Sh3<DIM, Q>;
-    vcontract<TC, Sh::a, Sh::b, Sh::c, 0, Q, Q, MatD<L, Q, V>, false>(Qc, Gd, EPB, QD, DIM * QD, tid, C::NT);
-    vcontract<TC, Sh::a, Sh::b, Sh::c, 1, Q, Q, MatD<L, Q, V>, false>(Qc, Gd + QD, EPB, QD, DIM * QD, tid, C::NT);
+    vcontract<Sh::a, Sh::b, Sh::c, 0, Q, Q, MatD<L, Q, V>, false>(Qc, Gd, EPB, QD, DIM * QD, tid, C::NT);
+    vcontract<Sh::a, Sh::b, Sh::c, 1, Q, Q, MatD<L, Q, V>, false>(Qc, Gd + QD, EPB, QD, DIM * QD, tid, C::NT);
     if constexpr (DIM == 3)
-      vcontract<TC, Sh::a, Sh::b, Sh::c, 2, Q, Q, MatD<L, Q, V>, false>(Qc, Gd + 2 * QD, EPB, QD, DIM * QD, tid, C::NT);
+      vcontract<Sh::a, Sh::b, Sh::c, 2, Q, Q, MatD<L, Q, V>, false>(Qc, Gd + 2 * QD, EPB, QD, DIM * QD, tid, C::NT);
     __syncthreads();
     // chain rule (src/Hex.cpp:1994-2006): d/dx = rx d/dr + sx d/ds + tx d/dt
     for (int w = tid; w < EPB * QD; w += C::NT) {
@@ -494,8 +481,8 @@ __global__ void __launch_bounds__(C::NT, NsCfg<C, V>::GRAD_MINB) ns_grad_kernel(
       }
     }
     __syncthreads();
-    lift_batch<C, DIM, V, TC>(Fc, LFc, S1, Gd, tid);
-    forward_batch<C, DIM, V, TC>(Gd, S2, S1, LFc, tid);
+    lift_batch<C, DIM, V>(Fc, LFc, S1, Gd, tid);
+    forward_batch<C, DIM, V>(Gd, S2, S1, LFc, tid);
     for (int w = tid; w < EPB * DIM * LD; w += C::NT) {
       const int s = w / (DIM * LD), rem = w - s * DIM * LD;
       const int e = e0 + s;
@@ -557,7 +544,7 @@ __device__ __forceinline__ void heat_flux(const V *t, V u, V v, V w, V ex, V ey,
 // (Gh = X holds one component's modal gradient), the stresses in place, the
 // energy gradient into the heat-flux slots, then the heat flux in place.
 // The arithmetic of every value is that of the staged path.
-template <class C, bool NODAL, class V, bool TC>
+template <class C, bool NODAL, class V>
 __device__ __forceinline__ void ns_visc_lean_front(const StageArgs &a, V *B, V *Gg, V *X, V *S1, V *S2, int e0,
                                                    int tid) {
   using N = NsCfg<C, V>;
@@ -575,7 +562,7 @@ __device__ __forceinline__ void ns_visc_lean_front(const StageArgs &a, V *B, V *
     for (int w = tid; w < NF * LD; w += C::NT)
       Gg[w] = e >= 0 ? V(a.X[(size_t)e0 * NF * LD + w]) : V(w % LD == 0 ? 1.0 : 0.0);
     __syncthreads();
-    for (int n = 0; n <= DIM; ++n) backward_batch<C, 1, V, TC>(Gg + n * LD, B + n * QD, S1, S2, tid);
+    for (int n = 0; n <= DIM; ++n) backward_batch<C, 1, V>(Gg + n * LD, B + n * QD, S1, S2, tid);
   }
   __syncthreads();
   // velocity gradient: component c, direction d into slot c*DIM + d
@@ -583,7 +570,7 @@ __device__ __forceinline__ void ns_visc_lean_front(const StageArgs &a, V *B, V *
     for (int w = tid; w < DIM * LD; w += C::NT)
       X[w] = e >= 0 ? V(a.Ghat[((size_t)e * NVC + c) * DIM * LD + w]) : V(0.0);
     __syncthreads();
-    for (int d = 0; d < DIM; ++d) backward_batch<C, 1, V, TC>(X + d * LD, Gg + (c * DIM + d) * QD, S1, S2, tid);
+    for (int d = 0; d < DIM; ++d) backward_batch<C, 1, V>(X + d * LD, Gg + (c * DIM + d) * QD, S1, S2, tid);
   }
   const V mu = V(a.vis), gPr = V(a.gamma / a.Pr);
   for (int p = tid; p < QD; p += C::NT) {
@@ -598,7 +585,7 @@ __device__ __forceinline__ void ns_visc_lean_front(const StageArgs &a, V *B, V *
   for (int w = tid; w < DIM * LD; w += C::NT)
     X[w] = e >= 0 ? V(a.Ghat[((size_t)e * NVC + DIM) * DIM * LD + w]) : V(0.0);
   __syncthreads();
-  for (int d = 0; d < DIM; ++d) backward_batch<C, 1, V, TC>(X + d * LD, Gg + (NT6 + d) * QD, S1, S2, tid);
+  for (int d = 0; d < DIM; ++d) backward_batch<C, 1, V>(X + d * LD, Gg + (NT6 + d) * QD, S1, S2, tid);
   for (int p = tid; p < QD; p += C::NT) {
     V t[6], q[3];
 #pragma unroll
@@ -613,8 +600,9 @@ __device__ __forceinline__ void ns_visc_lean_front(const StageArgs &a, V *B, V *
   static_assert(NGS == NT6 + DIM, "stress and heat-flux slots");
 }
 
-template <class C, int PHYS, bool NODAL, class V = double, bool TC = false>
-__global__ void __launch_bounds__(C::NT, NsCfg<C, V>::VISC_MINB) ns_visc_kernel(StageArgs a) {
+template <class C, int PHYS, bool NODAL>
+__global__ void __launch_bounds__(C::NT, NsCfg<C, float>::VISC_MINB) ns_visc_kernel(StageArgs a) {
+  using V = float;
   using N = NsCfg<C, V>;
   using R = typename N::Visc;
   constexpr int DIM = C::DIM, NF = C::NF, Q = C::Q, L = C::L, G = C::G, EPB = C::EPB, QD = C::QD;
@@ -632,17 +620,17 @@ __global__ void __launch_bounds__(C::NT, NsCfg<C, V>::VISC_MINB) ns_visc_kernel(
   const int tid = threadIdx.x, e0 = (a.vtiles ? a.vtiles[blockIdx.x] : (int)blockIdx.x) * EPB;
   load_geo_slots<C>(geo, lnk, eid, a, e0, tid);
   if constexpr (R::LEAN) {
-    ns_visc_lean_front<C, NODAL, V, TC>(a, B, Gg, X, S1, S2, e0, tid);
+    ns_visc_lean_front<C, NODAL, V>(a, B, Gg, X, S1, S2, e0, tid);
   } else if constexpr (NODAL) {
     load_nodal_v<C>(B, a.Xn, e0, a.ne, tid);
   } else {
     load_modal_v<C>(Gg, a.X, e0, a.ne, tid);  // modal input parked in the gradient region
     __syncthreads();
     if constexpr (N::NB1 == NF) {
-      backward_batch<C, NF, V, TC>(Gg, B, S1, S2, tid);
+      backward_batch<C, NF, V>(Gg, B, S1, S2, tid);
     } else {   // one slot: fields [0, NB1) then [NB1, NF)
-      backward_batch<C, N::NB1, V, TC>(Gg, B, S1, S2, tid);
-      backward_batch<C, NF - N::NB1, V, TC>(Gg + N::NB1 * LD, B + N::NB1 * QD, S1, S2, tid);
+      backward_batch<C, N::NB1, V>(Gg, B, S1, S2, tid);
+      backward_batch<C, NF - N::NB1, V>(Gg + N::NB1 * LD, B + N::NB1 * QD, S1, S2, tid);
     }
   }
   if constexpr (!R::LEAN) {
@@ -656,7 +644,7 @@ __global__ void __launch_bounds__(C::NT, NsCfg<C, V>::VISC_MINB) ns_visc_kernel(
       Gh[w] = e < a.ne ? V(a.Ghat[((size_t)e * NVC + c) * DIM * LD + rem]) : V(0.0);
     }
     __syncthreads();
-    backward_batch<C, DIM, V, TC>(Gh, Dv, S1, S2, tid);
+    backward_batch<C, DIM, V>(Gh, Dv, S1, S2, tid);
     if (c < DIM) {
       for (int w = tid; w < EPB * DIM * QD; w += C::NT) {
         const int s = w / (DIM * QD), rem = w - s * DIM * QD;
@@ -722,11 +710,11 @@ __global__ void __launch_bounds__(C::NT, NsCfg<C, V>::VISC_MINB) ns_visc_kernel(
     __syncthreads();
     constexpr int NB = NFACE * EPB * DIM;
     if constexpr (DIM == 3) {
-      vcontract<TC, Q, Q, 1, 0, Q, G, MatGL2G<L, Q, V>, false>(FF, S1, NB, Q * Q, G * Q, tid, C::NT);
+      vcontract<Q, Q, 1, 0, Q, G, MatGL2G<L, Q, V>, false>(FF, S1, NB, Q * Q, G * Q, tid, C::NT);
       __syncthreads();
-      vcontract<TC, G, Q, 1, 1, Q, G, MatGL2G<L, Q, V>, false>(S1, Fg, NB, G * Q, G * G, tid, C::NT);
+      vcontract<G, Q, 1, 1, Q, G, MatGL2G<L, Q, V>, false>(S1, Fg, NB, G * Q, G * G, tid, C::NT);
     } else {
-      vcontract<TC, Q, 1, 1, 0, Q, G, MatGL2G<L, Q, V>, false>(FF, Fg, NB, Q, G, tid, C::NT);
+      vcontract<Q, 1, 1, 0, Q, G, MatGL2G<L, Q, V>, false>(FF, Fg, NB, Q, G, tid, C::NT);
     }
     __syncthreads();
     // g_n . n (own normals), the viscous trace of this side
@@ -753,13 +741,13 @@ __global__ void __launch_bounds__(C::NT, NsCfg<C, V>::VISC_MINB) ns_visc_kernel(
       }
       __syncthreads();
       using Sh = Sh3<DIM, Q>;
-      if (r == 0) vcontract<TC, Sh::a, Sh::b, Sh::c, 0, Q, Q, MatD<L, Q, V>, false>(Cv, Dv, EPB, QD, QD, tid, C::NT);
-      else if (r == 1) vcontract<TC, Sh::a, Sh::b, Sh::c, 1, Q, Q, MatD<L, Q, V>, true>(Cv, Dv, EPB, QD, QD, tid, C::NT);
-      else vcontract<TC, Sh::a, Sh::b, Sh::c, 2, Q, Q, MatD<L, Q, V>, true>(Cv, Dv, EPB, QD, QD, tid, C::NT);
+      if (r == 0) vcontract<Sh::a, Sh::b, Sh::c, 0, Q, Q, MatD<L, Q, V>, false>(Cv, Dv, EPB, QD, QD, tid, C::NT);
+      else if (r == 1) vcontract<Sh::a, Sh::b, Sh::c, 1, Q, Q, MatD<L, Q, V>, true>(Cv, Dv, EPB, QD, QD, tid, C::NT);
+      else vcontract<Sh::a, Sh::b, Sh::c, 2, Q, Q, MatD<L, Q, V>, true>(Cv, Dv, EPB, QD, QD, tid, C::NT);
       __syncthreads();
     }
     // projected divergence of this field
-    forward_batch<C, 1, V, TC>(Dv, S2, S1, FF, tid);
+    forward_batch<C, 1, V>(Dv, S2, S1, FF, tid);
     for (int w = tid; w < EPB * LD; w += C::NT) {
       const int s = w / LD, m = w - s * LD;
       const int e = e0 + s;
