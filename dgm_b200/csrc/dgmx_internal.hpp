@@ -358,6 +358,7 @@ struct FusedOps {
   cudaError_t (*launch)(const StageArgs *args, int narena, const int *bodies, const int2 *items,
                         const int *nitems, int stage, int grid, cudaStream_t s);
   int (*epb)(int body);                  // elements per tile of a body
+  bool (*pair)(int body);                // whether an item may be two tiles
 };
 const FusedOps &fused_ops_fp64();
 const FusedOps &fused_ops_mixed();

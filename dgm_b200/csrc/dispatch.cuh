@@ -678,19 +678,31 @@ struct Launch2DNs {
   }
 };
 
-// 2-D tiles of one (physics, p, q): 128 threads (the default) and half of it,
-// and 256, where every interval's tasks run side by side, for a mesh of one
-// CTA per SM or less (16 x 16, p = 4: 6.5 us a stage against 7.4).
+// 2-D tiles of one (physics, p, q): E elements (128 modal rows) at 128 threads;
+// 256, where every interval's tasks run side by side, for a mesh of one CTA per
+// SM or less (16 x 16, p = 4: 6.5 us a stage against 7.4); and 64.  In FP64,
+// where the registers hold an SM to 16 warps, eight 64-thread CTAs of E elements
+// have twice the elements in flight, two rounds of rows per interval to hide
+// loads and FP64 chains behind: the default above what one wave of 128-thread
+// CTAs holds (p = 4, 128 / 64 threads: 50 x 50 10.5 / 13.6, 60 x 60 16.4 / 14.9,
+// 100 x 100 25.4 / 22.9, 300 x 300 209 / 176 us a stage; p = 2, 300 x 300 91 /
+// 80), unless fewer than seven fit the shared memory (p = 7, 90 x 90: 50 / 54).
 template <int PHYS, int P, int Q, bool MIXED = false>
 void reg2d() {
   constexpr int E = stage2d_epb(phys_nf(PHYS), P + 1), B = MIXED ? 6 : 4;
   const int key = PHYS + (MIXED ? kMixedKey : 0);
-  register_ops(key, P + 1, Q, Launch2D<PHYS, P + 1, Q, MIXED, E, 128, B>::ops());
-  register_ops(key, P + 1, Q, Launch2D<PHYS, P + 1, Q, MIXED, (E + 1) / 2, 64, 2 * B>::ops());
-  KernelOps o = Launch2D<PHYS, P + 1, Q, MIXED, E, 256, 1>::ops();
-  o.preferred = 0;
-  o.small = 148 * E;
-  register_ops(key, P + 1, Q, o);
+  using Half = Launch2D<PHYS, P + 1, Q, MIXED, MIXED ? (E + 1) / 2 : E, 64, 2 * B>;
+  KernelOps wide = Launch2D<PHYS, P + 1, Q, MIXED, E, 256, 1>::ops(),
+            full = Launch2D<PHYS, P + 1, Q, MIXED, E, 128, B>::ops(), half = Half::ops();
+  wide.preferred = half.preferred = 0;
+  wide.small = 148 * E;
+  if (!MIXED && 7 * (half.smem + 1024) <= 228 * 1024) {
+    half.preferred = 2;
+    full.small = 148 * B * E;
+  }
+  register_ops(key, P + 1, Q, wide);
+  register_ops(key, P + 1, Q, full);
+  register_ops(key, P + 1, Q, half);
 }
 template <int PHYS, int P, int Q>
 void reg2d_ns() {

@@ -22,12 +22,20 @@ constexpr int kFusedThreads = 128;
 // CTAs per SM the register allocation is held to
 constexpr int kFusedMinBlocks64 = 4, kFusedMinBlocksMixed = 5;
 
+// A work item is a tile of an arena, or, in FP32 and in a pool of more tiles
+// than the grid has CTAs, two tiles of a solve that follow one another where
+// their shared memory leaves the CTAs per SM as they are: a barrier interval
+// then has two rounds of modal rows to hide its loads behind (24 solves of 8 to
+// 64 elements a side, 40 steps: 27.8 -> 26.0 ms; FP64, with its bodies' spills,
+// 42 -> 46).
 template <bool MIXED, int B>
 struct FusedCfg {
   static constexpr int PHYS = B < 7 ? DGMX_EULER2D : DGMX_SHALLOW;
   static constexpr int P = B % 7 + 1, L = P + 1, Q = P + 2;
   static constexpr int EPB = stage2d_epb(phys_nf(PHYS), L);
-  using C = CfgD<PHYS, L, Q, EPB, kFusedThreads, 0, MIXED>;
+    static constexpr bool PAIR =
+      MIXED && CfgD<PHYS, L, Q, 2 * EPB, kFusedThreads, 0, MIXED>::SMEM <= 228 * 1024 / kFusedMinBlocksMixed - 1024;
+  using C = CfgD<PHYS, L, Q, PAIR ? 2 * EPB : EPB, kFusedThreads, 0, MIXED>;
 };
 
 template <bool MIXED, int B = 0>
@@ -41,21 +49,22 @@ constexpr size_t fused_smem() {
 }
 
 template <bool MIXED, int B = 0>
-__device__ __forceinline__ void fused_dispatch(int body, unsigned char *raw, const StageArgs &a, int tile,
+__device__ __forceinline__ void fused_dispatch(int body, unsigned char *raw, const StageArgs &a, int item,
                                                int tid) {
   if constexpr (B < kFusedBodies) {
     if (body == B) {
       using F = FusedCfg<MIXED, B>;
-      SmemD<typename F::C> sm(raw);
-      stage2d_tile<typename F::C, F::PHYS>(sm, a, tile * F::EPB, tid);
+      const int e0 = item / 2 * F::EPB, end = e0 + (item % 2 ? 2 : 1) * F::EPB;
+      SmemD<typename F::C> sm(raw, end < a.ne ? end : a.ne);
+      stage2d_tile<typename F::C, F::PHYS>(sm, a, e0, tid);
     } else {
-      fused_dispatch<MIXED, B + 1>(body, raw, a, tile, tid);
+      fused_dispatch<MIXED, B + 1>(body, raw, a, item, tid);
     }
   }
 }
 
 // args: [stage][arena] stage arguments; bodies[arena]: body index;
-// items[0 .. *nitems): (arena, tile) pairs.
+// items[0 .. *nitems): (arena, 2 tile + (1: and the tile behind it)).
 template <bool MIXED>
 __global__ void __launch_bounds__(kFusedThreads, MIXED ? kFusedMinBlocksMixed : kFusedMinBlocks64) fused_stage_kernel(const StageArgs *args, int narena,
                                                                        const int *bodies, const int2 *items,
@@ -90,6 +99,12 @@ template <bool MIXED, int B = 0>
 constexpr int fused_epb(int body) {
   if constexpr (B < kFusedBodies) return body == B ? FusedCfg<MIXED, B>::EPB : fused_epb<MIXED, B + 1>(body);
   else return 1;
+}
+
+template <bool MIXED, int B = 0>
+constexpr bool fused_pair(int body) {
+  if constexpr (B < kFusedBodies) return body == B ? FusedCfg<MIXED, B>::PAIR : fused_pair<MIXED, B + 1>(body);
+  else return false;
 }
 
 template <bool MIXED>

@@ -5,7 +5,8 @@ namespace dgmx {
 
 const FusedOps &fused_ops_mixed() {
   static const FusedOps ops{FusedHost<true>::init, FusedHost<true>::blocks_per_sm, FusedHost<true>::launch,
-                            [](int body) { return fused_epb<true>(body); }};
+                            [](int body) { return fused_epb<true>(body); },
+                            [](int body) { return fused_pair<true>(body); }};
   return ops;
 }
 

@@ -193,7 +193,7 @@ struct dgmx_pool {
   StageArgs *args_dev = nullptr, *args_pin = nullptr;   // [14][arenas]
   int args_cap = 0;                                     // arenas the table holds
   int *bodies_dev = nullptr, *bodies_pin = nullptr;
-  int2 *items_dev = nullptr, *items_pin = nullptr;      // (arena, tile)
+  int2 *items_dev = nullptr, *items_pin = nullptr;      // (arena, 2 tile + pair)
   int *nitems_dev = nullptr, *nitems_pin = nullptr;
   int items_cap = 0, fgrid = 1;
   cudaGraphExec_t fgraph = nullptr;
@@ -689,12 +689,19 @@ dgmx_status fused_upload(dgmx_pool *P) {
       return (size_t)P->arenas[x]->nf * P->arenas[x]->qd * P->arenas[x]->epb >
              (size_t)P->arenas[y]->nf * P->arenas[y]->qd * P->arenas[y]->epb;
     });
+    size_t ntile = 0;
+    for (int ai : order)
+      for (int id : P->arenas[ai]->live) ntile += P->solves[id].nalloc / P->arenas[ai]->epb;
+    // more tiles than CTAs: two tiles per item (fused.cuh)
     std::vector<int2> items;
     for (int ai : order) {
       const Arena &a = *P->arenas[ai];
+      const bool pair = ntile > (size_t)P->fgrid && P->fops->pair(a.body);
       for (int id : a.live) {
         const PoolSolve &sv = P->solves[id];
-        for (int t = sv.e0 / a.epb; t < (sv.e0 + sv.nalloc) / a.epb; ++t) items.push_back(make_int2(ai, t));
+        const int t1 = (sv.e0 + sv.nalloc) / a.epb;
+        for (int t = sv.e0 / a.epb; t < t1; t += pair ? 2 : 1)
+          items.push_back(make_int2(ai, 2 * t + (pair && t + 1 < t1)));
       }
     }
     if ((int)items.size() > P->items_cap) {

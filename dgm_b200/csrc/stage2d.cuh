@@ -53,7 +53,8 @@ struct SmemD {
   T *base;
   int *eid, *cls;
   RefState<T> *ref;
-  __device__ SmemD(unsigned char *raw) {
+  int end;   // first element behind the tile's own
+  __device__ SmemD(unsigned char *raw, int end_) : end(end_) {
     base = reinterpret_cast<T *>(raw);
     eid = reinterpret_cast<int *>(raw + C::DATA);
     cls = eid + C::EPB;
@@ -65,7 +66,7 @@ struct SmemD {
 template <class C>
 __device__ __forceinline__ void sd_load(const SmemD<C> &sm, const StageArgs &a, int e0, int tid) {
   for (int s = tid; s < C::EPB; s += C::NT) {
-    const int e = e0 + s, c = e < a.ne ? a.links[(size_t)e * 4].cls : -1;   // -1: unallocated
+    const int e = e0 + s, c = e < sm.end ? a.links[(size_t)e * 4].cls : -1;   // -1: unallocated
     sm.cls[s] = c >= 0 ? c : 0;
     sm.eid[s] = c >= 0 ? e : -1;
     if constexpr (C::MIXED)
@@ -100,7 +101,7 @@ __device__ __forceinline__ void sd_face_point(const SmemD<C> &sm, const StageArg
   using T = typename C::R;
   constexpr int NF = C::NF, G = C::G;
   const int s = w / (4 * G), rem = w - s * 4 * G, f = rem / G, g = rem - f * G, e = e0 + s;
-  if (e >= a.ne) return;
+  if (e >= sm.end) return;
   const int cls = __ldg(&a.links[(size_t)e * 4].cls);
   if (cls < 0) return;   // unallocated
   const FaceLink *lp = a.links + (size_t)e * 4 + f;
@@ -161,7 +162,7 @@ __device__ __forceinline__ void sd_state_row(const SmemD<C> &sm, const StageArgs
   using T = typename C::R;
   constexpr int L = C::L, Q = C::Q, RPS = C::NF * L;
   const int s = w / RPS, r = w - s * RPS, e = e0 + s;
-  if (e >= a.ne) return;
+  if (e >= sm.end) return;
   double x[L];
   ld_row<L>(a.X + ((size_t)e * RPS + r) * L, x);
   if constexpr (C::MIXED)
@@ -474,7 +475,7 @@ __device__ __forceinline__ void stage2d_tile(const SmemD<C> &sm, const StageArgs
 template <class C, int PHYS>
 __global__ void __launch_bounds__(C::NT, C::MINB) stage2d_kernel(StageArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  SmemD<C> sm(smem_raw);
+  SmemD<C> sm(smem_raw, a.ne);
   pdl_release();
   const int ntile = a.tiles ? *a.ntiles : (int)gridDim.x;
   for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
@@ -492,7 +493,7 @@ template <class C, int PHYS, bool SELF>
 __global__ void __launch_bounds__(C::NT, C::MINB) rhs2d_kernel(StageArgs a) {
   constexpr int NT = C::NT, L = C::L, Q = C::Q, RPS = C::NF * L;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  SmemD<C> sm(smem_raw);
+  SmemD<C> sm(smem_raw, a.ne);
   const int tid = threadIdx.x, e0 = blockIdx.x * C::EPB;
   sd_front<C, PHYS, true, SELF>(sm, a, e0, tid);
   for (int w = tid; w < C::EPB * RPS; w += NT) {
