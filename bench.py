@@ -728,7 +728,7 @@ def run_partitioned(args, torch, dgm_b200, dist, rank, world, local):
         _, kind = D.set_variant(pick)
         D.set_state(U_ic)
         tiles[name] = {"variant": pick,
-                       "kernel": {2: "stage_pipe_kernel", 3: "stage2_kernel"}.get(kind, "stage_kernel"),
+                       "kernel": {2: "stage_pipe_kernel", 3: "stage2_kernel"}.get(kind, "stage3_kernel"),
                        "elements_per_cta": int(rows[pick][0]), "min_ctas_per_sm": int(rows[pick][1]),
                        "threads_per_cta": int(rows[pick][2])}
         doms[name] = D
@@ -866,7 +866,7 @@ def main():
             pick = args.variant
         _, kind = D.set_variant(pick)
         tiles[name] = {"variant": pick,
-                       "kernel": {2: "stage_pipe_kernel", 3: "stage2_kernel"}.get(kind, "stage_kernel"),
+                       "kernel": {2: "stage_pipe_kernel", 3: "stage2_kernel"}.get(kind, "stage3_kernel"),
                        "elements_per_cta": int(rows[pick][0]), "min_ctas_per_sm": int(rows[pick][1]),
                        "threads_per_cta": int(rows[pick][2]), "candidates_us": [round(float(r[3]), 1) for r in rows]}
         doms[name] = D
