@@ -7,6 +7,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -1556,8 +1557,13 @@ dgmx_status dgmx_time_derivative_device(dgmx_domain *d, const double *U_dev, dou
   cudaError_t e = cudaSuccess;
   dgmx_status xs = DGMX_OK;
   // the own and neighbour traces, unless the tile interpolates both itself
-  // (ghost slots of a partition hold traces only)
-  if (!rhs->self_traces || d->partitioned()) {
+  // (ghost slots of a partition hold traces only).  In place, a tile's stores
+  // would reach U_dev before its neighbours' tiles have interpolated from it;
+  // with the traces written first, a tile reads its own elements alone.
+  const uintptr_t u0 = reinterpret_cast<uintptr_t>(U_dev), f0 = reinterpret_cast<uintptr_t>(F_dev);
+  const size_t span = sizeof(double) * d->nnodal();
+  const bool overlap = u0 < f0 + span && f0 < u0 + span;
+  if (!rhs->self_traces || d->partitioned() || overlap) {
     a.Tout = d->T[d->tcur ^ 1];
     e = rhs->traces_nodal(a, d->stream);
     ++d->launches;

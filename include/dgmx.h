@@ -265,7 +265,9 @@ const char *dgmx_restart_last_error(void);
 /* Domain::time_derivative(U, F) (src/Domain.hpp:243): F = -dU/dt at GLL
  * points, projected, for U given at GLL points.  Host buffers, Field layout. */
 dgmx_status dgmx_time_derivative(dgmx_domain *d, const double *U, double *F);
-/* Same with device buffers (Field layout), enqueued on the handle's stream. */
+/* Same with device buffers (Field layout), enqueued on the handle's stream.
+ * F_dev may be U_dev (in place); buffers that overlap in part give wrong
+ * values. */
 dgmx_status dgmx_time_derivative_device(dgmx_domain *d, const double *U_dev, double *F_dev);
 
 /* TimeInt::advance repeated nsteps times with a fixed dt (TVD3:
