@@ -126,7 +126,7 @@ __device__ __forceinline__ T end_value(int end, int m) {
 }
 
 
-// ---- the tile's links, class and (mixed form) reference state ----------------
+// ---- the tile's links and class -----------------------------------------------
 template <class C>
 __device__ __forceinline__ void s2_load(const Smem2<C> &sm, const StageArgs &a, int e0, int tid) {
   constexpr int NFACE = C::NFACE, EPB = C::EPB;
@@ -138,10 +138,17 @@ __device__ __forceinline__ void s2_load(const Smem2<C> &sm, const StageArgs &a, 
       const int gc = e < a.ne ? a.gclass[e] : -1;
       sm.cls[s] = gc >= 0 ? gc : 0;
       sm.eid[s] = gc >= 0 ? e : -1;
-      if constexpr (C::MIXED)
-        sm.ref[s] = *reinterpret_cast<const RefState<float> *>(a.uref + kUrefStride * solve_of(a, gc >= 0 ? e : -1) + 10);
     }
   }
+}
+// ---- and (mixed form) reference state, which kernels write: after pdl_wait ------
+template <class C>
+__device__ __forceinline__ void s2_load_ref(const Smem2<C> &sm, const StageArgs &a, int tid) {
+  if constexpr (C::MIXED)
+    for (int w = tid; w < C::EPB * C::NFACE; w += C::NT)
+      if (w % C::NFACE == 0)   // the thread that wrote eid
+        sm.ref[w / C::NFACE] =
+            *reinterpret_cast<const RefState<float> *>(a.uref + kUrefStride * solve_of(a, sm.eid[w / C::NFACE]) + 10);
 }
 
 // ---- interval 1a: numerical flux at every face point --------------------------
@@ -780,6 +787,7 @@ template <class C, int PHYS>
 __device__ __forceinline__ void stage2_tile(const Smem2<C> &sm, const StageArgs &a, int e0, int tid) {
   s2_load<C>(sm, a, e0, tid);
   pdl_wait();
+  s2_load_ref<C>(sm, a, tid);
   __syncthreads();
   s2_interval1<C, PHYS>(sm, a, e0, tid);
   __syncthreads();

@@ -69,9 +69,14 @@ __device__ __forceinline__ void sd_load(const SmemD<C> &sm, const StageArgs &a, 
     const int e = e0 + s, c = e < sm.end ? a.links[(size_t)e * 4].cls : -1;   // -1: unallocated
     sm.cls[s] = c >= 0 ? c : 0;
     sm.eid[s] = c >= 0 ? e : -1;
-    if constexpr (C::MIXED)
-      sm.ref[s] = *reinterpret_cast<const RefState<float> *>(a.uref + kUrefStride * solve_of(a, c >= 0 ? e : -1) + 10);
   }
+}
+// The mixed form's reference state, which kernels write: after pdl_wait.
+template <class C>
+__device__ __forceinline__ void sd_load_ref(const SmemD<C> &sm, const StageArgs &a, int tid) {
+  if constexpr (C::MIXED)
+    for (int s = tid; s < C::EPB; s += C::NT)
+      sm.ref[s] = *reinterpret_cast<const RefState<float> *>(a.uref + kUrefStride * solve_of(a, sm.eid[s]) + 10);
 }
 
 // Trace values of GLL values (Field layout) at Gauss point g of face f of
@@ -443,6 +448,7 @@ __device__ __forceinline__ void sd_front(const SmemD<C> &sm, const StageArgs &a,
   constexpr int NT = C::NT, NC = C::EPB * C::Q;
   sd_load<C>(sm, a, e0, tid);
   pdl_wait();
+  sd_load_ref<C>(sm, a, tid);
   for (int w = tid; w < C::EPB * 4 * C::G; w += NT) sd_face_point<C, PHYS, SELF>(sm, a, e0, w);
   // from the last thread down: a tile with threads enough for both does the
   // rows beside the face points
