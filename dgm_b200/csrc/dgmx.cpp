@@ -1718,9 +1718,10 @@ int dgmx_kernel_list(int *rows, int cap) {
 
 // Autotuner: times every compiled tile variant (elements per CTA, register
 // cap) of this handle's (physics, L, Q) on the handle's own mesh with
-// right-hand-side-only stage launches (the state is not modified) and keeps
-// the fastest.  rows (optional, cap rows of 4 doubles): epb, minb, threads,
-// microseconds per launch.  Returns the variant count in *nvariants and the
+// right-hand-side-only stages (the state is not modified; Navier-Stokes: the
+// viscous kernels and the stage kernel) and keeps the fastest.  rows
+// (optional, cap rows of 4 doubles): epb, minb, threads, microseconds per
+// stage.  Returns the variant count in *nvariants and the
 // chosen index in *chosen.
 dgmx_status dgmx_autotune(dgmx_domain *d, int reps, double *rows, int cap, int *nvariants, int *chosen) {
   if (!d || reps <= 0) return DGMX_ERR_ARGUMENT;
@@ -1750,15 +1751,15 @@ dgmx_status dgmx_autotune(dgmx_domain *d, int reps, double *rows, int cap, int *
     a.kind = kRHS; a.X = d->U; a.U = d->U; a.Ut = d->Ut; a.A = scratch;
     a.Tin = d->T[d->tcur]; a.Tout = d->T[d->tcur ^ 1];
     if (d->mixed()) { a.Utf = d->Utf; a.Tinf = d->Tf[d->tcur]; a.Toutf = d->Tf[d->tcur ^ 1]; }
-    // Navier-Stokes: with the tile's viscous kernels (the tensor-core form's
-    // are fixed, and so is the stage kernel that goes with them)
+    // Navier-Stokes: with the viscous kernels of the handle's form, which come
+    // from the tile too.  The tensor-core form runs the same kernels whatever
+    // the tile: they are timed, and the tile stays.
+    const KernelOps &k = d->visc_tc ? *v.tensor : v;
     auto pass = [&]() {
       cudaError_t q = cudaSuccess;
-      if (d->ns() && !d->visc32) {
-        if (v.ns_grad) q = v.ns_grad(a, false, d->stream);
-        if (q == cudaSuccess) q = v.ns_visc(a, false, d->stream);
-      }
-      return q == cudaSuccess ? v.stage(a, d->stream) : q;
+      if (d->visc_tc) q = k.ns_grad32(a, false, d->stream);
+      if (d->ns() && q == cudaSuccess) q = (d->visc32 ? k.ns_visc32 : k.ns_visc)(a, false, d->stream);
+      return q == cudaSuccess ? k.stage(a, d->stream) : q;
     };
     for (int w = 0; w < 2 && e == cudaSuccess; ++w) e = pass();
     cudaEventRecord(e0, d->stream);
@@ -1766,14 +1767,14 @@ dgmx_status dgmx_autotune(dgmx_domain *d, int reps, double *rows, int cap, int *
     cudaEventRecord(e1, d->stream);
     if (e == cudaSuccess) e = cudaEventSynchronize(e1);
     if (e != cudaSuccess) { st = d->cuda(e, "autotune launch"); break; }
-    d->launches += 2 + reps;
+    d->launches += (long)(2 + reps) * (d->ns() ? (d->visc_tc ? 3 : 2) : 1);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
     ms /= reps;
     if ((int)i < cap && rows) {
       rows[4 * i + 0] = v.epb; rows[4 * i + 1] = v.minb; rows[4 * i + 2] = v.nt; rows[4 * i + 3] = 1e3 * ms;
     }
-    if (best < 0 || ms < best_ms) { best = (int)i; best_ms = ms; }
+    if (d->visc_tc ? &v == d->ops : best < 0 || ms < best_ms) { best = (int)i; best_ms = ms; }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
