@@ -799,9 +799,9 @@ __device__ __forceinline__ void ns3_grad_k(const T *w0, const T *X, const double
 // projected divergence (a.Pv, [e][n][L^3]) and the viscous normal-flux
 // traces (a.V).  NODAL: the state comes from GLL values (a.Xn).  F32: the
 // gradients and stresses in FP32 (precision = DGMX_MIXED); the primitive
-// variables are formed in FP64 and rounded, the internal energy as its
-// difference from the element's first point (a constant the gradient does
-// not see: e ~ 1/(gamma (gamma-1) Ma^2) against variations of O(1)).
+// variables are formed in FP64 and rounded as their differences from the
+// element's middle point (constants the gradient does not see: for the internal
+// energy 1/(gamma (gamma-1) Ma^2) against variations of O(1)).
 template <class C, int PHYS, bool NODAL, bool F32>
 __global__ void __launch_bounds__(C::NT, C::MINB) ns_flux_kernel(StageArgs a) {
   using N = NsFlux<C>;
@@ -848,13 +848,14 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns_flux_kernel(StageArgs a) {
     F2 *W2 = reinterpret_cast<F2 *>(W), *X2 = reinterpret_cast<F2 *>(X);
     f3_lift_cols<C>(X2, X2, 12, tid);
     // gradient of the pairs (u, v) and (w, e), pair c in W2[3c .. 3c+2]
-    const double eref = U[4 * BS];
+    constexpr int MID = (Q / 2) * (SI + SJ + 1);
     pencils_i<C>(2, tid, [&](int c, int jk) {
+      const double *f = U + (1 + 2 * c) * BS, r0 = f[MID], r1 = f[BS + MID];
       F2 v[Q];
 #pragma unroll
       for (int i = 0; i < Q; ++i) {
-        const double *p = U + (1 + 2 * c) * BS + jk + i * SI;
-        v[i] = F2(float(p[0]), float(c == 0 ? p[BS] : p[BS] - eref));
+        const double *p = f + jk + i * SI;
+        v[i] = F2(float(p[0] - r0), float(p[BS] - r1));
       }
       ns3_grad_i<C>(v, W2 + 3 * c * BS + jk, W2 + (3 * c + 1) * BS + jk);
     });

@@ -709,11 +709,11 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns2d_flux_kernel(StageArgs a) 
       const int s = w / (2 * Q), r = w - s * 2 * Q, c = r / Q, j = r - c * Q;
       if (eid[s] < 0) continue;
       const double *p = slot(s) + (c == 0 ? BS : 3 * BS) + j;
-      const double eref = slot(s)[3 * BS];
+      // differences from the middle point, as in ns_flux_kernel
+      const double *mid = slot(s) + (c == 0 ? BS : 3 * BS) + (Q / 2) * (PQ + 1), r0 = mid[0], r1 = c == 0 ? mid[BS] : 0.0;
       F2 v[Q];
 #pragma unroll
-      for (int i = 0; i < Q; ++i)
-        v[i] = c == 0 ? F2(float(p[i * PQ]), float(p[BS + i * PQ])) : F2(float(p[i * PQ] - eref), 0.0f);
+      for (int i = 0; i < Q; ++i) v[i] = F2(float(p[i * PQ] - r0), c == 0 ? float(p[BS + i * PQ] - r1) : 0.0f);
       F2 *W = reinterpret_cast<F2 *>(slot(s) + N::O_W) + 2 * c * BS + j;
       ns2_grad_i<C>(v, W, W + BS);
     }
