@@ -640,9 +640,9 @@ struct Launch2DNs {
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     };
     attr(ns2d_flux_kernel<C, PHYS, false, false>, N::SMEM);
-    attr(ns2d_flux_kernel<C, PHYS, true, false>, N::SMEM);
+    attr(ns2d_flux_kernel<C, PHYS, true, false>, N::SMEM_NODAL);
     attr(ns2d_flux_kernel<C, PHYS, false, true>, N::SMEM);
-    attr(ns2d_flux_kernel<C, PHYS, true, true>, N::SMEM);
+    attr(ns2d_flux_kernel<C, PHYS, true, true>, N::SMEM_NODAL);
     attr(stage2d_kernel<C, PHYS>, C::SMEM);
     attr(rhs2d_kernel<C, PHYS, false>, C::SMEM);
     return e;
@@ -651,7 +651,7 @@ struct Launch2DNs {
   static cudaError_t flux(const StageArgs &a, bool nodal, cudaStream_t s) {
     const unsigned g = a.vtiles ? a.nvtiles : (a.ne + EPB - 1) / EPB;
     return launch_dependent(nodal ? ns2d_flux_kernel<C, PHYS, true, F32> : ns2d_flux_kernel<C, PHYS, false, F32>, g, NT,
-                            N::SMEM, s, a);
+                            nodal ? N::SMEM_NODAL : N::SMEM, s, a);
   }
   static cudaError_t stage_grid(const StageArgs &a, int g, cudaStream_t s) {
     return launch_dependent(stage2d_kernel<C, PHYS>, (unsigned)g, NT, C::SMEM, s, a);

@@ -75,6 +75,9 @@ struct Geo3 {
   double tv[6];      // n = tv metric[r] on face f
   double jr[6];
   double nrm[6][3], onrm[6][3];
+  double mean[5];    // a state of the element (Navier-Stokes: mean[0] a pressure)
+  double c[15];      // FP64: constants of its fluxes (direction r, field n at 5 r + n);
+                     // the mixed form: the reference state of its volume term
   int master, bc, cls;
   FaceLink lnk[6];
 };
@@ -187,17 +190,20 @@ __device__ __forceinline__ void f3_expand_k(T *buf, int nbuf, int tid) {
     st_pencil<C::Q>(p, 1, u);
   });
 }
-// k pass of the state from the modal rows in global memory (the mixed form
-// takes the solve's reference state out of the constant mode first).
+// k pass of the state from the modal rows in global memory.  The mixed form
+// leaves the constant mode out: its value goes to mean[n].
 template <class C>
-__device__ __forceinline__ void f3_state_k(typename C::R *buf, const StageArgs &a, int e, int tid) {
+__device__ __forceinline__ void f3_state_k(typename C::R *buf, double *mean, const StageArgs &a, int e, int tid) {
   using T = typename C::R;
   pencils_k<C>(C::NF, tid, [&](int n, int o, int aa, int b) {
     const int r = (n * C::L + aa) * C::L + b;
     double x[C::L];
     ld_row<C::L>(a.X + ((size_t)e * (C::NF * C::L * C::L) + r) * C::L, x);
     if constexpr (C::MIXED)
-      if (aa == 0 && b == 0) x[0] -= a.uref[kUrefStride * solve_of(a, e) + 5 + n];
+      if (aa == 0 && b == 0) {
+        mean[n] = 0.35355339059327379 * x[0];   // 2^(-3/2)
+        x[0] = 0.0;
+      }
     T v[C::L], u[C::Q];
 #pragma unroll
     for (int c = 0; c < C::L; ++c) v[c] = T(x[c]);
@@ -205,13 +211,16 @@ __device__ __forceinline__ void f3_state_k(typename C::R *buf, const StageArgs &
     st_pencil<C::Q>(buf + n * C::BS + o, 1, u);
   });
 }
-// GLL values of the state in Field layout [n][e][Q^3].
+// GLL values of the state in Field layout [n][e][Q^3]; the middle point's go to
+// mean[n].
 template <class C>
-__device__ __forceinline__ void f3_state_nodal(double *buf, const StageArgs &a, int e, int tid) {
+__device__ __forceinline__ void f3_state_nodal(double *buf, double *mean, const StageArgs &a, int e, int tid) {
   constexpr int Q = C::Q, QD = C::QD;
   for (int w = tid; w < C::NF * QD; w += C::NT) {
     const int n = w / QD, p = w - n * QD, i = p / (Q * Q), jk = p - i * Q * Q, j = jk / Q, k = jk - j * Q;
-    buf[n * C::BS + i * C::SI + j * C::SJ + k] = a.Xn[((size_t)n * a.ne + e) * QD + p];
+    const double v = a.Xn[((size_t)n * a.ne + e) * QD + p];
+    buf[n * C::BS + i * C::SI + j * C::SJ + k] = v;
+    if (p == QD / 2) mean[n] = v;
   }
 }
 
@@ -541,11 +550,11 @@ __device__ __forceinline__ void f3_store_nodal(const double *buf, const StageArg
 
 // ---------------------------------------------------------------------- Euler
 // Contravariant fluxes G_r = metric[r] . F(U) at the points: state buffers
-// 0..4 -> flux buffers 5 r + n, in place point by point.  The mixed form
-// evaluates F(Ub + u') - F(Ub) (volume_flux_pert, kernels.cuh).
-template <class C>
-__device__ __forceinline__ void f3_point_fluxes(typename C::R *G, const Geo3 &g, const RefState<typename C::R> *ref,
-                                                const StageArgs &a, int tid) {
+// 0..4 -> flux buffers 5 r + n, in place point by point; SHIFT: less the
+// constants g.c.  The mixed form evaluates F(Ub + u') - F(Ub)
+// (volume_flux_pert, kernels.cuh) about the element's mean.
+template <class C, bool SHIFT>
+__device__ __forceinline__ void f3_point_fluxes(typename C::R *G, const Geo3 &g, const StageArgs &a, int tid) {
   using T = typename C::R;
   constexpr int Q = C::Q, BS = C::BS;
   const T gm1 = T(a.gamma) - T(1.0);
@@ -559,7 +568,7 @@ __device__ __forceinline__ void f3_point_fluxes(typename C::R *G, const Geo3 &g,
 #pragma unroll
     for (int n = 0; n < 5; ++n) U[n] = p[n * BS];
     if constexpr (C::MIXED) {
-      const RefState<T> &b = *ref;
+      const RefState<T> &b = *reinterpret_cast<const RefState<T> *>(g.c);
       const T ir = p_rcp(b.r + U[0]);
       const T mx = b.m[0] + U[1], my = b.m[1] + U[2], mz = b.m[2] + U[3];
       const T ux = (U[1] - b.u[0] * U[0]) * ir, uy = (U[2] - b.u[1] * U[0]) * ir, uz = (U[3] - b.u[2] * U[0]) * ir;
@@ -590,11 +599,16 @@ __device__ __forceinline__ void f3_point_fluxes(typename C::R *G, const Geo3 &g,
         const T m0 = m[3 * r], m1 = m[3 * r + 1], m2 = m[3 * r + 2];
         const T V = fma(m2, ww, fma(m1, v, m0 * u));
         T *o = p + 5 * r * BS;
-        o[0] = U[0] * V;
-        o[BS] = fma(U[1], V, pr * m0);
-        o[2 * BS] = fma(U[2], V, pr * m1);
-        o[3 * BS] = fma(U[3], V, pr * m2);
-        o[4 * BS] = Ep * V;
+        // a product, or the product less a constant (read each time: held in
+        // registers the constants spill)
+        auto mul = [&](T x, T y, int n) {
+          return SHIFT ? fma(x, y, -*(const volatile double *)(g.c + 5 * r + n)) : x * y;
+        };
+        o[0] = mul(U[0], V, 0);
+        o[BS] = fma(U[1], V, mul(pr, m0, 1));
+        o[2 * BS] = fma(U[2], V, mul(pr, m1, 2));
+        o[3 * BS] = fma(U[3], V, mul(pr, m2, 3));
+        o[4 * BS] = mul(Ep, V, 4);
       }
     }
   }
@@ -616,6 +630,12 @@ __global__ void __launch_bounds__(C::NT, C::MINB) stage3_kernel(StageArgs a) {
   using T = typename C::R;
   using N = Stage3<C>;
   constexpr int L = C::L, BS = C::BS, SI = C::SI, SJ = C::SJ, GF = C::GF;
+  // The constants of FP64 fluxes: on GLL values up to p = 4.  Above, this form
+  // rounds no more than the derivative-first form without (1.31, 1.64, 1.2 times
+  // its distance from a 64-bit evaluation at p = 2, 3, 4, with them 0.86; 1.03 and
+  // 0.87 at p = 5 and 7), nor do stages, whose update of the state rounds more
+  // than the operators (0.99)
+  constexpr bool SHIFT = NODAL && L <= 5;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *U = reinterpret_cast<T *>(smem_raw), *X = U + N::O_X, *W1 = U + 5 * BS;
   Geo3 &g = *reinterpret_cast<Geo3 *>(smem_raw + N::DATA);
@@ -631,7 +651,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) stage3_kernel(StageArgs a) {
     if constexpr (C::MIXED) {
       if (tid == 0) *ref = *reinterpret_cast<const RefState<T> *>(a.uref + kUrefStride * solve_of(a, e) + 10);
     }
-    if constexpr (NODAL) f3_state_nodal<C>(U, a, e, tid); else f3_state_k<C>(U, a, e, tid);
+    if constexpr (NODAL) f3_state_nodal<C>(U, g.mean, a, e, tid); else f3_state_k<C>(U, g.mean, a, e, tid);
     if (const int n = element_ahead<C>(a, e); n >= 0 && !a.tiles) {
       if constexpr (!NODAL) prefetch_span<C::NT>(a.X + (size_t)n * 5 * C::LD, 5 * C::LD * 8, tid);
       prefetch_span<C::NT>(trace_in<C>(a) + (size_t)n * 30 * GF, 30 * GF * (int)sizeof(T), tid);
@@ -642,10 +662,21 @@ __global__ void __launch_bounds__(C::NT, C::MINB) stage3_kernel(StageArgs a) {
     if constexpr (!NODAL) f3_expand_j<C>(U, 5, tid);
     __syncthreads();
     f3_faces<C, PHYS>(X, g, ref, a, e, tid);
+    if constexpr (C::MIXED) {
+      if (tid == C::NT - 1) {
+        T m[5];
+#pragma unroll
+        for (int n = 0; n < 5; ++n) m[n] = T(g.mean[n]);
+        *reinterpret_cast<RefState<T> *>(g.c) = element_reference<PHYS, T>(m, T(a.gamma));
+      }
+    } else if constexpr (NODAL) {
+      const int k = tid - (C::NT - 15);
+      if (SHIFT && k >= 0) g.c[k] = flux_constant<3>(g.mean, g.metric + k / 5 * 3, a.gamma, k % 5);
+    }
     if constexpr (!NODAL) f3_expand_i<C>(U, 5, tid);
     __syncthreads();
     f3_lift_rows<C>(X, 30, tid);
-    f3_point_fluxes<C>(U, g, ref, a, tid);
+    f3_point_fluxes<C, SHIFT>(U, g, a, tid);
     __syncthreads();
     f3_lift_cols<C>(X, X, 30, tid);
     f3_div_i<C>(U, tid);
@@ -795,6 +826,22 @@ __device__ __forceinline__ void ns3_grad_k(const T *w0, const T *X, const double
   }
 }
 
+// Constants of the convective fluxes (pencil.cuh): those of the point at p
+// (density, velocity, internal energy, buffers apart), one per thread k < 15,
+// and its pressure.
+template <class C>
+__device__ __forceinline__ void ns3_flux_constants(const double *p, Geo3 &g, double gamma, int k) {
+  const int r = k / 5, n = k - 5 * r;
+  const float rho = float(p[0]), u = float(p[C::BS]), v = float(p[2 * C::BS]), w = float(p[3 * C::BS]);
+  const float ei = float(p[4 * C::BS]);
+  const float m0 = float(g.metric[3 * r]), m1 = float(g.metric[3 * r + 1]), m2 = float(g.metric[3 * r + 2]);
+  const float V = fmaf(m2, w, fmaf(m1, v, m0 * u)), pr = (float(gamma) - 1.0f) * rho * ei;
+  const float H = fmaf(rho, fmaf(0.5f, fmaf(w, w, fmaf(v, v, u * u)), ei), pr);
+  const float x = n == 1 ? u : (n == 2 ? v : w), mn = n == 1 ? m0 : (n == 2 ? m1 : m2);
+  g.c[k] = flux_constant(n == 0 ? rho * V : (n == 4 ? H * V : fmaf(rho * V, x, pr * mn)));
+  if (k == 0) g.mean[0] = flux_constant(pr);
+}
+
 // One element: state, projected gradients, stresses, volume flux, its
 // projected divergence (a.Pv, [e][n][L^3]) and the viscous normal-flux
 // traces (a.V).  NODAL: the state comes from GLL values (a.Xn).  F32: the
@@ -814,7 +861,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns_flux_kernel(StageArgs a) {
   pdl_release();
   f3_load_links<C>(g, a, e, tid);
   pdl_wait();
-  if constexpr (NODAL) f3_state_nodal<C>(U, a, e, tid); else f3_state_k<C>(U, a, e, tid);
+  if constexpr (NODAL) f3_state_nodal<C>(U, g.mean, a, e, tid); else f3_state_k<C>(U, nullptr, a, e, tid);
   if (const int n = element_ahead<C>(a, e); n >= 0) {
     if constexpr (!NODAL) prefetch_span<NT>(a.X + (size_t)n * 5 * C::LD, 5 * C::LD * 8, tid);
     prefetch_span<NT>(a.Tin + (size_t)n * 30 * GF, 30 * GF * 8, tid);
@@ -844,11 +891,12 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns_flux_kernel(StageArgs a) {
   }
   __syncthreads();
   const double kap = a.gamma / a.Pr * a.vis;
+  constexpr int MID = (Q / 2) * (SI + SJ + 1);
+  if (tid >= NT - 15) ns3_flux_constants<C>(U + MID, g, a.gamma, tid - (NT - 15));
   if constexpr (F32) {
     F2 *W2 = reinterpret_cast<F2 *>(W), *X2 = reinterpret_cast<F2 *>(X);
     f3_lift_cols<C>(X2, X2, 12, tid);
     // gradient of the pairs (u, v) and (w, e), pair c in W2[3c .. 3c+2]
-    constexpr int MID = (Q / 2) * (SI + SJ + 1);
     pencils_i<C>(2, tid, [&](int c, int jk) {
       const double *f = U + (1 + 2 * c) * BS, r0 = f[MID], r1 = f[BS + MID];
       F2 v[Q];
@@ -988,7 +1036,12 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns_flux_kernel(StageArgs a) {
       const double qx = fma(t13, ww, fma(t12, v, fma(t11, u, t[6])));
       const double qy = fma(t23, ww, fma(t22, v, fma(t12, u, t[7])));
       const double qz = fma(t33, ww, fma(t23, v, fma(t13, u, t[8])));
-      const double pr = gm1 * rho * ei;
+      // Less the element's constants (pencil.cuh): all of them on GLL values up
+      // to p = 5; in stages, where the update of the state rounds more, those
+      // that low Mach numbers make large (the pressure, which costs nothing,
+      // and the energy flux)
+      constexpr bool ALL = NODAL && L <= 6;
+      const double gr = gm1 * rho, pr = gr * ei, pd = ALL ? pr : fma(gr, ei, -g.mean[0]);
       const double H = fma(rho, fma(0.5, fma(ww, ww, fma(v, v, u * u)), ei), pr);   // E + p
 #pragma unroll
       for (int r = 0; r < 3; ++r) {
@@ -997,11 +1050,12 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns_flux_kernel(StageArgs a) {
         const double wx = fma(m2, t13, fma(m1, t12, m0 * t11)), wy = fma(m2, t23, fma(m1, t22, m0 * t12));
         const double wz = fma(m2, t33, fma(m1, t23, m0 * t13)), we = fma(m2, qz, fma(m1, qy, m0 * qx));
         double *o = p + 5 * r * BS;
-        o[0] = rV;
-        o[BS] = fma(rV, u, fma(pr, m0, -wx));
-        o[2 * BS] = fma(rV, v, fma(pr, m1, -wy));
-        o[3 * BS] = fma(rV, ww, fma(pr, m2, -wz));
-        o[4 * BS] = fma(H, V, -we);
+        const volatile double *c = g.c + 5 * r;
+        o[0] = ALL ? fma(rho, V, -c[0]) : rV;
+        o[BS] = fma(rV, u, fma(pd, m0, -(ALL ? c[1] + wx : wx)));
+        o[2 * BS] = fma(rV, v, fma(pd, m1, -(ALL ? c[2] + wy : wy)));
+        o[3 * BS] = fma(rV, ww, fma(pd, m2, -(ALL ? c[3] + wz : wz)));
+        o[4 * BS] = fma(H, V, -c[4]) - we;
         const int idx = r == 0 ? i : (r == 1 ? j : k);
         if (idx == 0 || idx == Q - 1) {
           const int f = idx == 0 ? (r == 0 ? 4 : (r == 1 ? 1 : 0)) : (r == 0 ? 2 : (r == 1 ? 3 : 5));

@@ -502,6 +502,25 @@ template <> __device__ __forceinline__ float p_sqrt<float>(float x) {
 template <class T> __device__ __forceinline__ T p_rsqrt(T x) { return T(1) / sqrt(x); }
 template <> __device__ __forceinline__ float p_rsqrt<float>(float x) { return rsqrtf(x); }
 
+// Reference state from conserved values U: what volume_flux_pert reads of it.
+// The volume term takes each element's own mean as its reference: the state
+// then enters without its constant mode, and the fluxes without the constant
+// F(mean), whose projected divergence vanishes but whose rounding does not
+// (pencil.cuh).
+template <int PHYS, class T>
+__device__ __forceinline__ RefState<T> element_reference(const T *U, T gamma) {
+  constexpr bool SW = PHYS == DGMX_SHALLOW;
+  constexpr int DIM = (PHYS == DGMX_EULER3D || PHYS == DGMX_NS3D) ? 3 : 2, NF = SW ? 3 : DIM + 2;
+  RefState<T> b;
+  const T ir = p_rcp(U[0]);
+  T s = T(0);
+  b.r = U[0];
+#pragma unroll
+  for (int i = 0; i < DIM; ++i) { b.m[i] = U[1 + i]; b.u[i] = U[1 + i] * ir; s = fma(b.m[i], b.u[i], s); }
+  b.H = SW ? T(0) : U[NF - 1] + (gamma - T(1.0)) * fma(T(-0.5), s, U[NF - 1]);
+  return b;
+}
+
 // F(Ub + d) - F(Ub) in every direction (volume term).
 template <int PHYS, class T>
 __device__ __forceinline__ void volume_flux_pert(const RefState<T> &b, const T *d, T gamma, T (*F)[5]) {

@@ -49,6 +49,7 @@ struct Cfg2 {
   // directions over three warps, 3 keeps them in one thread (default: FP64
   // 1, FP32 3)
   static constexpr int VDIRS = VDIRS_ > 0 ? VDIRS_ : (MIXED_ ? 3 : 1);
+  static_assert(EPB_ == 1, "one element per CTA");
   static_assert(VDIRS == 1 || VDIRS == 3, "the volume pass takes one or all three directions per thread");
   static constexpr int PHYSICS = PHYS;
   using R = std::conditional_t<MIXED_, float, double>;
@@ -95,7 +96,13 @@ struct Cfg2 {
   static_assert(O_T2 >= S_UN, "T2 (read in interval 3) must not overlap UN (written in interval 3)");
   static constexpr int SZ_SLOT = O_XL + S_XL;
   static constexpr size_t DATA = ((size_t)EPB * SZ_SLOT * sizeof(R) + 15) / 16 * 16;
-  static constexpr size_t SMEM = DATA + (size_t)EPB * (NFACE * sizeof(FaceLink) + 16 + (MIXED_ ? sizeof(RefState<R>) : 0));
+  // flux constants of the right-hand side on GLL values: between the GLL values
+  // and the flux arrays (Y, written behind the volume pass, ends there)
+  static constexpr int O_CST = S_UN;
+  static_assert(MIXED_ || S_Y - S_UN >= 15 || L > 5, "room for the constants where rhs2_kernel is built");
+  // links, element and class, the mixed form's reference states: the domain's
+  // and the element's
+  static constexpr size_t SMEM = DATA + (size_t)EPB * (NFACE * sizeof(FaceLink) + 16 + (MIXED_ ? 2 * sizeof(RefState<R>) : 0));
 };
 
 template <class C>
@@ -104,13 +111,14 @@ struct Smem2 {
   T *base;
   FaceLink *lnk;
   int *eid, *cls;
-  RefState<T> *ref;
+  RefState<T> *ref, *own;
   __device__ Smem2(unsigned char *raw) {
     base = reinterpret_cast<T *>(raw);
     lnk = reinterpret_cast<FaceLink *>(raw + C::DATA);
     eid = reinterpret_cast<int *>(lnk + C::EPB * C::NFACE);
     cls = eid + C::EPB;
-    ref = reinterpret_cast<RefState<T> *>(reinterpret_cast<unsigned char *>(eid) + 16 * C::EPB);
+    own = reinterpret_cast<RefState<T> *>(reinterpret_cast<unsigned char *>(eid) + 16 * C::EPB);
+    ref = own + C::EPB;
   }
   __device__ T *slot(int s) const { return base + (size_t)s * C::SZ_SLOT; }
 };
@@ -276,9 +284,9 @@ __device__ __forceinline__ void s2_face_point(const Smem2<C> &sm, const StageArg
 }
 
 // ---- interval 1b: backward k-pass from the modal rows in global memory ----
-// T1[b][n a][k] = sum_c B[c][k] u[n][a][b][c]; the mixed form takes the
-// solve's reference state out of the constant mode in FP64 first.  Elements
-// past the end get the constant state (their results are discarded).
+// T1[b][n a][k] = sum_c B[c][k] u[n][a][b][c]; the mixed form leaves the
+// constant mode out: its value is kept (s2_reference).  Elements past the end
+// get the constant state (their results are discarded).
 template <class C>
 __device__ __forceinline__ void s2_backward_k_row(const Smem2<C> &sm, const StageArgs &a, int e0, int w) {
   using T = typename C::R;
@@ -287,12 +295,15 @@ __device__ __forceinline__ void s2_backward_k_row(const Smem2<C> &sm, const Stag
   double v[L];
   if (e < a.ne) {
     ld_row<L>(a.X + ((size_t)e * RPS + r) * L, v);
-    if constexpr (C::MIXED)
-      if (r % (L * L) == 0) v[0] -= a.uref[kUrefStride * solve_of(a, e) + 5 + r / (L * L)];
   } else {
 #pragma unroll
-    for (int k = 0; k < L; ++k) v[k] = (!C::MIXED && k == 0 && r % (L * L) == 0) ? 1.0 : 0.0;
+    for (int k = 0; k < L; ++k) v[k] = k == 0 && r % (L * L) == 0 ? 1.0 : 0.0;
   }
+  if constexpr (C::MIXED)
+    if (r % (L * L) == 0) {
+      reinterpret_cast<double *>(sm.own)[r / (L * L)] = 0.35355339059327379 * v[0];   // 2^(-3/2)
+      v[0] = 0.0;
+    }
   // planes of NF L Q = 4 (mod 16) values at p = 3: this pass's (n a, b) rows
   // and the j pass's contiguous reads both fall on distinct banks
   T x[L], u[Q];
@@ -385,9 +396,14 @@ __device__ __forceinline__ void s2_backward_i(const Smem2<C> &sm, int tid) {
 // contravariant velocity V_r = metric[r] . u:  G_r[rho] = rho V_r,
 // G_r[m_d] = m_d V_r + p metric[r][d], G_r[E] = (E + p) V_r.  The mixed form
 // evaluates F(Ub + u') - F(Ub) (as volume_flux_pert, kernels.cuh) the same
-// way.  One direction per thread (20 accumulators; the columns of a direction
-// fill whole warps) or all three (60); Cfg2::VDIRS chooses.
-template <class C, int NR, int R0>
+// way, about the element's mean.  One direction per thread (20 accumulators;
+// the columns of a direction fill whole warps) or all three (60); Cfg2::VDIRS
+// chooses.
+// SHIFT: less the constants at O_CST (pencil.cuh);
+// FP64 stages leave the fluxes whole: their own update of the state rounds
+// more than the operators do (distance from a 64-bit evaluation 1.00 of the
+// derivative-first form's).
+template <class C, int NR, int R0, bool SHIFT>
 __device__ __forceinline__ void s2_volume_column(const Smem2<C> &sm, const StageArgs &a, int s, int jk) {
   using T = typename C::R;
   constexpr int NF = C::NF, L = C::L, Q = C::Q;
@@ -412,7 +428,7 @@ __device__ __forceinline__ void s2_volume_column(const Smem2<C> &sm, const Stage
 #pragma unroll
     for (int n = 0; n < NF; ++n) U[n] = un[(n * Q + i) * Q * Q];
     if constexpr (C::MIXED) {
-      const RefState<T> &b = sm.ref[s];
+      const RefState<T> &b = sm.own[s];
       const T rho = b.r + U[0], ir = p_rcp(rho);
       const T mx = b.m[0] + U[1], my = b.m[1] + U[2], mz = b.m[2] + U[3];
       const T upx = (U[1] - b.u[0] * U[0]) * ir, upy = (U[2] - b.u[1] * U[0]) * ir, upz = (U[3] - b.u[2] * U[0]) * ir;
@@ -446,11 +462,18 @@ __device__ __forceinline__ void s2_volume_column(const Smem2<C> &sm, const Stage
       for (int r = 0; r < NR; ++r) {
         const T m0 = met[r][0], m1 = met[r][1], m2 = met[r][2];
         const T V = fma(m2, ww, fma(m1, v, m0 * u));
-        Gr[r][0] = U[0] * V;
-        Gr[r][1] = fma(U[1], V, p * m0);
-        Gr[r][2] = fma(U[2], V, p * m1);
-        Gr[r][3] = fma(U[3], V, p * m2);
-        Gr[r][4] = Ep * V;
+        // a product, or the product less a constant (above p = 2 read each time:
+        // held in registers they spill)
+        auto mul = [&](T x, T y, int n) {
+          if constexpr (!SHIFT) return x * y;
+          const T *c = sm.slot(s) + C::O_CST + 5 * (R0 + r) + n;
+          return fma(x, y, L > 3 ? -*(const volatile T *)c : -*c);
+        };
+        Gr[r][0] = mul(U[0], V, 0);
+        Gr[r][1] = fma(U[1], V, mul(p, m0, 1));
+        Gr[r][2] = fma(U[2], V, mul(p, m1, 2));
+        Gr[r][3] = fma(U[3], V, mul(p, m2, 3));
+        Gr[r][4] = mul(Ep, V, 4);
       }
     }
   };
@@ -485,7 +508,7 @@ __device__ __forceinline__ void s2_volume_column(const Smem2<C> &sm, const Stage
       for (int b = 0; b < L; ++b) dst[(R0 + r) * (C::S_X1 + 1) + (n * L + b) * Q] = acc[r][n][b];
 }
 
-template <class C, int PHYS>
+template <class C, int PHYS, bool SHIFT>
 __device__ __forceinline__ void s2_volume(const Smem2<C> &sm, const StageArgs &a, int tid) {
   constexpr int Q = C::Q, EPB = C::EPB;
   // one direction per thread: the columns of one direction fill whole warps
@@ -496,10 +519,10 @@ __device__ __forceinline__ void s2_volume(const Smem2<C> &sm, const StageArgs &a
     if (jk >= Q * Q) continue;
     // the direction is a template argument, so the coefficients stay
     // constant-bank operands of the FMAs
-    if constexpr (C::VDIRS == 3) s2_volume_column<C, 3, 0>(sm, a, s, jk);
-    else if (r == 0) s2_volume_column<C, 1, 0>(sm, a, s, jk);
-    else if (r == 1) s2_volume_column<C, 1, 1>(sm, a, s, jk);
-    else s2_volume_column<C, 1, 2>(sm, a, s, jk);
+    if constexpr (C::VDIRS == 3) s2_volume_column<C, 3, 0, SHIFT>(sm, a, s, jk);
+    else if (r == 0) s2_volume_column<C, 1, 0, SHIFT>(sm, a, s, jk);
+    else if (r == 1) s2_volume_column<C, 1, 1, SHIFT>(sm, a, s, jk);
+    else s2_volume_column<C, 1, 2, SHIFT>(sm, a, s, jk);
   }
 }
 
@@ -792,10 +815,18 @@ __device__ __forceinline__ void stage2_tile(const Smem2<C> &sm, const StageArgs 
   s2_interval1<C, PHYS>(sm, a, e0, tid);
   __syncthreads();
   s2_interval2<C>(sm, tid);
+  if constexpr (C::MIXED) {   // the last thread: the interval's tasks start with the first
+    if (tid == C::NT - 1) {
+      float m[5];
+#pragma unroll
+      for (int n = 0; n < 5; ++n) m[n] = float(reinterpret_cast<const double *>(sm.own)[n]);
+      sm.own[0] = element_reference<PHYS, float>(m, float(a.gamma));
+    }
+  }
   __syncthreads();
   s2_backward_i<C>(sm, tid);
   __syncthreads();
-  s2_volume<C, PHYS>(sm, a, tid);
+  s2_volume<C, PHYS, false>(sm, a, tid);
   __syncthreads();
   s2_pass_j<C>(sm, tid);
   __syncthreads();
@@ -852,16 +883,29 @@ __global__ void __launch_bounds__(C::NT, C::MINB) rhs2_kernel(StageArgs a) {
     prefetch_l2_lines(a.Xn + ((size_t)n * a.ne + e) * QD, QD * 8, l / NF);
   }
   __syncthreads();
+  // the middle point's state and the metric, for the constants: on their way
+  // while the face points are done
+  const int k = tid - (C::NT - 15);
+  double own = 0.0;
+  if (k > 0) own = k <= NF ? a.Xn[((size_t)(k - 1) * a.ne + e) * QD + QD / 2] : __ldg(&a.classes[sm.cls[0]].metric[k - 1 - NF]);
   for (int w = tid; w < C::NFACE * C::GF; w += C::NT) s2_face_point<C, PHYS>(sm, a, e, w);
+  if (k > 0) sl[C::O_CST + k] = own;
   __syncthreads();
   for (int w = tid; w < C::NFACE * NF; w += C::NT) s2_lift<C>(sm, w);
+  static_assert(C::NT % 32 == 0, "the constants are made by threads of one warp");
+  if (k >= 0) {
+    const double *U = sl + C::O_CST + 1, *m = U + NF + k / 5 * 3;
+    const double c = flux_constant<3>(U, m, a.gamma, k % 5);
+    __syncwarp(0xfffe0000u);
+    sl[C::O_CST + k] = c;
+  }
   __syncthreads();   // the nodal values take the place of the face terms
   for (int w = tid; w < NF * QD; w += C::NT) {
     const int n = w / QD;
     sl[C::O_UN + w] = a.Xn[((size_t)n * a.ne + e) * QD + (w - n * QD)];
   }
   __syncthreads();
-  s2_volume<C, PHYS>(sm, a, tid);
+  s2_volume<C, PHYS, true>(sm, a, tid);
   __syncthreads();
   s2_pass_j<C>(sm, tid);
   __syncthreads();

@@ -44,7 +44,15 @@ struct CfgD {
   // element pitch = Q (mod banks): a warp's columns read consecutive banks
   static constexpr int SLOT = align_to(O_FP + S_F, Q, BANKS);
   static constexpr size_t DATA = ((size_t)EPB * SLOT * sizeof(R) + 15) / 16 * 16;
-  static constexpr size_t SMEM = DATA + (size_t)EPB * (16 + (MIXED_ ? sizeof(RefState<R>) : 0));
+  // element and class; the mixed form's element mean (four values)
+  static constexpr size_t SMEM = DATA + (size_t)EPB * (MIXED_ ? 32 : 16);
+  // flux constants of the right-hand side on GLL values (direction d, field n at
+  // NF d + n) in the place of the end lines, which only stages use
+  static constexpr int O_CST = O_FP;
+  // those constants up to p = 4: above, this form rounds no more than the
+  // derivative-first form without (1.24, 1.68, 1.19 times its distance from a
+  // 64-bit evaluation at p = 2, 3, 4, with the constants 0.69; 0.92 at p = 5)
+  static constexpr bool SHIFT = L <= 5;
 };
 
 template <class C>
@@ -52,13 +60,13 @@ struct SmemD {
   using T = typename C::R;
   T *base;
   int *eid, *cls;
-  RefState<T> *ref;
+  T *mean;
   int end;   // first element behind the tile's own
   __device__ SmemD(unsigned char *raw, int end_) : end(end_) {
     base = reinterpret_cast<T *>(raw);
     eid = reinterpret_cast<int *>(raw + C::DATA);
     cls = eid + C::EPB;
-    ref = reinterpret_cast<RefState<T> *>(reinterpret_cast<unsigned char *>(eid) + 16 * C::EPB);
+    mean = reinterpret_cast<T *>(reinterpret_cast<unsigned char *>(eid) + 16 * C::EPB);
   }
   __device__ T *slot(int s) const { return base + (size_t)s * C::SLOT; }
 };
@@ -70,13 +78,6 @@ __device__ __forceinline__ void sd_load(const SmemD<C> &sm, const StageArgs &a, 
     sm.cls[s] = c >= 0 ? c : 0;
     sm.eid[s] = c >= 0 ? e : -1;
   }
-}
-// The mixed form's reference state, which kernels write: after pdl_wait.
-template <class C>
-__device__ __forceinline__ void sd_load_ref(const SmemD<C> &sm, const StageArgs &a, int tid) {
-  if constexpr (C::MIXED)
-    for (int s = tid; s < C::EPB; s += C::NT)
-      sm.ref[s] = *reinterpret_cast<const RefState<float> *>(a.uref + kUrefStride * solve_of(a, sm.eid[s]) + 10);
 }
 
 // Trace values of GLL values (Field layout) at Gauss point g of face f of
@@ -100,8 +101,11 @@ __device__ __forceinline__ void sd_nodal_trace(const StageArgs &a, int e, int f,
 
 // ---- interval 1a: (F^ - F(U_own)).n J_side/J_el at face point g of face f ------
 // SELF: both sides' traces are interpolated here from the GLL values instead
-// of being read from trace buffers.
-template <class C, int PHYS, bool SELF>
+// of being read from trace buffers.  KEEP: the element's own flux at a point
+// of faces 0 and 3 becomes the constants of its volume fluxes along j and i
+// (pencil.cuh; their outward normal times J_side/J_el is -metric[d]).  Where it
+// is not finite, neither is the face's term, nor then the element's result.
+template <class C, int PHYS, bool KEEP, bool SELF>
 __device__ __forceinline__ void sd_face_point(const SmemD<C> &sm, const StageArgs &a, int e0, int w) {
   using T = typename C::R;
   constexpr int NF = C::NF, G = C::G;
@@ -144,6 +148,10 @@ __device__ __forceinline__ void sd_face_point(const SmemD<C> &sm, const StageArg
     ok = face_flux<PHYS, T>(UL, UR, nm, T(a.gamma), a.flux, Fh, FL, FR);
 #pragma unroll
     for (int k = 0; k < NF; ++k) eo[k * C::PF] = (master ? Fh[k] - FL[k] : FR[k] - Fh[k]) * jr;
+    if (KEEP && g == G / 2 && f % 3 == 0)
+#pragma unroll
+      for (int k = 0; k < NF; ++k)
+        sm.slot(s)[C::O_CST + (f == 0 ? NF : 0) + k] = jr * (master ? -FL[k] : FR[k]);
     if constexpr (is_ns(PHYS)) {
       // BR1 viscous lift: the central average leaves (V_own + V_nbr)/2, zero
       // on boundary sides (src/Navier_Stokes.cpp:113-252)
@@ -170,8 +178,11 @@ __device__ __forceinline__ void sd_state_row(const SmemD<C> &sm, const StageArgs
   if (e >= sm.end) return;
   double x[L];
   ld_row<L>(a.X + ((size_t)e * RPS + r) * L, x);
-  if constexpr (C::MIXED)
-    if (r % L == 0) x[0] -= a.uref[kUrefStride * solve_of(a, e) + 5 + r / L];
+  if constexpr (C::MIXED)   // the constant mode is left out; its value:
+    if (r % L == 0) {
+      sm.mean[4 * s + r / L] = T(0.5 * x[0]);
+      x[0] = 0.0;
+    }
   T v[L], u[Q];
 #pragma unroll
   for (int k = 0; k < L; ++k) v[k] = T(x[k]);
@@ -180,16 +191,18 @@ __device__ __forceinline__ void sd_state_row(const SmemD<C> &sm, const StageArgs
 }
 
 // ---- interval 2: one column of points, one flux direction -----------------------
-// Contravariant flux G = metric[R] . F(U) of one point, into g[n].
-template <class C, int PHYS>
+// Contravariant flux G = metric[R] . F(U) of one point, less the constants c
+// (SHIFT), into g[n].
+template <class C, int PHYS, bool SHIFT>
 __device__ __forceinline__ void sd_point_flux(const typename C::R *U, const typename C::R *m, typename C::R gamma,
-                                              const RefState<typename C::R> &ref, typename C::R *g) {
+                                              const RefState<typename C::R> &ref, const typename C::R *c,
+                                              typename C::R *g) {
   using T = typename C::R;
   T F[3][5];
   if constexpr (C::MIXED) volume_flux_pert<PHYS, T>(ref, U, gamma, F);
   else volume_flux<PHYS, T>(U, gamma, F);
 #pragma unroll
-  for (int n = 0; n < C::NF; ++n) g[n] = fma(m[1], F[1][n], m[0] * F[0][n]);
+  for (int n = 0; n < C::NF; ++n) g[n] = fma(m[1], F[1][n], SHIFT ? fma(m[0], F[0][n], -c[n]) : m[0] * F[0][n]);
 }
 
 // X_R[n][a] = sum_i C[a][i] G_R[n][i] along the column's points, C = E for the
@@ -221,7 +234,14 @@ __device__ __forceinline__ void sd_column(const SmemD<C> &sm, const StageArgs &a
   T acc[NF][L];
 #pragma unroll
   for (int n = 0; n < NF; ++n) zero<L>(acc[n]);
-  const RefState<T> &ref = sm.ref[C::MIXED ? s : 0];
+  // The mixed form's fluxes are about the element's mean, the right-hand
+  // side's on GLL values less the element's constants (pencil.cuh).  FP64
+  // stages leave them whole: their own update of the state rounds more than
+  // the operators do (0.96 of the derivative-first form's distance from a
+  // 64-bit evaluation).
+  RefState<T> ref;
+  if constexpr (C::MIXED) ref = element_reference<PHYS, T>(sm.mean + 4 * s, gamma);
+  const T *cst = sm.slot(s) + C::O_CST + NF * R;
 #pragma unroll
   for (int i = 0; i < (Q + 1) / 2; ++i) {
     const bool mid = 2 * i + 1 == Q;
@@ -242,8 +262,8 @@ __device__ __forceinline__ void sd_column(const SmemD<C> &sm, const StageArgs &a
         Um[n] = e - o;
       }
     }
-    sd_point_flux<C, PHYS>(Up, m, gamma, ref, Gp);
-    if (!mid) sd_point_flux<C, PHYS>(Um, m, gamma, ref, Gm);
+    sd_point_flux<C, PHYS, NODAL && C::SHIFT>(Up, m, gamma, ref, cst, Gp);
+    if (!mid) sd_point_flux<C, PHYS, NODAL && C::SHIFT>(Um, m, gamma, ref, cst, Gm);
 #pragma unroll
     for (int n = 0; n < NF; ++n) {
       const T sum = mid ? Gp[n] : Gp[n] + Gm[n], dif = mid ? T(0) : Gp[n] - Gm[n];
@@ -448,8 +468,7 @@ __device__ __forceinline__ void sd_front(const SmemD<C> &sm, const StageArgs &a,
   constexpr int NT = C::NT, NC = C::EPB * C::Q;
   sd_load<C>(sm, a, e0, tid);
   pdl_wait();
-  sd_load_ref<C>(sm, a, tid);
-  for (int w = tid; w < C::EPB * 4 * C::G; w += NT) sd_face_point<C, PHYS, SELF>(sm, a, e0, w);
+  for (int w = tid; w < C::EPB * 4 * C::G; w += NT) sd_face_point<C, PHYS, NODAL && C::SHIFT && !is_ns(PHYS), SELF>(sm, a, e0, w);
   // from the last thread down: a tile with threads enough for both does the
   // rows beside the face points
   if constexpr (!NODAL && !is_ns(PHYS))
@@ -553,7 +572,12 @@ struct NsFlux2 {
   static constexpr int FQ = C::Q % 2 == 0 ? C::Q + 1 : C::Q;      // [f][n] lines of Q
   static constexpr int SLOT = align_to(O_J + cmax(12 * C::PF, 12 * FQ), C::Q, 16);
   static constexpr size_t DATA = (size_t)C::EPB * SLOT * sizeof(double);
-  static constexpr size_t SMEM = (DATA + 15) / 16 * 16 + 16 * C::EPB;
+  static constexpr size_t SMEM = (DATA + 15) / 16 * 16 + 16 * C::EPB;   // elements and classes
+  // flux constants of the right-hand side on GLL values, up to p = 5 (without
+  // them 1.56, 1.86, 1.64, 1.31 and, at p = 7, 0.90 times the derivative-first
+  // form's distance from a 64-bit evaluation)
+  static constexpr bool SHIFT = C::L <= 6;
+  static constexpr size_t SMEM_NODAL = SMEM + (SHIFT ? 8 * sizeof(double) * C::EPB : 0);
 };
 
 // One column's gradient pass along i: E_i v and P_i v.
@@ -604,6 +628,8 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns2d_flux_kernel(StageArgs a) 
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double *base = reinterpret_cast<double *>(smem_raw);
   int *eid = reinterpret_cast<int *>(smem_raw + (N::DATA + 15) / 16 * 16), *cls = eid + EPB;
+  constexpr bool SHIFT = NODAL && N::SHIFT;
+  double *cst = reinterpret_cast<double *>(smem_raw + N::SMEM);
   const int tid = threadIdx.x, e0 = (a.vtiles ? a.vtiles[blockIdx.x] : (int)blockIdx.x) * EPB;
   auto slot = [&](int s) { return base + (size_t)s * N::SLOT; };
   pdl_release();
@@ -702,6 +728,20 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns2d_flux_kernel(StageArgs a) 
     p[BS] = u; p[2 * BS] = v; p[3 * BS] = ei;
   }
   __syncthreads();
+  // constants of the fluxes (pencil.cuh): the convective ones of the middle
+  // point; stages leave the fluxes whole, as stage2d_kernel's
+  if constexpr (SHIFT) for (int w = NT - 1 - tid; w < 2 * EPB; w += NT) {
+    const int s = w / 2, d = w - 2 * s;
+    if (eid[s] < 0) continue;
+    const double *p = slot(s) + (Q / 2) * (PQ + 1), *m = a.classes[cls[s]].metric + 3 * d;
+    const double rho = p[0], u = p[BS], v = p[2 * BS], ei = p[3 * BS];
+    const double pr = (a.gamma - 1.0) * rho * ei, V = fma(m[1], v, m[0] * u), rV = rho * V;
+    double *c = cst + 4 * w;
+    c[0] = flux_constant(rV);
+    c[1] = flux_constant(fma(rV, u, pr * m[0]));
+    c[2] = flux_constant(fma(rV, v, pr * m[1]));
+    c[3] = flux_constant(fma(rho, fma(0.5, fma(v, v, u * u), ei), pr) * V);
+  }
   const double mu = a.vis, kap = a.gamma / a.Pr * a.vis;
   // gradients, then stresses (t11, t12, t22) and heat flux at the points
   if constexpr (F32) {
@@ -850,10 +890,11 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns2d_flux_kernel(StageArgs a) 
       const double V = fma(m1, v, m0 * u), rV = rho * V;
       const double wx = fma(m1, t12, m0 * t11), wy = fma(m1, t22, m0 * t12), we = fma(m1, qy, m0 * qx);
       double *o = p + 4 * d * BS;
-      o[0] = rV;
-      o[BS] = fma(rV, u, fma(pr, m0, -wx));
-      o[2 * BS] = fma(rV, v, fma(pr, m1, -wy));
-      o[3 * BS] = fma(H, V, -we);
+      const volatile double *c = cst + 4 * (2 * s + d);
+      o[0] = SHIFT ? fma(rho, V, -c[0]) : rV;
+      o[BS] = fma(rV, u, fma(pr, m0, -(SHIFT ? c[1] + wx : wx)));
+      o[2 * BS] = fma(rV, v, fma(pr, m1, -(SHIFT ? c[2] + wy : wy)));
+      o[3 * BS] = SHIFT ? fma(H, V, -c[3]) - we : fma(H, V, -we);
       const int idx = d == 0 ? i : j;
       if (idx == 0 || idx == Q - 1) {
         const int f = d == 0 ? (idx == 0 ? 3 : 1) : (idx == 0 ? 0 : 2);
