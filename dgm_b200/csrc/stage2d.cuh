@@ -882,8 +882,15 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns2d_flux_kernel(StageArgs a) 
       t11 = q[0]; t12 = q[BS]; t22 = q[3 * BS]; hx = q[4 * BS]; hy = q[5 * BS];
     }
     const double qx = fma(t12, v, fma(t11, u, hx)), qy = fma(t22, v, fma(t12, u, hy));
-    const double pr = (a.gamma - 1.0) * rho * ei;
-    const double H = fma(rho, fma(0.5, fma(v, v, u * u), ei), pr);   // E + p
+    double pr, H;   // pressure, E + p
+    if constexpr (SHIFT) {   // from the energy itself, as in ns_flux_kernel
+      const double E = a.Xn[((size_t)3 * a.ne + eid[s]) * Q * Q + r];
+      pr = (a.gamma - 1.0) * fma(-0.5 * rho, fma(v, v, u * u), E);
+      H = E + pr;
+    } else {
+      pr = (a.gamma - 1.0) * rho * ei;
+      H = fma(rho, fma(0.5, fma(v, v, u * u), ei), pr);
+    }
 #pragma unroll
     for (int d = 0; d < 2; ++d) {
       const double m0 = __ldg(&gc->metric[3 * d]), m1 = __ldg(&gc->metric[3 * d + 1]);
