@@ -919,7 +919,7 @@ dgmx_status create_impl(const dgmx_mesh *m, const dgmx_params *p, dgmx_domain **
     }
   }
   const bool plain = bspec && !bspec->sides.empty();
-  d->ops = default_ops(phys, pp + 1, qq, m->ne, plain);
+  d->ops = default_ops(phys, pp + 1, qq, m->ne, plain, p->device);
   if (d->visc32) {
     if (const std::vector<KernelOps> *vs = find_variants(phys, pp + 1, qq))
       for (const KernelOps &o : *vs)
@@ -930,7 +930,7 @@ dgmx_status create_impl(const dgmx_mesh *m, const dgmx_params *p, dgmx_domain **
     }
   }
   if (d->ops && d->prm.precision == DGMX_MIXED) {
-    d->ops_m = default_ops(phys + kMixedKey, pp + 1, qq, m->ne, plain);
+    d->ops_m = default_ops(phys + kMixedKey, pp + 1, qq, m->ne, plain, p->device);
     if (!d->ops_m) {
       g_create_error = "no mixed-precision kernels built for p=" + std::to_string(pp) + ", q=" + std::to_string(qq);
       return DGMX_ERR_UNSUPPORTED;

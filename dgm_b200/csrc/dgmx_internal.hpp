@@ -293,9 +293,10 @@ constexpr int kMixedKey = 1000;
 struct KernelOps {
   int epb = 0, nt = 0, minb = 0, mixed = 0;
   int warp = 0;                                        // kind: 0 CTA tile, 2 prefetching persistent kernel
-  // default choice (default_ops): the tile preferred most, except that one
-  // with small >= elements goes first (a mesh that one wave of its CTAs holds
-  // gains from more threads and registers per element, not from occupancy)
+  // default choice (default_ops): the tile preferred most, except that the
+  // first one goes first that the mesh gives no more than `small` elements per
+  // SM (a mesh that one wave of its CTAs holds gains from more threads and
+  // registers per element, not from occupancy)
   int preferred = 0, small = 0;
   size_t smem = 0;
   cudaError_t (*init)(const Tables1D &t) = nullptr;   // tables + smem attributes, current device
@@ -325,9 +326,11 @@ struct KernelOps {
   const KernelOps *tensor = nullptr;
 };
 void register_ops(int physics, int L, int Q, const KernelOps &ops);
-// The default tile for a mesh of ne elements; plain: one that handles
-// boundary sides (kind 0).
-const KernelOps *default_ops(int physics, int L, int Q, int ne, bool plain);
+// The default tile for a mesh of ne elements on the device; plain: one that
+// handles boundary sides (kind 0).
+const KernelOps *default_ops(int physics, int L, int Q, int ne, bool plain, int device);
+// Streaming multiprocessors of a device.
+int sm_count(int device);
 const std::vector<KernelOps> *find_variants(int physics, int L, int Q);
 void list_ops(std::vector<std::vector<int>> &out);
 

@@ -245,15 +245,8 @@ inline int sm_count() {
   static int cached[64] = {0};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return 148;
-  if (!cached[dev]) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) {
-      cudaGetLastError();
-      n = 148;
-    }
-    cached[dev] = n;
-  }
+  if (dev < 0 || dev >= 64) return sm_count(0);
+  if (!cached[dev]) cached[dev] = sm_count(dev);
   return cached[dev];
 }
 
@@ -464,7 +457,7 @@ void reg2() {
   // 315, FP32 201 against 215; p = 2, 20^3: 39 against 54; above, the third
   // form's tile is faster); a mesh of one wave takes the uncapped tile (p = 3,
   // 8^3: 7.4 us against 11 to 12 for the capped ones)
-  constexpr int PREF = P <= 4 ? 2 : 0, ONE_WAVE = P <= 4 ? 4 * 148 : 0;
+  constexpr int PREF = P <= 4 ? 2 : 0, ONE_WAVE = P <= 4 ? 4 : 0;
   reg2_variant<PHYS, P, Q, 1, NTB, 0, MIXED>(0, MIXED ? 0 : ONE_WAVE);
   if constexpr (B96 >= 2) reg2_variant<PHYS, P, Q, 1, NTB, B96, MIXED>(0, MIXED ? ONE_WAVE : 0);
   if constexpr (A96 >= 2) reg2_variant<PHYS, P, Q, 1, NTA, A96, MIXED>();
@@ -567,7 +560,7 @@ void reg3_ns() {
   register_ops(PHYS, P + 1, Q, Launch3Ns<PHYS, P + 1, Q>::ops());
   // p = 3: 512 elements 21 us against 29, 4096 elements 95 against 94
   KernelOps o = Launch3Ns<PHYS, P + 1, Q, (P < 4 ? 128 : 256), (P < 4 ? 96 : 112), 128, 80>::ops();
-  if (P < 4) o.small = 2048;
+  if (P < 4) o.small = 14;
   register_ops(PHYS, P + 1, Q, o);
 }
 
@@ -695,10 +688,10 @@ void reg2d() {
   KernelOps wide = Launch2D<PHYS, P + 1, Q, MIXED, E, 256, 1>::ops(),
             full = Launch2D<PHYS, P + 1, Q, MIXED, E, 128, B>::ops(), half = Half::ops();
   wide.preferred = half.preferred = 0;
-  wide.small = 148 * E;
+  wide.small = E;
   if (!MIXED && 7 * (half.smem + 1024) <= 228 * 1024) {
     half.preferred = 2;
-    full.small = 148 * B * E;
+    full.small = B * E;
   }
   register_ops(key, P + 1, Q, wide);
   register_ops(key, P + 1, Q, full);

@@ -354,7 +354,7 @@ dgmx_status get_arena(dgmx_pool *P, int phys, int L, int Q, Arena **out) {
   a->gf = a->dim == 2 ? Q - 1 : (Q - 1) * (Q - 1);
   a->ld = a->dim == 2 ? L * L : L * L * L;
   a->qd = a->dim == 2 ? Q * Q : Q * Q * Q;
-  a->fops = default_ops(phys, L, Q, 1 << 20, false);
+  a->fops = default_ops(phys, L, Q, 1 << 20, false, P->prm.device);
   const int key = phys + (mixed ? kMixedKey : 0);
   const std::vector<KernelOps> *vs = find_variants(key, L, Q);
   if (!a->fops || !vs || vs->empty())
@@ -369,11 +369,11 @@ dgmx_status get_arena(dgmx_pool *P, int phys, int L, int Q, Arena **out) {
     // plain default tile supplies its trace and projection kernels
     dgmx_status st = fused_setup(P);
     if (st != DGMX_OK) return st;
-    a->sops = default_ops(key, L, Q, 1 << 20, false);
+    a->sops = default_ops(key, L, Q, 1 << 20, false, P->prm.device);
     a->epb = P->fops->epb(a->body);
   } else {
     const int v = P->prm.autotune ? tuned_variant(phys, mixed, L, Q, P->prm.gamma, P->prm.flux, P->prm.device) : -1;
-    a->sops = (v >= 0 && v < (int)vs->size()) ? &(*vs)[v] : default_ops(key, L, Q, 1 << 20, false);
+    a->sops = (v >= 0 && v < (int)vs->size()) ? &(*vs)[v] : default_ops(key, L, Q, 1 << 20, false, P->prm.device);
     a->epb = a->sops->epb;
   }
   a->tab = make_tables(L, Q, Q - 1);

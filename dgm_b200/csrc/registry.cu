@@ -22,14 +22,24 @@ void register_ops(int physics, int L, int Q, const KernelOps &ops) {
   table()[std::make_tuple(physics, L, Q)].push_back(ops);
 }
 
-const KernelOps *default_ops(int physics, int L, int Q, int ne, bool plain) {
+int sm_count(int device) {
+  int n = 0;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0) {
+    cudaGetLastError();
+    n = 148;
+  }
+  return n;
+}
+
+const KernelOps *default_ops(int physics, int L, int Q, int ne, bool plain, int device) {
+  const int sms = sm_count(device);
   std::lock_guard<std::mutex> lk(table_mutex());
   auto it = table().find(std::make_tuple(physics, L, Q));
   if (it == table().end()) return nullptr;
   const KernelOps *best = nullptr;
   for (const KernelOps &o : it->second) {
     if (plain && o.warp != 0) continue;
-    if (o.small >= ne) return &o;
+    if ((long long)o.small * sms >= ne) return &o;
     if (!best || o.preferred > best->preferred) best = &o;
   }
   return best;
