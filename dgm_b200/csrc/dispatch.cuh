@@ -558,9 +558,12 @@ struct Launch3Ns {
 template <int PHYS, int P, int Q>
 void reg3_ns() {
   register_ops(PHYS, P + 1, Q, Launch3Ns<PHYS, P + 1, Q>::ops());
-  // p = 3: 512 elements 21 us against 29, 4096 elements 95 against 94
+  // p = 3: 512 elements 21 us against 29, 1728 46 against 50, 2744 66 against 67,
+  // 4096 95 against 94.  p = 1 and 2, one wave of its CTAs: 216 elements 11.9 and
+  // 14.4 us against 12.4 and 16.2, 729 12.8 and 17.6 against 16.0 and 23.7; 1000
+  // 21.3 and 27.2 against 17.4 and 26.1, 8000 91 and 127 against 68 and 109
   KernelOps o = Launch3Ns<PHYS, P + 1, Q, (P < 4 ? 128 : 256), (P < 4 ? 96 : 112), 128, 80>::ops();
-  if (P < 4) o.small = 14;
+  if (P < 4) o.small = P == 3 ? 14 : 5;
   register_ops(PHYS, P + 1, Q, o);
 }
 
@@ -676,10 +679,15 @@ struct Launch2DNs {
 // SM or less (16 x 16, p = 4: 6.5 us a stage against 7.4); and 64.  In FP64,
 // where the registers hold an SM to 16 warps, eight 64-thread CTAs of E elements
 // have twice the elements in flight, two rounds of rows per interval to hide
-// loads and FP64 chains behind: the default above what one wave of 128-thread
-// CTAs holds (p = 4, 128 / 64 threads: 50 x 50 10.5 / 13.6, 60 x 60 16.4 / 14.9,
-// 100 x 100 25.4 / 22.9, 300 x 300 209 / 176 us a stage; p = 2, 300 x 300 91 /
-// 80), unless fewer than seven fit the shared memory (p = 7, 90 x 90: 50 / 54).
+// loads and FP64 chains behind: up to p = 5 the default above what one wave of
+// 128-thread CTAs holds (us a stage, 128 / 64 threads: p = 1, 100 x 100 9.5 /
+// 10.1, 200 x 200 22.3 / 22.3; p = 2, 150 x 150 21.7 / 19.9, 300 x 300 91 / 80;
+// p = 3, 100 x 100 16.1 / 17.2, 200 x 200 51.5 / 48.0; p = 4, 60 x 60 16.4 / 14.9,
+// 100 x 100 26.0 / 23.3, 300 x 300 209 / 176; p = 5, 80 x 80 24.2 / 22.5, 160 x 160
+// 76.3 / 71.2), unless fewer than seven fit the shared memory.  At p = 6, where
+// it spills 680 bytes (128 threads 276), only while one wave of it holds the mesh:
+// 50 x 50 20.3 / 19.9, 60 x 60 21.9 / 20.5, but 75 x 75 29.7 / 33.6, 120 x 120 62.6
+// / 69.3, 200 x 200 175 / 181.
 template <int PHYS, int P, int Q, bool MIXED = false>
 void reg2d() {
   constexpr int E = stage2d_epb(phys_nf(PHYS), P + 1), B = MIXED ? 6 : 4;
@@ -690,8 +698,8 @@ void reg2d() {
   wide.preferred = half.preferred = 0;
   wide.small = E;
   if (!MIXED && 7 * (half.smem + 1024) <= 228 * 1024) {
-    half.preferred = 2;
     full.small = B * E;
+    if (P < 6) half.preferred = 2; else half.small = 7 * E;
   }
   register_ops(key, P + 1, Q, wide);
   register_ops(key, P + 1, Q, full);
