@@ -358,6 +358,15 @@ void reg3() {
   constexpr int NT = form3_threads(P + 1);
   register_ops(key, P + 1, Q, Launch3<PHYS, P + 1, Q, MIXED>::ops());
   register_ops(key, P + 1, Q, Launch3<PHYS, P + 1, Q, MIXED, NT, MIXED ? 56 : 80>::ops());
+  if constexpr (MIXED && P >= 6) {
+    // 512 threads where no SM has more than one CTA (p = 7, 8 to 125 elements:
+    // 9.2 to 9.4 us a stage against 12.9 to 16.6 with 256, p = 6 9.2 to 9.4
+    // against 11.1 to 14.1; 216 elements 17.6 and 17.4 against 16.2 and 14.4)
+    KernelOps o = Launch3<PHYS, P + 1, Q, MIXED, 512, 128>::ops();
+    o.preferred = 0;
+    o.small = 1;
+    register_ops(key, P + 1, Q, o);
+  }
 }
 
 // The second-form stage kernel (stage2.cuh) for LSRK and right-hand-side
