@@ -113,11 +113,10 @@ struct dgmx_domain {
   double bcpar[kMaxBcTypes + 1][5] = {};
   bool hold = false;
   double *R0 = nullptr, *cbar = nullptr;                 // hold: [e][n] constant coefficients, [n] means
-  // Navier-Stokes with precision = DGMX_MIXED: the BR1 viscous kernels run in
-  // FP32 (from the uncapped tile vops); stage, registers and traces stay FP64
+  // Navier-Stokes with precision = DGMX_MIXED: the BR1 viscous terms run in
+  // FP32 (the tile's ns_visc32); stage, registers and traces stay FP64
   bool visc32 = false;
-  bool visc_tc = false;     // the FP32 viscous kernels' contractions on the tensor cores (3xTF32)
-  const KernelOps *vops = nullptr;
+  bool visc_tc = false;     // in ops->tensor's kernels, contractions on the tensor cores (3xTF32)
   // element partition: ghost slots in the trace buffers and the halo
   // exchange lists (plan.nranks == 1: the whole mesh, no exchange)
   PartitionPlan plan;
@@ -229,17 +228,13 @@ struct dgmx_domain {
   bool ns() const { return prm.physics == DGMX_NS2D || prm.physics == DGMX_NS3D; }
   // the tile whose viscous kernels run (what they leave in Pv is read by the
   // stage kernel of the same form)
-  const KernelOps *visc_ops() const {
-    if (!visc32) return ops;
-    return visc_tc ? ops->tensor : (ops->ns_visc32 ? ops : vops);
-  }
-  bool separate_grad() const { return (visc32 ? visc_ops()->ns_grad32 : visc_ops()->ns_grad) != nullptr; }
+  const KernelOps *visc_ops() const { return visc_tc ? ops->tensor : ops; }
+  // the gradients' kernel, which the tensor-core form alone has
   cudaError_t ns_grad(const StageArgs &a, bool nodal, cudaStream_t s) const {
-    if (!separate_grad()) return cudaSuccess;
-    return visc32 ? visc_ops()->ns_grad32(a, nodal, s) : visc_ops()->ns_grad(a, nodal, s);
+    return visc_tc ? visc_ops()->ns_grad32(a, nodal, s) : cudaSuccess;
   }
   cudaError_t ns_visc(const StageArgs &a, bool nodal, cudaStream_t s) const {
-    return visc32 ? visc_ops()->ns_visc32(a, nodal, s) : visc_ops()->ns_visc(a, nodal, s);
+    return (visc32 ? visc_ops()->ns_visc32 : visc_ops()->ns_visc)(a, nodal, s);
   }
   int visc_epb() const { return visc_ops()->epb; }
   // the viscous flux kernel over tile list which (0 boundary, 1 interior);
@@ -250,7 +245,7 @@ struct dgmx_domain {
     a.vtiles = vtiles + (which == 0 ? 0 : nvt_b);
     return ns_visc(a, false, s);
   }
-  // projected gradients in global memory: tiles with a gradient kernel only
+  // projected gradients in global memory: the tensor-core form only
   cudaError_t alloc_gradients() { return Ghat ? cudaSuccess : dalloc(&Ghat, (size_t)ne * (dim + 1) * dim * ld); }
   bool mixed() const { return prm.precision == DGMX_MIXED; }
   const KernelOps *stage_ops() const { return mixed() ? ops_m : (visc_tc ? ops->tensor : ops); }
@@ -570,7 +565,7 @@ dgmx_status enqueue_step(dgmx_domain *d, double dt) {
     cudaError_t e;
     if (d->ns()) {
       if ((e = d->ns_grad(a, false, d->stream)) != cudaSuccess) return d->cuda(e, "viscous gradient kernel");
-      if (d->separate_grad()) ++d->launches;
+      if (d->visc_tc) ++d->launches;
       if (overlaps(d)) {
         const dgmx_status xs = visc_overlapped(d, a);
         if (xs != DGMX_OK) return xs;
@@ -609,7 +604,7 @@ int launches_per_stage(const dgmx_domain *d) {
   // the viscous flux kernel
   const int split = (overlaps(d) && !d->hold ? 1 : 0) + (overlaps(d) && d->ns() ? 1 : 0);
   const int hold = d->hold ? (rank ? 3 : 2) : 0;   // (scatter,) reduce, apply
-  return (d->ns() ? (d->separate_grad() ? 3 : 2) : 1) + split + hold + halo;
+  return (d->ns() ? (d->visc_tc ? 3 : 2) : 1) + split + hold + halo;
 }
 
 // Host repeat of launch_reference_integrals' summation order over the
@@ -920,14 +915,9 @@ dgmx_status create_impl(const dgmx_mesh *m, const dgmx_params *p, dgmx_domain **
   }
   const bool plain = bspec && !bspec->sides.empty();
   d->ops = default_ops(phys, pp + 1, qq, m->ne, plain, p->device);
-  if (d->visc32) {
-    if (const std::vector<KernelOps> *vs = find_variants(phys, pp + 1, qq))
-      for (const KernelOps &o : *vs)
-        if (o.ns_visc32) { d->vops = &o; break; }
-    if (!d->vops) {
-      g_create_error = "no FP32 viscous kernels built for p=" + std::to_string(pp) + ", q=" + std::to_string(qq);
-      return DGMX_ERR_UNSUPPORTED;
-    }
+  if (d->visc32 && d->ops && !d->ops->ns_visc32) {
+    g_create_error = "no FP32 viscous kernels built for p=" + std::to_string(pp) + ", q=" + std::to_string(qq);
+    return DGMX_ERR_UNSUPPORTED;
   }
   if (d->ops && d->prm.precision == DGMX_MIXED) {
     d->ops_m = default_ops(phys + kMixedKey, pp + 1, qq, m->ne, plain, p->device);
@@ -993,7 +983,6 @@ dgmx_status create_impl(const dgmx_mesh *m, const dgmx_params *p, dgmx_domain **
   };
   st = DGMX_OK;
   if (!chk(d->ops->init(d->tab), "kernel table upload")) { g_create_error = d->errmsg; d->release(); return st; }
-  if (d->vops && d->vops != d->ops && !chk(d->vops->init(d->tab), "kernel table upload")) { g_create_error = d->errmsg; d->release(); return st; }
   if (d->ops_m && !chk(d->ops_m->init(d->tab), "kernel table upload")) { g_create_error = d->errmsg; d->release(); return st; }
   if (!chk(cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking), "stream")) { g_create_error = d->errmsg; d->release(); return st; }
   bool ok = chk(dalloc(&d->U, d->nmodal()), "alloc U") && chk(dalloc(&d->Ut, d->nmodal()), "alloc Ut") &&
@@ -1010,8 +999,7 @@ dgmx_status create_impl(const dgmx_mesh *m, const dgmx_params *p, dgmx_domain **
                              chk(dalloc(&d->Tf[0], d->ntrace()), "alloc T0 (FP32)") &&
                              chk(dalloc(&d->Tf[1], d->ntrace()), "alloc T1 (FP32)") &&
                              chk(dalloc(&d->uref, (size_t)kUrefStride), "alloc reference state"))) &&
-            (!d->ns() || ((!d->separate_grad() || chk(d->alloc_gradients(), "alloc gradients")) &&
-                          chk(dalloc(&d->Vtr, (size_t)d->nslot * d->nfaces * (d->nf - 1) * d->gf), "alloc viscous traces") &&
+            (!d->ns() || (chk(dalloc(&d->Vtr, (size_t)d->nslot * d->nfaces * (d->nf - 1) * d->gf), "alloc viscous traces") &&
                           chk(dalloc(&d->Pv, (size_t)d->ne * d->nf * d->ld), "alloc viscous divergence"))) &&
             (!d->ns() || d->dim != 3 || (chk(dalloc(&d->R0, (size_t)d->ne * d->nf), "alloc hold coefficients") &&
                                           chk(dalloc(&d->cbar, (size_t)d->nf), "alloc hold means"))) &&
@@ -1578,7 +1566,7 @@ dgmx_status dgmx_time_derivative_device(dgmx_domain *d, const double *U_dev, dou
   if (d->ns()) {
     if ((e = d->ns_grad(a, true, d->stream)) != cudaSuccess) return d->cuda(e, "viscous gradient kernel");
     if ((e = d->ns_visc(a, true, d->stream)) != cudaSuccess) return d->cuda(e, "viscous flux kernel");
-    d->launches += d->separate_grad() ? 2 : 1;
+    d->launches += d->visc_tc ? 2 : 1;
     if ((xs = exchange(d, visc_halo(d))) != DGMX_OK) return xs;
   }
   a.R0 = d->hold ? d->R0 : nullptr;
@@ -2054,7 +2042,7 @@ dgmx_status dgmx_group_advance(dgmx_group *g, double dt, int nsteps) {
           const StageArgs a = stage_args(d, sp, dt);
           if (e == cudaSuccess) e = d->ns_grad(a, false, s);
           if (e == cudaSuccess) e = d->ns_visc_tiles(a, 0, s);
-          d->launches += d->separate_grad() ? 2 : 1;
+          d->launches += d->visc_tc ? 2 : 1;
         }
         if (e == cudaSuccess) e = cudaEventRecord(g->ev_b, s);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(g->xs, g->ev_b, 0);

@@ -252,7 +252,7 @@ struct StageArgs {
   double *Ghat;           // projected primitive gradients, modal [e][comp][dir][L^d]
   double *V;              // viscous normal-flux traces [e][face][field-1][gf]
   double *Pv;             // projected viscous divergence, modal [e][field-1][L^d], or
-                          // (tiles without ns_grad) that of the whole volume flux, [e][field][L^d]
+                          // (tiles without ns_grad32) that of the whole volume flux, [e][field][L^d]
   // boundary types t = 1..15 (GeomClass::bc): kind (DGMX_BC_*) and parameters
   int bckind[kMaxBcTypes + 1];
   double bcpar[kMaxBcTypes + 1][5];
@@ -311,14 +311,12 @@ struct KernelOps {
   int self_traces = 0;                                 // rhs_nodal without a.Tin interpolates both traces itself
   cudaError_t (*forward)(const StageArgs &a, const double *Un, double *Um, cudaStream_t s) = nullptr;
   cudaError_t (*backward)(const StageArgs &a, const double *Um, double *Un, cudaStream_t s) = nullptr;
-  // Navier-Stokes only: lifted gradients, then viscous traces + divergence
-  // (no ns_grad: ns_visc does both and leaves the projected divergence of the
-  // whole volume flux in a.Pv for this tile's stage and rhs_nodal);
-  // nodal = read GLL values from a.Xn instead of the modal register a.X
-  cudaError_t (*ns_grad)(const StageArgs &a, bool nodal, cudaStream_t s) = nullptr;
+  // Navier-Stokes only: gradients, viscous traces and the projected divergence
+  // of the whole volume flux in a.Pv for this tile's stage and rhs_nodal, with
+  // the viscous terms in FP64 or FP32; nodal = read GLL values from a.Xn instead
+  // of the modal register a.X.  Tiles with ns_grad32 (the tensor-core form) take
+  // the lifted gradients from it, and a.Pv holds the viscous divergence alone.
   cudaError_t (*ns_visc)(const StageArgs &a, bool nodal, cudaStream_t s) = nullptr;
-  // the same in FP32 (Navier-Stokes with precision = DGMX_MIXED); set on the
-  // uncapped tile of each (physics, L, Q, EPB)
   cudaError_t (*ns_grad32)(const StageArgs &a, bool nodal, cudaStream_t s) = nullptr;
   cudaError_t (*ns_visc32)(const StageArgs &a, bool nodal, cudaStream_t s) = nullptr;
   // the tile of the 3xTF32 tensor-core form (3-D, p >= 5): its ns_grad32 and

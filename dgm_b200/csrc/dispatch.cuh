@@ -553,8 +553,7 @@ struct Launch3Ns {
     o.epb = 1; o.nt = NTF; o.minb = CF::MINB; o.smem = F::SMEM; o.preferred = 1;
     o.init = init; o.stage = stage; o.stage_grid = stage_grid; o.blocks_per_sm = blocks_per_sm;
     o.rhs_nodal = rhs_nodal;
-    o.ns_grad = nullptr; o.ns_visc = flux<false>;
-    o.ns_grad32 = nullptr; o.ns_visc32 = flux<true>;
+    o.ns_visc = flux<false>; o.ns_visc32 = flux<true>;
     if constexpr (L >= 6) {
       // 3xTF32: at q = 9 the first-form stage tile runs 512 threads (one per
       // point, 736, would get 80 registers and spill about 1 KB each)

@@ -961,7 +961,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns_flux_kernel(StageArgs a) {
       double *w = W + 3 * c * BS + o;
       double z[3][L];
       ns3_grad_k<C>(w, X + c * 6 * C::XLS, g.metric, aa, bb, z);
-  #pragma unroll
+#pragma unroll
       for (int d = 0; d < 3; ++d) st_pencil<L>(w + d * BS, 1, z[d]);
     });
     __syncthreads();
@@ -973,7 +973,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns_flux_kernel(StageArgs a) {
       double *p = W + i * SI + j * SJ + k;
       double t[6];
       viscous_stress<3, double>(p, BS, a.vis, t);
-  #pragma unroll
+#pragma unroll
       for (int n = 0; n < 6; ++n) p[n * BS] = t[n];
     }
     pencils_i<C>(1, tid, [&](int, int jk) {
@@ -992,9 +992,9 @@ __global__ void __launch_bounds__(C::NT, C::MINB) ns_flux_kernel(StageArgs a) {
       double *w = W + 6 * BS + o;
       double z[3][L], u[Q];
       ns3_grad_k<C>(w, X + 18 * C::XLS, g.metric, aa, bb, z);
-  #pragma unroll
+#pragma unroll
       for (int d = 0; d < 3; ++d) {
-  #pragma unroll
+#pragma unroll
         for (int c = 0; c < L; ++c) z[d][c] *= kap;
         eo_expand<L, Q>(z[d], u);
         st_pencil<Q>(w + d * BS, 1, u);

@@ -33,7 +33,7 @@ struct FusedCfg {
   static constexpr int PHYS = B < 7 ? DGMX_EULER2D : DGMX_SHALLOW;
   static constexpr int P = B % 7 + 1, L = P + 1, Q = P + 2;
   static constexpr int EPB = stage2d_epb(phys_nf(PHYS), L);
-    static constexpr bool PAIR =
+  static constexpr bool PAIR =
       MIXED && CfgD<PHYS, L, Q, 2 * EPB, kFusedThreads, 0, MIXED>::SMEM <= 228 * 1024 / kFusedMinBlocksMixed - 1024;
   using C = CfgD<PHYS, L, Q, PAIR ? 2 * EPB : EPB, kFusedThreads, 0, MIXED>;
 };

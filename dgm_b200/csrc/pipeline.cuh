@@ -235,12 +235,6 @@ __device__ __forceinline__ void stage_tile_pipe(const Smem<C> &sm, const StageAr
       float q[L];
 #pragma unroll
       for (int k = 0; k < L; ++k) q[k] = Rr[k];
-      if (a.Ssrc)
-#pragma unroll
-        for (int k = 0; k < L; ++k) q[k] -= float(a.src_scale * a.Ssrc[gi + k]);
-      if (a.Rsub)
-#pragma unroll
-        for (int k = 0; k < L; ++k) q[k] -= float(a.Rsub[gi + k]);
       if (a.kind == kRHS) {
 #pragma unroll
         for (int k = 0; k < L; ++k) a.A[gi + k] = q[k];
@@ -263,15 +257,6 @@ __device__ __forceinline__ void stage_tile_pipe(const Smem<C> &sm, const StageAr
       double q[L];
 #pragma unroll
       for (int k = 0; k < L; ++k) q[k] = Rr[k];
-      if (a.Ssrc)
-#pragma unroll
-        for (int k = 0; k < L; ++k) q[k] -= a.src_scale * a.Ssrc[gi + k];
-      if (a.Rcap)
-#pragma unroll
-        for (int k = 0; k < L; ++k) a.Rcap[gi + k] = q[k];
-      if (a.Rsub)
-#pragma unroll
-        for (int k = 0; k < L; ++k) q[k] -= a.Rsub[gi + k];
       if (a.kind == kRHS) {
 #pragma unroll
         for (int k = 0; k < L; ++k) a.A[gi + k] = q[k];

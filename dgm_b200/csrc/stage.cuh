@@ -678,12 +678,6 @@ __device__ __forceinline__ void stage_tile(const Smem<C> &sm, const StageArgs &a
       float rr[L];
 #pragma unroll
       for (int k = 0; k < L; ++k) rr[k] = Rr[k];
-      if (a.Ssrc)
-#pragma unroll
-        for (int k = 0; k < L; ++k) rr[k] -= float(a.src_scale * a.Ssrc[gi + k]);
-      if (a.Rsub)
-#pragma unroll
-        for (int k = 0; k < L; ++k) rr[k] -= float(a.Rsub[gi + k]);
       if (a.kind == kRHS) {
 #pragma unroll
         for (int k = 0; k < L; ++k) a.A[gi + k] = rr[k];
@@ -708,15 +702,6 @@ __device__ __forceinline__ void stage_tile(const Smem<C> &sm, const StageArgs &a
       double rr[L];
 #pragma unroll
       for (int k = 0; k < L; ++k) rr[k] = Rr[k];
-      if (a.Ssrc)
-#pragma unroll
-        for (int k = 0; k < L; ++k) rr[k] -= a.src_scale * a.Ssrc[gi + k];
-      if (a.Rcap)   // first RHS (shallow-water balance)
-#pragma unroll
-        for (int k = 0; k < L; ++k) a.Rcap[gi + k] = rr[k];
-      if (a.Rsub)
-#pragma unroll
-        for (int k = 0; k < L; ++k) rr[k] -= a.Rsub[gi + k];
       if constexpr (PHYS == DGMX_NS2D || PHYS == DGMX_NS3D) {
         if (n >= 1)
 #pragma unroll
@@ -904,18 +889,6 @@ __global__ void __launch_bounds__(C::NT, C::MINB) rhs_nodal_kernel(StageArgs a) 
     for (int w = tid; w < EPB * BLK; w += C::NT) {
       const int e = e0 + w / BLK, n = (w % BLK) / C::LD, m = w % C::LD;
       if (e < a.ne && n >= 1) sm.R[w] = sm.R[w] - a.Pv[((size_t)e * (NF - 1) + (n - 1)) * C::LD + m];
-    }
-    csync<C>();
-  }
-  if (a.Ssrc || a.Rcap || a.Rsub) {
-    constexpr int BLK = NF * C::LD;
-    for (int w = tid; w < EPB * BLK; w += C::NT) {
-      const int e = e0 + w / BLK;
-      if (e >= a.ne) continue;
-      const size_t gi = (size_t)e0 * BLK + w;
-      if (a.Ssrc) sm.R[w] = sm.R[w] - a.src_scale * a.Ssrc[gi];
-      if (a.Rcap) a.Rcap[gi] = sm.R[w];
-      if (a.Rsub) sm.R[w] = sm.R[w] - a.Rsub[gi];
     }
     csync<C>();
   }

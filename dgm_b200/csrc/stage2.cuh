@@ -621,12 +621,6 @@ __device__ __forceinline__ void s2_update(const Smem2<C> &sm, const StageArgs &a
         float q[L];
 #pragma unroll
         for (int c = 0; c < L; ++c) q[c] = R[c];
-        if (a.Ssrc)
-#pragma unroll
-          for (int c = 0; c < L; ++c) q[c] -= float(a.src_scale * a.Ssrc[gi + c]);
-        if (a.Rsub)
-#pragma unroll
-          for (int c = 0; c < L; ++c) q[c] -= float(a.Rsub[gi + c]);
         if (a.kind == kRHS) {
 #pragma unroll
           for (int c = 0; c < L; ++c) { a.A[gi + c] = q[c]; ub[c] = float(c == 0 ? x[c] - ref0 : x[c]); }
@@ -649,15 +643,6 @@ __device__ __forceinline__ void s2_update(const Smem2<C> &sm, const StageArgs &a
         double q[L];
 #pragma unroll
         for (int c = 0; c < L; ++c) q[c] = R[c];
-        if (a.Ssrc)
-#pragma unroll
-          for (int c = 0; c < L; ++c) q[c] -= a.src_scale * a.Ssrc[gi + c];
-        if (a.Rcap)
-#pragma unroll
-          for (int c = 0; c < L; ++c) a.Rcap[gi + c] = q[c];
-        if (a.Rsub)
-#pragma unroll
-          for (int c = 0; c < L; ++c) q[c] -= a.Rsub[gi + c];
         if (a.kind == kRHS) {
 #pragma unroll
           for (int c = 0; c < L; ++c) { a.A[gi + c] = q[c]; ub[c] = x[c]; }
