@@ -367,6 +367,8 @@ class Domain:
         return F
 
     def time_derivative_device(self, U_ptr: int, F_ptr: int):
+        """The same on device buffers, enqueued on the handle's stream; F_ptr
+        may be U_ptr."""
         self._check(lib().dgmx_time_derivative_device(self.h, ctypes.c_void_p(U_ptr), ctypes.c_void_p(F_ptr)))
 
     def advance(self, dt: float, nsteps: int = 1):
@@ -389,7 +391,7 @@ class Domain:
 
     def autotune(self, reps: int = 20):
         """Pick the fastest compiled tile variant on this mesh; returns
-        (rows of (epb, minb, threads, us per launch), chosen index)."""
+        (rows of (epb, minb, threads, us per stage), chosen index)."""
         L = lib()
         f = L.dgmx_autotune
         f.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.POINTER(ctypes.c_double), ctypes.c_int,

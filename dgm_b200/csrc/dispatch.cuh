@@ -462,10 +462,11 @@ void reg2() {
   constexpr int B96 = blocks_for_regs<CB>(NTB, 96), B80 = blocks_for_regs<CB>(NTB, 80);
   constexpr int B64 = blocks_for_regs<CB>(NTB, 64), A64 = blocks_for_regs<CA>(NTA, 64);
   reg2_variant<PHYS, P, Q, 1, NTA, 0, MIXED>();
-  // up to p = 4 the default (p = 3, 32^3: FP64 260 us against the third form's
-  // 315, FP32 201 against 215; p = 2, 20^3: 39 against 54; above, the third
-  // form's tile is faster); a mesh of one wave takes the uncapped tile (p = 3,
-  // 8^3: 7.4 us against 11 to 12 for the capped ones)
+  // up to p = 4 the default (p = 3, 32^3: FP64 239 us against the third form's
+  // 314, FP32 190 against 214; p = 2, 20^3: 37.5 against 54 and 33 against 41; p = 4,
+  // 18^3: 112 against 124 and 71 against 82; at p = 5, 14^3, 87 against 91 and 57
+  // against 57); a mesh of one wave takes the uncapped tile (p = 3, 8^3: 6.7 us
+  // against 7.9 to 11.8 for the capped ones)
   constexpr int PREF = P <= 4 ? 2 : 0, ONE_WAVE = P <= 4 ? 4 : 0;
   reg2_variant<PHYS, P, Q, 1, NTB, 0, MIXED>(0, MIXED ? 0 : ONE_WAVE);
   if constexpr (B96 >= 2) reg2_variant<PHYS, P, Q, 1, NTB, B96, MIXED>(0, MIXED ? ONE_WAVE : 0);

@@ -356,9 +356,12 @@ int dgmx_kernel_list(int *rows, int cap);
 
 /* Autotuner (no counterpart in the reference): times every compiled tile
  * variant for this handle's physics and order on its own mesh with
- * right-hand-side-only launches (the state is unchanged) and keeps the
+ * right-hand-side-only stages (the state is unchanged; Navier-Stokes: the
+ * viscous kernels of the handle's form and the stage kernel) and keeps the
  * fastest.  rows (optional): cap rows of (elements per CTA, min CTAs per SM,
- * threads per CTA, microseconds per launch). */
+ * threads per CTA, microseconds per stage).  With the tensor-core
+ * contractions on, every tile runs the same kernels: they are timed and the
+ * handle's tile stays. */
 dgmx_status dgmx_autotune(dgmx_domain *d, int reps, double *rows, int cap, int *nvariants, int *chosen);
 
 /* Selects compiled tile variant `index` (0 .. nvariants-1, the order of
