@@ -84,7 +84,7 @@ static cudaError_t upload_tables2_lq(const Tables1D &t) {
 }
 
 // Whether CV::MINB CTAs of the FP32 viscous kernels' tile CV fit one SM's
-// shared memory (Navier-Stokes only: other physics have no viscous kernels).
+// shared memory (3-D Navier-Stokes only: other physics have no such kernels).
 template <bool NS, class CV>
 struct ViscPairFits {
   static constexpr bool value = false;
@@ -108,7 +108,7 @@ struct Launch {
   // NsCfg::Grad::TRG and NsCfg::Visc::LEAN, ~50 KB each) let CTAs' barrier
   // waits overlap the others' work (p = 7, q = 9: 15 % faster than 384 x 3).
   using CV2 = Cfg<PHYS, L, Q, EPB, 4, MIXED, 256>;
-  static constexpr bool kViscPair = C::QD > 512 && EPB == 1 && ViscPairFits<is_ns(PHYS) && !MIXED, CV2>::value;
+  static constexpr bool kViscPair = C::QD > 512 && EPB == 1 && ViscPairFits<PHYS == DGMX_NS3D && !MIXED, CV2>::value;
   using CV = std::conditional_t<kViscPair, CV2, C>;
   static dim3 grid(int ne) { return dim3((unsigned)((ne + EPB - 1) / EPB)); }
   static dim3 vgrid(const StageArgs &a) { return a.vtiles ? dim3((unsigned)a.nvtiles) : grid(a.ne); }

@@ -45,16 +45,15 @@ constexpr size_t ns_data_bytes(int values) { return ((size_t)values * sizeof(V) 
 template <class C, class V = float>
 struct NsCfg {
   static constexpr int DIM = C::DIM, NF = C::NF, L = C::L, Q = C::Q, G = C::G;
+  static_assert(DIM == 3, "the 3xTF32 option is 3-D");
   static constexpr int EPB = C::EPB, NFACE = C::NFACE, NT = C::NT;
   static constexpr int QD = C::QD, LD = C::LD, GF = C::GF, QF = C::QF, LF = C::LF;
-  static constexpr int NVC = DIM + 1;       // primitive components u, v, (w), e
+  static constexpr int NVC = DIM + 1;       // primitive components u, v, w, e
   static constexpr int NG = NVC * DIM;      // gradient components
   static constexpr int NV = NF - 1;         // viscous fields
   static_assert(NV * DIM == NG, "viscous flux components reuse the gradient slots");
-  static constexpr int P1 = DIM == 3 ? Q * L * L : Q * L;     // backward pass-1 size
-  static constexpr int P2 = DIM == 3 ? Q * Q * L : 0;         // backward pass-2 size
-  static constexpr int F1 = DIM == 3 ? L * Q * Q : L * Q;     // forward pass-1 size
-  static constexpr int F2 = DIM == 3 ? L * L * Q : 0;         // forward pass-2 size
+  static constexpr int P1 = Q * L * L, P2 = Q * Q * L;   // backward pass sizes
+  static constexpr int F1 = L * Q * Q, F2 = L * L * Q;   // forward pass sizes
   // fields per backward-transform batch: one slot's fields in two batches
   // (at most 3 at a time) keep the transform scratch at the size the
   // per-component passes need
@@ -79,7 +78,7 @@ struct NsCfg {
     static constexpr bool TRG = NT < QD;
     static constexpr int E = TRG ? 0 : NFACE * NF * GF * DW, E2 = E, Rs = F32 ? 2 * DW : 0;
     static constexpr int Fc = NFACE * DIM * GF, LFc = cmax(NFACE * DIM * QF, DIM * F2);
-    static constexpr int S1 = cmax(cmax(NB1 * P1, DIM == 3 ? NFACE * DIM * Q * G : 0), DIM * F1);
+    static constexpr int S1 = cmax(cmax(NB1 * P1, NFACE * DIM * Q * G), DIM * F1);
     static constexpr int S2 = cmax(cmax(NB1 * P2, DIM * F2), DIM * LD);
     static constexpr int SLOT = A + B + E + E2 + Rs + Fc + LFc + S1 + S2;
     static constexpr size_t DATA = ns_data_bytes<V>(EPB * SLOT);
@@ -87,7 +86,7 @@ struct NsCfg {
   };
   // ns_visc_kernel regions (per slot, values of the working type).  G holds the velocity
   // gradient, then in place the symmetric stress and the heat flux (NGS
-  // slots: 6 + 3 in 3-D, 3 + 2 in 2-D; the modal input is parked there
+  // slots: 6 + 3; the modal input is parked there
   // first); the energy gradient goes to Dv, which then accumulates one
   // field's divergence at a time.  B holds the state until the stresses are
   // formed, then the face values FF and the divergence input Cv; X holds the
@@ -101,13 +100,13 @@ struct NsCfg {
     // forms the stresses before the energy gradient is brought into the
     // heat-flux slots, and keeps the divergence behind the face values in B.
     static constexpr bool LEAN = NT < QD && EPB == 1;
-    static constexpr int NGS = DIM == 3 ? 9 : 5;
+    static constexpr int NGS = 9;
     static constexpr int FF = cmax(NFACE * DIM * QF, F2), Cv = QD;
     static constexpr int B = LEAN ? cmax((DIM + 1) * QD, FF + Cv + QD) : cmax(NF * QD, FF + Cv);
     static constexpr int G = cmax(NGS * QD, NF * LD);
     static constexpr int X = cmax(DIM * LD, NFACE * DIM * GF);
-    static constexpr int S1 = LEAN ? cmax(P1, cmax(DIM == 3 ? NFACE * DIM * C::G * Q : 0, F1))
-                                   : cmax(cmax(NB1 * P1, DIM * P1), cmax(DIM == 3 ? NFACE * DIM * C::G * Q : 0, F1));
+    static constexpr int S1 = LEAN ? cmax(P1, cmax(NFACE * DIM * C::G * Q, F1))
+                                   : cmax(cmax(NB1 * P1, DIM * P1), cmax(NFACE * DIM * C::G * Q, F1));
     static constexpr int S2 = LEAN ? cmax(cmax(P2, LD), F2) : cmax(cmax(NB1 * P2, DIM * P2), LD);
     static constexpr int Dv = LEAN ? 0 : DIM * QD;
     static constexpr int SLOT = B + G + X + S1 + S2 + Dv;
@@ -117,12 +116,9 @@ struct NsCfg {
     static_assert(DATA % 8 == 0 && DATA >= (size_t)EPB * SLOT * sizeof(V), "geometry slots 8-byte aligned");
   };
   // slot of component d of the viscous flux vector g_n (n: momentum x, y,
-  // [z], energy) in the symmetric stress / heat-flux layout
+  // z, energy) in the symmetric stress / heat-flux layout
   static constexpr __host__ __device__ int gslot(int n, int d) {
-    if (DIM == 3) {
-      return n == 3 ? 6 + d : (n == 0 ? d : (n == 1 ? (d == 0 ? 1 : 2 + d) : (d == 0 ? 2 : (d == 1 ? 4 : 5))));
-    }
-    return n == 2 ? 3 + d : (n == 0 ? d : 1 + d);
+    return n == 3 ? 6 + d : (n == 0 ? d : (n == 1 ? (d == 0 ? 1 : 2 + d) : (d == 0 ? 2 : (d == 1 ? 4 : 5))));
   }
   // CTAs per SM for a viscous kernel of smem bytes: the tile's register cap
   // when it has one, else as many as shared memory holds while the register
@@ -194,35 +190,22 @@ template <class C, int NB, class V>
 __device__ __forceinline__ void lift_batch(const V *Fg, V *LFc, V *S, V *dst, int tid) {
   constexpr int DIM = C::DIM, L = C::L, Q = C::Q, G = C::G, EPB = C::EPB, QD = C::QD, QF = C::QF;
   constexpr int NBT = C::NFACE * EPB * NB;
-  if constexpr (DIM == 3) {
-    vcontract<G, G, 1, 0, G, Q, MatG2GL<L, Q, V>, false>(Fg, S, NBT, G * G, Q * G, tid, C::NT);
-    __syncthreads();
-    vcontract<Q, G, 1, 1, G, Q, MatG2GL<L, Q, V>, false>(S, LFc, NBT, Q * G, Q * Q, tid, C::NT);
-  } else {
-    vcontract<G, 1, 1, 0, G, Q, MatG2GL<L, Q, V>, false>(Fg, LFc, NBT, G, Q, tid, C::NT);
-  }
+  vcontract<G, G, 1, 0, G, Q, MatG2GL<L, Q, V>, false>(Fg, S, NBT, G * G, Q * G, tid, C::NT);
+  __syncthreads();
+  vcontract<Q, G, 1, 1, G, Q, MatG2GL<L, Q, V>, false>(S, LFc, NBT, Q * G, Q * Q, tid, C::NT);
   __syncthreads();
   const V w0 = V(1.0) / cW<V, L, Q>[0], w1 = V(1.0) / cW<V, L, Q>[Q - 1];
   for (int w = tid; w < EPB * NB * QD; w += C::NT) {
     const int slot = w / (NB * QD), rem = w - slot * NB * QD, b = rem / QD, p = rem - b * QD;
     V acc = dst[w];
-    if constexpr (DIM == 3) {
-      const int i = p / (Q * Q), j = (p / Q) % Q, k = p % Q;
-      auto lf = [&](int f, int x, int y) { return LFc[((f * EPB + slot) * NB + b) * QF + x * Q + y]; };
-      if (k == 0) acc = fma(w0, lf(0, i, j), acc);
-      if (j == 0) acc = fma(w0, lf(1, i, k), acc);
-      if (i == Q - 1) acc = fma(w1, lf(2, j, k), acc);
-      if (j == Q - 1) acc = fma(w1, lf(3, i, k), acc);
-      if (i == 0) acc = fma(w0, lf(4, j, k), acc);
-      if (k == Q - 1) acc = fma(w1, lf(5, i, j), acc);
-    } else {
-      const int i = p / Q, j = p % Q;
-      auto lf = [&](int f, int x) { return LFc[((f * EPB + slot) * NB + b) * QF + x]; };
-      if (j == 0) acc = fma(w0, lf(0, i), acc);
-      if (i == Q - 1) acc = fma(w1, lf(1, j), acc);
-      if (j == Q - 1) acc = fma(w1, lf(2, i), acc);
-      if (i == 0) acc = fma(w0, lf(3, j), acc);
-    }
+    const int i = p / (Q * Q), j = (p / Q) % Q, k = p % Q;
+    auto lf = [&](int f, int x, int y) { return LFc[((f * EPB + slot) * NB + b) * QF + x * Q + y]; };
+    if (k == 0) acc = fma(w0, lf(0, i, j), acc);
+    if (j == 0) acc = fma(w0, lf(1, i, k), acc);
+    if (i == Q - 1) acc = fma(w1, lf(2, j, k), acc);
+    if (j == Q - 1) acc = fma(w1, lf(3, i, k), acc);
+    if (i == 0) acc = fma(w0, lf(4, j, k), acc);
+    if (k == Q - 1) acc = fma(w1, lf(5, i, j), acc);
     dst[w] = acc;
   }
   __syncthreads();
@@ -235,23 +218,15 @@ __device__ __forceinline__ void forward_batch(V *src, V *dst, V *S1, V *S2, int 
   constexpr int DIM = C::DIM, L = C::L, Q = C::Q, QD = C::QD, LD = C::LD, NBT = C::EPB * NB;
   for (int w = tid; w < NBT * QD; w += C::NT) {
     const int p = w % QD;
-    V wq;
-    if constexpr (DIM == 3) wq = cW<V, L, Q>[p / (Q * Q)] * cW<V, L, Q>[(p / Q) % Q] * cW<V, L, Q>[p % Q];
-    else wq = cW<V, L, Q>[p / Q] * cW<V, L, Q>[p % Q];
+    const V wq = cW<V, L, Q>[p / (Q * Q)] * cW<V, L, Q>[(p / Q) % Q] * cW<V, L, Q>[p % Q];
     src[w] = wq * src[w];
   }
   __syncthreads();
-  if constexpr (DIM == 3) {
-    vcontract<Q, Q, Q, 0, Q, L, MatBt<L, Q, V>, false>(src, S1, NBT, QD, L * Q * Q, tid, C::NT);
-    __syncthreads();
-    vcontract<L, Q, Q, 1, Q, L, MatBt<L, Q, V>, false>(S1, S2, NBT, L * Q * Q, L * L * Q, tid, C::NT);
-    __syncthreads();
-    vcontract<L, L, Q, 2, Q, L, MatBt<L, Q, V>, false>(S2, dst, NBT, L * L * Q, LD, tid, C::NT);
-  } else {
-    vcontract<Q, Q, 1, 0, Q, L, MatBt<L, Q, V>, false>(src, S1, NBT, QD, L * Q, tid, C::NT);
-    __syncthreads();
-    vcontract<L, Q, 1, 1, Q, L, MatBt<L, Q, V>, false>(S1, dst, NBT, L * Q, LD, tid, C::NT);
-  }
+  vcontract<Q, Q, Q, 0, Q, L, MatBt<L, Q, V>, false>(src, S1, NBT, QD, L * Q * Q, tid, C::NT);
+  __syncthreads();
+  vcontract<L, Q, Q, 1, Q, L, MatBt<L, Q, V>, false>(S1, S2, NBT, L * Q * Q, L * L * Q, tid, C::NT);
+  __syncthreads();
+  vcontract<L, L, Q, 2, Q, L, MatBt<L, Q, V>, false>(S2, dst, NBT, L * L * Q, LD, tid, C::NT);
   __syncthreads();
 }
 
@@ -259,17 +234,11 @@ __device__ __forceinline__ void forward_batch(V *src, V *dst, V *S1, V *S2, int 
 template <class C, int NB, class V>
 __device__ __forceinline__ void backward_batch(const V *src, V *dst, V *S1, V *S2, int tid) {
   constexpr int L = C::L, Q = C::Q, NBT = C::EPB * NB;
-  if constexpr (C::DIM == 3) {
-    vcontract<L, L, L, 0, L, Q, MatB<L, Q, V>, false>(src, S1, NBT, C::LD, Q * L * L, tid, C::NT);
-    __syncthreads();
-    vcontract<Q, L, L, 1, L, Q, MatB<L, Q, V>, false>(S1, S2, NBT, Q * L * L, Q * Q * L, tid, C::NT);
-    __syncthreads();
-    vcontract<Q, Q, L, 2, L, Q, MatB<L, Q, V>, false>(S2, dst, NBT, Q * Q * L, C::QD, tid, C::NT);
-  } else {
-    vcontract<L, L, 1, 0, L, Q, MatB<L, Q, V>, false>(src, S1, NBT, C::LD, Q * L, tid, C::NT);
-    __syncthreads();
-    vcontract<Q, L, 1, 1, L, Q, MatB<L, Q, V>, false>(S1, dst, NBT, Q * L, C::QD, tid, C::NT);
-  }
+  vcontract<L, L, L, 0, L, Q, MatB<L, Q, V>, false>(src, S1, NBT, C::LD, Q * L * L, tid, C::NT);
+  __syncthreads();
+  vcontract<Q, L, L, 1, L, Q, MatB<L, Q, V>, false>(S1, S2, NBT, Q * L * L, Q * Q * L, tid, C::NT);
+  __syncthreads();
+  vcontract<Q, Q, L, 2, L, Q, MatB<L, Q, V>, false>(S2, dst, NBT, Q * Q * L, C::QD, tid, C::NT);
   __syncthreads();
 }
 
@@ -323,14 +292,14 @@ __device__ __forceinline__ void load_own_traces_v(V *E, const double *T, int e0,
 // The FP32 gradient kernel's state: the slot's modal registers (or, NODAL,
 // GLL values) with the density and energy means taken out in double before
 // rounding.  Modal: the constant coefficients c0 of density and energy go to
-// Rs as means c0 phi0 (phi0 = 2^(-DIM/2), the constant orthonormal mode) and
+// Rs as means c0 phi0 (phi0 = 2^(-3/2), the constant orthonormal mode) and
 // are zeroed.  Nodal: each element's values at its first point are the
 // reference values subtracted.  Elements past the end read a unit density.
 template <class C>
 __device__ __forceinline__ void load_state_shifted(float *dst, double *Rs, const double *src, bool nodal, int e0,
                                                    int ne, int tid) {
   constexpr int NF = C::NF, LD = C::LD, QD = C::QD, EPB = C::EPB;
-  const double phi0 = C::DIM == 3 ? 0.35355339059327373 : 0.5;
+  const double phi0 = 0.35355339059327373;
   if (nodal) {
     for (int w = tid; w < EPB * NF * QD; w += C::NT) {
       const int s = w / (NF * QD), rem = w - s * NF * QD, n = rem / QD, p = rem - n * QD;
@@ -463,20 +432,19 @@ __global__ void __launch_bounds__(C::NT, NsCfg<C, float>::GRAD_MINB) ns_grad_ker
     using Sh = Sh3<DIM, Q>;
     vcontract<Sh::a, Sh::b, Sh::c, 0, Q, Q, MatD<L, Q, V>, false>(Qc, Gd, EPB, QD, DIM * QD, tid, C::NT);
     vcontract<Sh::a, Sh::b, Sh::c, 1, Q, Q, MatD<L, Q, V>, false>(Qc, Gd + QD, EPB, QD, DIM * QD, tid, C::NT);
-    if constexpr (DIM == 3)
-      vcontract<Sh::a, Sh::b, Sh::c, 2, Q, Q, MatD<L, Q, V>, false>(Qc, Gd + 2 * QD, EPB, QD, DIM * QD, tid, C::NT);
+    vcontract<Sh::a, Sh::b, Sh::c, 2, Q, Q, MatD<L, Q, V>, false>(Qc, Gd + 2 * QD, EPB, QD, DIM * QD, tid, C::NT);
     __syncthreads();
     // chain rule (src/Hex.cpp:1994-2006): d/dx = rx d/dr + sx d/ds + tx d/dt
     for (int w = tid; w < EPB * QD; w += C::NT) {
       const int s = w / QD, p = w - s * QD;
       V *g = Gd + s * DIM * QD + p;
       const double *m = geo[s].metric;
-      const V fr = g[0], fs = g[QD], ft = DIM == 3 ? g[2 * QD] : V(0.0);
+      const V fr = g[0], fs = g[QD], ft = g[2 * QD];
 #pragma unroll
       for (int k = 0; k < DIM; ++k) {
         V v = V(m[0 * 3 + k]) * fr;
         v = fma(V(m[1 * 3 + k]), fs, v);
-        if (DIM == 3) v = fma(V(m[2 * 3 + k]), ft, v);
+        v = fma(V(m[2 * 3 + k]), ft, v);
         g[k * QD] = v;
       }
     }
@@ -524,18 +492,12 @@ __device__ __forceinline__ void viscous_stress(const V *g, int stride, V mu, V *
 }
 
 // The energy flux tau . u + (gamma mu / Pr) grad e at one point.
-template <int DIM, class V>
+template <class V>
 __device__ __forceinline__ void heat_flux(const V *t, V u, V v, V w, V ex, V ey, V ez, V mu, V gPr, V *q) {
-  if constexpr (DIM == 3) {
-    V qx = t[0] * u; qx = fma(t[1], v, qx); qx = fma(t[2], w, qx);
-    V qy = t[1] * u; qy = fma(t[3], v, qy); qy = fma(t[4], w, qy);
-    V qz = t[2] * u; qz = fma(t[4], v, qz); qz = fma(t[5], w, qz);
-    q[0] = fma(gPr, mu * ex, qx); q[1] = fma(gPr, mu * ey, qy); q[2] = fma(gPr, mu * ez, qz);
-  } else {
-    V qx = t[0] * u; qx = fma(t[1], v, qx);
-    V qy = t[1] * u; qy = fma(t[2], v, qy);
-    q[0] = fma(gPr, mu * ex, qx); q[1] = fma(gPr, mu * ey, qy);
-  }
+  V qx = t[0] * u; qx = fma(t[1], v, qx); qx = fma(t[2], w, qx);
+  V qy = t[1] * u; qy = fma(t[3], v, qy); qy = fma(t[4], w, qy);
+  V qz = t[2] * u; qz = fma(t[4], v, qz); qz = fma(t[5], w, qz);
+  q[0] = fma(gPr, mu * ex, qx); q[1] = fma(gPr, mu * ey, qy); q[2] = fma(gPr, mu * ez, qz);
 }
 
 // The viscous kernel's first part for the lean tile (NsCfg::Visc::LEAN,
@@ -549,7 +511,7 @@ __device__ __forceinline__ void ns_visc_lean_front(const StageArgs &a, V *B, V *
                                                    int tid) {
   using N = NsCfg<C, V>;
   constexpr int DIM = C::DIM, NF = C::NF, QD = C::QD, LD = C::LD, NVC = N::NVC, NGS = N::Visc::NGS;
-  constexpr int NT6 = DIM == 3 ? 6 : 3;
+  constexpr int NT6 = 6;
   static_assert(C::EPB == 1, "the lean viscous tile holds one element");
   const int e = e0 < a.ne ? e0 : -1;
   // state: density and momenta (the stresses need the velocity only)
@@ -591,9 +553,9 @@ __device__ __forceinline__ void ns_visc_lean_front(const StageArgs &a, V *B, V *
 #pragma unroll
     for (int k = 0; k < NT6; ++k) t[k] = Gg[k * QD + p];
     const V r = B[p];
-    const V u = B[QD + p] / r, v = B[2 * QD + p] / r, w = DIM == 3 ? B[3 * QD + p] / r : V(0.0);
+    const V u = B[QD + p] / r, v = B[2 * QD + p] / r, w = B[3 * QD + p] / r;
     const V *ge = Gg + NT6 * QD + p;
-    heat_flux<DIM, V>(t, u, v, w, ge[0], ge[QD], DIM == 3 ? ge[2 * QD] : V(0.0), mu, gPr, q);
+    heat_flux<V>(t, u, v, w, ge[0], ge[QD], ge[2 * QD], mu, gPr, q);
 #pragma unroll
     for (int d = 0; d < DIM; ++d) Gg[(NT6 + d) * QD + p] = q[d];
   }
@@ -665,14 +627,9 @@ __global__ void __launch_bounds__(C::NT, NsCfg<C, float>::VISC_MINB) ns_visc_ker
     const V r = U[0];
     V t[6], q[3];
     viscous_stress<DIM, V>(g, QD, mu, t);
-    if constexpr (DIM == 3) {
-      const V u = U[1] / r, v = U[2] / r, ww = U[3] / r;
-      heat_flux<DIM, V>(t, u, v, ww, ge[0], ge[QD], ge[2 * QD], mu, gPr, q);
-    } else {
-      const V u = U[1] / r, v = U[2] / r;
-      heat_flux<DIM, V>(t, u, v, V(0.0), ge[0], ge[QD], V(0.0), mu, gPr, q);
-    }
-    constexpr int NT6 = DIM == 3 ? 6 : 3;
+    const V u = U[1] / r, v = U[2] / r, ww = U[3] / r;
+    heat_flux<V>(t, u, v, ww, ge[0], ge[QD], ge[2 * QD], mu, gPr, q);
+    constexpr int NT6 = 6;
 #pragma unroll
     for (int k = 0; k < NT6; ++k) g[k * QD] = t[k];
 #pragma unroll
@@ -687,35 +644,22 @@ __global__ void __launch_bounds__(C::NT, NsCfg<C, float>::VISC_MINB) ns_visc_ker
       const int s = rem / (DIM * QF), rem2 = rem - s * DIM * QF, d = rem2 / QF, x = rem2 - d * QF;
       const V *src = Gg + (s * NGS + N::gslot(n, d)) * QD;
       int p;
-      if constexpr (DIM == 3) {
-        const int u = x / Q, v = x % Q;
-        switch (f) {
-          case 0: p = (u * Q + v) * Q + 0; break;
-          case 1: p = (u * Q + 0) * Q + v; break;
-          case 2: p = ((Q - 1) * Q + u) * Q + v; break;
-          case 3: p = (u * Q + (Q - 1)) * Q + v; break;
-          case 4: p = (0 * Q + u) * Q + v; break;
-          default: p = (u * Q + v) * Q + (Q - 1); break;
-        }
-      } else {
-        switch (f) {
-          case 0: p = x * Q + 0; break;
-          case 1: p = (Q - 1) * Q + x; break;
-          case 2: p = x * Q + (Q - 1); break;
-          default: p = 0 * Q + x; break;
-        }
+      const int u = x / Q, v = x % Q;
+      switch (f) {
+        case 0: p = (u * Q + v) * Q + 0; break;
+        case 1: p = (u * Q + 0) * Q + v; break;
+        case 2: p = ((Q - 1) * Q + u) * Q + v; break;
+        case 3: p = (u * Q + (Q - 1)) * Q + v; break;
+        case 4: p = (0 * Q + u) * Q + v; break;
+        default: p = (u * Q + v) * Q + (Q - 1); break;
       }
       FF[w] = src[p];
     }
     __syncthreads();
     constexpr int NB = NFACE * EPB * DIM;
-    if constexpr (DIM == 3) {
-      vcontract<Q, Q, 1, 0, Q, G, MatGL2G<L, Q, V>, false>(FF, S1, NB, Q * Q, G * Q, tid, C::NT);
-      __syncthreads();
-      vcontract<G, Q, 1, 1, Q, G, MatGL2G<L, Q, V>, false>(S1, Fg, NB, G * Q, G * G, tid, C::NT);
-    } else {
-      vcontract<Q, 1, 1, 0, Q, G, MatGL2G<L, Q, V>, false>(FF, Fg, NB, Q, G, tid, C::NT);
-    }
+    vcontract<Q, Q, 1, 0, Q, G, MatGL2G<L, Q, V>, false>(FF, S1, NB, Q * Q, G * Q, tid, C::NT);
+    __syncthreads();
+    vcontract<G, Q, 1, 1, Q, G, MatGL2G<L, Q, V>, false>(S1, Fg, NB, G * Q, G * G, tid, C::NT);
     __syncthreads();
     // g_n . n (own normals), the viscous trace of this side
     for (int w = tid; w < EPB * NFACE * GF; w += C::NT) {
@@ -725,7 +669,7 @@ __global__ void __launch_bounds__(C::NT, NsCfg<C, float>::VISC_MINB) ns_visc_ker
       const double *nr = geo[s].onrm[f];
       V v = V(nr[0]) * Fg[((f * EPB + s) * DIM + 0) * GF + gq];
       v = fma(V(nr[1]), Fg[((f * EPB + s) * DIM + 1) * GF + gq], v);
-      if (DIM == 3) v = fma(V(nr[2]), Fg[((f * EPB + s) * DIM + 2) * GF + gq], v);
+      v = fma(V(nr[2]), Fg[((f * EPB + s) * DIM + 2) * GF + gq], v);
       a.V[(((size_t)e * NFACE + f) * NV + n) * GF + gq] = double(v);
     }
     // collocation divergence of g_n (contravariant form) into Dv [slot][QD]
@@ -736,7 +680,7 @@ __global__ void __launch_bounds__(C::NT, NsCfg<C, float>::VISC_MINB) ns_visc_ker
         const V *gs = Gg + s * NGS * QD + p;
         V v = V(m[3 * r + 0]) * gs[N::gslot(n, 0) * QD];
         v = fma(V(m[3 * r + 1]), gs[N::gslot(n, 1) * QD], v);
-        if (DIM == 3) v = fma(V(m[3 * r + 2]), gs[N::gslot(n, 2) * QD], v);
+        v = fma(V(m[3 * r + 2]), gs[N::gslot(n, 2) * QD], v);
         Cv[w] = v;
       }
       __syncthreads();
