@@ -220,7 +220,7 @@ __device__ __forceinline__ void f3_state_nodal(double *buf, double *mean, const 
     const int n = w / QD, p = w - n * QD, i = p / (Q * Q), jk = p - i * Q * Q, j = jk / Q, k = jk - j * Q;
     const double v = a.Xn[((size_t)n * a.ne + e) * QD + p];
     buf[n * C::BS + i * C::SI + j * C::SJ + k] = v;
-    if (p == QD / 2) mean[n] = v;
+    if (p == Q / 2 * (Q * Q + Q + 1)) mean[n] = v;
   }
 }
 

@@ -285,7 +285,7 @@ __device__ __forceinline__ void s2_face_point(const Smem2<C> &sm, const StageArg
 
 // ---- interval 1b: backward k-pass from the modal rows in global memory ----
 // T1[b][n a][k] = sum_c B[c][k] u[n][a][b][c]; the mixed form leaves the
-// constant mode out: its value is kept (s2_reference).  Elements past the end
+// constant mode out: its value is kept (element_reference).  Elements past the end
 // get the constant state (their results are discarded).
 template <class C>
 __device__ __forceinline__ void s2_backward_k_row(const Smem2<C> &sm, const StageArgs &a, int e0, int w) {
@@ -872,7 +872,7 @@ __global__ void __launch_bounds__(C::NT, C::MINB) rhs2_kernel(StageArgs a) {
   // while the face points are done
   const int k = tid - (C::NT - 15);
   double own = 0.0;
-  if (k > 0) own = k <= NF ? a.Xn[((size_t)(k - 1) * a.ne + e) * QD + QD / 2] : __ldg(&a.classes[sm.cls[0]].metric[k - 1 - NF]);
+  if (k > 0) own = k <= NF ? a.Xn[((size_t)(k - 1) * a.ne + e) * QD + Q / 2 * (Q * Q + Q + 1)] : __ldg(&a.classes[sm.cls[0]].metric[k - 1 - NF]);
   for (int w = tid; w < C::NFACE * C::GF; w += C::NT) s2_face_point<C, PHYS>(sm, a, e, w);
   if (k > 0) sl[C::O_CST + k] = own;
   __syncthreads();
