@@ -464,12 +464,16 @@ void reg2() {
   reg2_variant<PHYS, P, Q, 1, NTA, 0, MIXED>();
   // up to p = 4 the default (p = 3, 32^3: FP64 239 us against the third form's
   // 314, FP32 190 against 214; p = 2, 20^3: 37.5 against 54 and 33 against 41; p = 4,
-  // 18^3: 112 against 124 and 71 against 82; at p = 5, 14^3, 87 against 91 and 57
-  // against 57); a mesh of one wave takes the uncapped tile (p = 3, 8^3: 6.7 us
-  // against 7.9 to 11.8 for the capped ones)
-  constexpr int PREF = P <= 4 ? 2 : 0, ONE_WAVE = P <= 4 ? 4 : 0;
+  // 16^3: 76 against 94 and, 18^3, 71 against 82; at p = 5, 14^3, 87 against 91 and
+  // 57 against 57); a mesh of one wave takes the uncapped tile (p = 3, 8^3: 6.7 us
+  // against 7.9 to 11.8 for the capped ones).  FP64 at p = 4, where shared memory
+  // holds five CTAs at 80 registers as at 96: the wider tile at 96 for every mesh
+  // (5^3 8.8 us, uncapped 8.6; 8^3 12.3 / 15.8; 16^3 76 / 81; 30^3 467 / 510).
+  constexpr bool WIDE = !MIXED && P <= 4 && A80 == A96;
+  constexpr int PREF = P <= 4 ? 2 : 0, ONE_WAVE = P <= 4 && !WIDE ? 4 : 0;
   reg2_variant<PHYS, P, Q, 1, NTB, 0, MIXED>(0, MIXED ? 0 : ONE_WAVE);
-  if constexpr (B96 >= 2) reg2_variant<PHYS, P, Q, 1, NTB, B96, MIXED>(0, MIXED ? ONE_WAVE : 0);
+  static_assert(!WIDE || B96 >= 2, "a preferred tile");
+  if constexpr (B96 >= 2) reg2_variant<PHYS, P, Q, 1, NTB, B96, MIXED>(WIDE ? PREF : 0, MIXED ? ONE_WAVE : 0);
   if constexpr (A96 >= 2) reg2_variant<PHYS, P, Q, 1, NTA, A96, MIXED>();
   if constexpr (B80 >= 2 && B80 != B96) reg2_variant<PHYS, P, Q, 1, NTB, B80, MIXED>();
   if constexpr (A80 >= 2 && A80 != A96) reg2_variant<PHYS, P, Q, 1, NTA, A80, MIXED>(MIXED ? 0 : PREF);
